@@ -53,15 +53,15 @@ struct FusedArgs {
 };
 
 // ---- integer-exact norm reciprocal (include/slopfab/cuda/deterministic_math.cuh:26-197) ----
-__device__ __forceinline__ uint64_t shift_rne(uint64_t v, unsigned s) {
-  const uint64_t q = v >> s;
-  const uint64_t rem = v & ((uint64_t(1) << s) - 1);
-  const uint64_t half = uint64_t(1) << (s - 1);
-  return q + ((rem > half || (rem == half && (q & 1))) ? 1 : 0);
+// RNE(v / 2^S) of a product whose result fits 32 bits: half minus one, plus one more when the kept part is odd.
+template <int S> __device__ __forceinline__ uint32_t shift_rne32(uint64_t v) {
+  return uint32_t((v + ((uint64_t(1) << (S - 1)) - 1) + (uint32_t(v >> S) & 1u)) >> S);
 }
 // 1/sqrt(v) for a positive normal v: Newton in unsigned Q30 with round-half-even shifts, six
-// steps from a seed chosen by the exponent's parity, then rounded to 24 bits.
-__device__ float rsqrt_q30(float value) {
+// steps from a seed chosen by the exponent's parity, then rounded to 24 bits. Every operand fits 32 bits (checked on the
+// host for all 2^24 significand / parity pairs), so a step is three 32 x 32 -> 64 multiplications: the steps are a serial
+// chain that the threads of a row wait for.
+__device__ __forceinline__ float rsqrt_q30(float value) {
   const uint32_t mag = __float_as_uint(value) & 0x7FFFFFFFu;
   if (mag == 0u) return __uint_as_float(0x7F800000u);
   if ((__float_as_uint(value) & 0x80000000u) || mag > 0x7F800000u) return __uint_as_float(0x7FC00000u);
@@ -77,22 +77,24 @@ __device__ float rsqrt_q30(float value) {
     sig |= 0x00800000u;
   }
   const int odd = expo & 1;
-  const uint64_t m = uint64_t(sig) << (7 + odd);
+  const uint32_t m = sig << (7 + odd);
   const int out_scale = -(expo - odd) / 2;
-  uint64_t y = odd ? 637534208ull : 872415232ull;
-#pragma unroll 1
+  uint32_t y = odd ? 637534208u : 872415232u;
+#pragma unroll
   for (int it = 0; it < 6; ++it) {
-    const uint64_t y2 = shift_rne(y * y, 30);
-    const uint64_t my2 = shift_rne(m * y2, 30);
-    y = shift_rne(y * (3ull * (1ull << 30) - my2), 31);
+    const uint32_t y2 = shift_rne32<30>(uint64_t(y) * y);
+    const uint32_t my2 = shift_rne32<30>(uint64_t(m) * y2);
+    y = shift_rne32<31>(uint64_t(y) * (3u * (1u << 30) - my2));
   }
-  int t = 63 - __clzll((long long)y);
-  uint64_t r = shift_rne(y, unsigned(t - 23));
-  if (r == (1ull << 24)) {
+  int t = 31 - __clz(y);  // 28 .. 30
+  const uint32_t drop = uint32_t(t - 23), half = 1u << (drop - 1), rem = y & ((1u << drop) - 1);
+  uint32_t r = y >> drop;
+  r += rem > half || (rem == half && (r & 1u)) ? 1u : 0u;
+  if (r == (1u << 24)) {
     r >>= 1;
     ++t;
   }
-  return __uint_as_float((uint32_t(t - 30 + out_scale + 127) << 23) | (uint32_t(r) & 0x007FFFFFu));
+  return __uint_as_float((uint32_t(t - 30 + out_scale + 127) << 23) | (r & 0x007FFFFFu));
 }
 // rsqrt(RNE(sum / dim) + eps); IEEE division and addition are the reference's integer forms.
 __device__ float norm_rsqrt(float sum, int dim, float eps) {
@@ -620,12 +622,22 @@ void quantize_nvfp4_block(const __nv_bfloat16* x, const NormArgs& norm, uint8_t*
 
 // ---- head-wise q/k RMSNorm and MM-RoPE, the two steps between the fused projection and attention ----
 // launch_head_rmsnorm (src/cuda/nn_kernels.cu:296-305 -> rmsnorm_warp_kernel, :100-136) followed by launch_rope_h3
-// (src/cuda/nn_position.cu:15-68,111-123), in place, one warp per (row, head), head_dim 128, on a row pitch so that
-// the q and k thirds of the fused projection are processed where they lie. Bit-exact: 16 lanes hold 8 channels each;
-// the sum of squares is the reference's per-lane chain and xor butterfly; the normalised value is rounded to bf16
-// before the rotation (the reference stores it between its two kernels); the rotation pairs channel j with j + 48
-// over the first 96 channels with the reference's subnormal canonicalisation at every step.
+// (src/cuda/nn_position.cu:15-68,111-123), in place, head_dim 128, on a row pitch so that the q and k thirds of the fused
+// projection are processed where they lie. Bit-exact: 16 lanes hold 8 channels each; the sum of squares is the reference's
+// per-lane chain and xor butterfly (whose first step adds the zeros of its idle upper lanes); the normalised value is
+// rounded to bf16 before the rotation (the reference stores it between its two kernels); the rotation pairs channel j with
+// j + 48 over the first 96 channels with the reference's subnormal canonicalisation.
+//
+// What bounds it: HBM (read and write 256 bytes per head) once the instruction count is down, so a warp takes EIGHT heads of
+// one row, four per half warp: four 16-byte loads per lane in flight, the row's cos / sin read once for all of them, and the
+// serial part of the norm - the integer Newton reciprocal - run once for the eight heads side by side in different lanes.
+// The canonicalisation costs one running minimum: a lane whose operands, products and results are all normal numbers has
+// nothing to canonicalise; one that saw a smaller magnitude (a zero counts) recomputes its eight channels step by step.
+// Measured, q and k of 4747 rows x 40 heads: 61 us (3.2 TB/s); one warp per head with the reciprocal in one lane and the
+// canonicalisation in every channel: 436 us.
 namespace {
+constexpr int kHeadsPerWarp = 8;
+
 __device__ __forceinline__ float rope_bf16_value(unsigned short bits) {
   return (bits & 0x7fffu) < 0x0080u ? __uint_as_float(unsigned(bits & 0x8000u) << 16) : __uint_as_float(unsigned(bits) << 16);
 }
@@ -643,84 +655,124 @@ __device__ __forceinline__ float rope_fma_product(float a, float b, float base) 
   if (magnitude < 0x00800000u && (__float_as_uint(a) & 0x7fffffffu) != 0u && (__float_as_uint(b) & 0x7fffffffu) != 0u) return base;
   return fmaf(a, b, base);
 }
+// One channel with every canonicalisation spelled out. `low`: channels 0-47 of the head, `other` is the partner's value.
+__device__ __forceinline__ unsigned short rope_channel(bool low, unsigned short own, unsigned short other, float cos_v, float sin_v) {
+  const float c = rope_float_value(cos_v), s = rope_float_value(sin_v), x = rope_bf16_value(own), o = rope_bf16_value(other);
+  const float base = rope_float_value(__fmul_rn(x, c));
+  return rope_bf16_result(low ? __fsub_rn(base, rope_float_value(__fmul_rn(o, s))) : rope_fma_product(o, s, base));
+}
+__device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
+__device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 
+template <bool NORM, bool ROPE>
 __global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __restrict__ x, int ld, const __nv_bfloat16* __restrict__ w,
                                                              const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
-                                                             int rows, int heads, float eps) {
-  const int lane = threadIdx.x & 31;
-  const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // (row, head)
-  if (unit >= (long long)rows * heads) return;
-  const int row = int(unit / heads), head = int(unit % heads);
-  __nv_bfloat16* v = x + size_t(row) * ld + head * 128;
-  const bool active = lane < 16;
-  uint4 raw = make_uint4(0, 0, 0, 0);
-  if (active) raw = *reinterpret_cast<const uint4*>(v + lane * 8);
-  unsigned short h[8];
-  {
-    const unsigned u[4] = {raw.x, raw.y, raw.z, raw.w};
+                                                             int tables_vec, int rows, int heads, float eps) {
+  constexpr int kPer = kHeadsPerWarp / 2;  // heads per half warp
+  const int lane = threadIdx.x & 31, l = lane & 15, half = lane >> 4;
+  const int groups = (heads + kHeadsPerWarp - 1) / kHeadsPerWarp;
+  const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // (row, group of heads)
+  if (unit >= (long long)rows * groups) return;
+  const int row = int(unit / groups), head0 = int(unit % groups) * kHeadsPerWarp + half;
+  __nv_bfloat16* v = x + size_t(row) * ld + size_t(head0) * 128 + l * 8;
+  uint32_t h[kPer][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) h[2 * i] = (unsigned short)(u[i] & 0xFFFFu), h[2 * i + 1] = (unsigned short)(u[i] >> 16);
+  for (int i = 0; i < kPer; ++i) {
+    uint4 raw = make_uint4(0, 0, 0, 0);
+    if (head0 + 2 * i < heads) raw = *reinterpret_cast<const uint4*>(v + i * 256);
+    h[i][0] = raw.x, h[i][1] = raw.y, h[i][2] = raw.z, h[i][3] = raw.w;
   }
-  if (w != nullptr) {
-    float buf[8];
-    float sum_sq = 0.0f;
-    if (active) {
+  // lanes 0-5 hold channels 8 l .. (the low halves), lanes 6-11 their partners j + 48, lanes 12-15 pass through
+  const bool low = l < 6, rotates = l < 12;
+  float c[8], s[8];
+  if constexpr (ROPE) {
+    const size_t at = size_t(row) * 96 + (low ? l : (rotates ? l - 6 : 0)) * 8;
+    if (tables_vec) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        buf[i] = __uint_as_float(unsigned(h[i]) << 16);
-        sum_sq = fmaf(buf[i], buf[i], sum_sq);
+      for (int i = 0; i < 2; ++i) {
+        const float4 c4 = __ldg(reinterpret_cast<const float4*>(cos_tab + at) + i), s4 = __ldg(reinterpret_cast<const float4*>(sin_tab + at) + i);
+        c[4 * i] = c4.x, c[4 * i + 1] = c4.y, c[4 * i + 2] = c4.z, c[4 * i + 3] = c4.w;
+        s[4 * i] = s4.x, s[4 * i + 1] = s4.y, s[4 * i + 2] = s4.z, s[4 * i + 3] = s4.w;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c[i] = __ldg(cos_tab + at + i), s[i] = __ldg(sin_tab + at + i);
+    }
+  }
+  if constexpr (NORM) {
+    float sum[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      sum[i] = 0.0f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        sum[i] = fmaf(bf16_lo(h[i][k]), bf16_lo(h[i][k]), sum[i]);
+        sum[i] = fmaf(bf16_hi(h[i][k]), bf16_hi(h[i][k]), sum[i]);
       }
     }
 #pragma unroll
-    for (int offset = 16; offset > 0; offset >>= 1) sum_sq = __fadd_rn(sum_sq, __shfl_xor_sync(0xFFFFFFFFu, sum_sq, offset));
-    float inv = lane == 0 ? norm_rsqrt(sum_sq, 128, eps) : 0.0f;
-    inv = __shfl_sync(0xFFFFFFFFu, inv, 0);
-    if (active) {
-      const uint4 wr = *reinterpret_cast<const uint4*>(w + lane * 8);
-      const unsigned wu[4] = {wr.x, wr.y, wr.z, wr.w};
+    for (int off = 8; off > 0; off >>= 1)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float wf = __uint_as_float(((wu[i >> 1] >> (16 * (i & 1))) & 0xFFFFu) << 16);
-        h[i] = __bfloat16_as_ushort(__float2bfloat16(__fmul_rn(__fmul_rn(buf[i], inv), wf)));
-      }
+      for (int i = 0; i < kPer; ++i) sum[i] = __fadd_rn(sum[i], __shfl_xor_sync(0xFFFFFFFFu, sum[i], off));
+    // lane l of a half takes the reciprocal of head l % 4 of that half
+    static_assert(kPer == 4, "the selection below");
+    const float even = (l & 2) ? sum[2] : sum[0], odd = (l & 2) ? sum[3] : sum[1];
+    const float mine = (l & 1) ? odd : even;
+    // mean = RNE(sum / 128), the same as the product with the power of two
+    const float inv_mine = rsqrt_q30(__fadd_rn(__fmul_rn(mine, 1.0f / 128.0f), eps));
+    const uint4 wr = __ldg(reinterpret_cast<const uint4*>(w + l * 8));
+    const uint32_t wu[4] = {wr.x, wr.y, wr.z, wr.w};
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const float inv = __shfl_sync(0xFFFFFFFFu, inv_mine, (lane & 16) | i);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        h[i][k] = bf16_pair(__fmul_rn(__fmul_rn(bf16_lo(h[i][k]), inv), bf16_lo(wu[k])), __fmul_rn(__fmul_rn(bf16_hi(h[i][k]), inv), bf16_hi(wu[k])));
     }
   }
-  if (cos_tab != nullptr) {
-    // lanes 0-5 hold channels j = 8*lane .. (the low halves), lanes 6-11 their partners j + 48, lanes 12-15 pass through
-    const bool low = lane < 6, high = lane >= 6 && lane < 12;
-    const int partner = low ? lane + 6 : lane - 6;
-    unsigned short other[8];
+  if constexpr (ROPE) {
+    const int partner = low ? lane + 6 : (rotates ? lane - 6 : lane);
+    constexpr float kMinNormal = 1.17549435e-38f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const unsigned mine = unsigned(h[2 * i]) | (unsigned(h[2 * i + 1]) << 16);
-      const unsigned got = __shfl_sync(0xFFFFFFFFu, mine, partner & 31);
-      other[2 * i] = (unsigned short)(got & 0xFFFFu), other[2 * i + 1] = (unsigned short)(got >> 16);
-    }
-    if (low || high) {
-      const int j0 = (low ? lane : lane - 6) * 8;
-      const float* cr = cos_tab + size_t(row) * 96 + j0;
-      const float* sr = sin_tab + size_t(row) * 96 + j0;
+    for (int i = 0; i < kPer; ++i) {
+      uint32_t o[4], r[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float c = rope_float_value(cr[i]), s = rope_float_value(sr[i]);
-        const float lo = rope_bf16_value(low ? h[i] : other[i]);
-        const float hi = rope_bf16_value(low ? other[i] : h[i]);
-        if (low) {
-          const float left = rope_float_value(__fmul_rn(lo, c)), right = rope_float_value(__fmul_rn(hi, s));
-          h[i] = rope_bf16_result(__fsub_rn(left, right));
-        } else {
-          const float base = rope_float_value(__fmul_rn(hi, c));
-          h[i] = rope_bf16_result(rope_fma_product(lo, s, base));
+      for (int k = 0; k < 4; ++k) o[k] = __shfl_sync(0xFFFFFFFFu, h[i][k], partner);
+      float least = kMinNormal;  // of every magnitude that the reference would canonicalise
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float out[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float xv = e ? bf16_hi(h[i][k]) : bf16_lo(h[i][k]), ov = e ? bf16_hi(o[k]) : bf16_lo(o[k]);
+          const float base = __fmul_rn(xv, c[2 * k + e]), p = __fmul_rn(ov, s[2 * k + e]);
+          out[e] = low ? __fsub_rn(base, p) : fmaf(ov, s[2 * k + e], base);
+          least = fminf(fminf(least, fabsf(base)), fabsf(p));
+          least = fminf(fminf(least, fabsf(xv)), fminf(fabsf(ov), fabsf(out[e])));
         }
+        r[k] = bf16_pair(out[0], out[1]);
+      }
+      if (rotates) {
+        if (least < kMinNormal) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const unsigned short a = rope_channel(low, (unsigned short)(h[i][k] & 0xFFFFu), (unsigned short)(o[k] & 0xFFFFu), c[2 * k], s[2 * k]);
+            const unsigned short b = rope_channel(low, (unsigned short)(h[i][k] >> 16), (unsigned short)(o[k] >> 16), c[2 * k + 1], s[2 * k + 1]);
+            r[k] = unsigned(a) | (unsigned(b) << 16);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) h[i][k] = r[k];
       }
     }
   }
-  if (active) {
-    uint4 o;
-    o.x = unsigned(h[0]) | (unsigned(h[1]) << 16), o.y = unsigned(h[2]) | (unsigned(h[3]) << 16);
-    o.z = unsigned(h[4]) | (unsigned(h[5]) << 16), o.w = unsigned(h[6]) | (unsigned(h[7]) << 16);
-    *reinterpret_cast<uint4*>(v + lane * 8) = o;
-  }
+#pragma unroll
+  for (int i = 0; i < kPer; ++i)
+    if (head0 + 2 * i < heads) *reinterpret_cast<uint4*>(v + i * 256) = make_uint4(h[i][0], h[i][1], h[i][2], h[i][3]);
 }
 }  // namespace
 
@@ -733,8 +785,15 @@ void head_norm_rope(__nv_bfloat16* x, int ld, const __nv_bfloat16* norm_weight, 
   if (ld < heads * 128 || ld % 8 != 0 || reinterpret_cast<uintptr_t>(x) % 16 != 0 ||
       (norm_weight != nullptr && reinterpret_cast<uintptr_t>(norm_weight) % 16 != 0))
     throw std::invalid_argument("head_norm_rope: the row pitch must cover heads * 128 and keep 16-byte alignment");
-  const long long units = (long long)rows * heads;
-  head_norm_rope_kernel<<<unsigned((units + 7) / 8), 256, 0, stream>>>(x, ld, norm_weight, cos_tab, sin_tab, rows, heads, eps);
+  const long long units = (long long)rows * ((heads + kHeadsPerWarp - 1) / kHeadsPerWarp);
+  const int tables_vec = ((reinterpret_cast<uintptr_t>(cos_tab) | reinterpret_cast<uintptr_t>(sin_tab)) & 15) == 0;
+  const unsigned grid = unsigned((units + 7) / 8);
+  if (norm_weight != nullptr && cos_tab != nullptr)
+    head_norm_rope_kernel<true, true><<<grid, 256, 0, stream>>>(x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
+  else if (norm_weight != nullptr)
+    head_norm_rope_kernel<true, false><<<grid, 256, 0, stream>>>(x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
+  else
+    head_norm_rope_kernel<false, true><<<grid, 256, 0, stream>>>(x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
   check_launch("head_norm_rope");
 }
 

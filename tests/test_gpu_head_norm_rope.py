@@ -79,3 +79,22 @@ def test_refusals():
         sfq.check(sfq.lib.sfq_head_norm_rope(sfq.ptr(t), 128, None, None, None, 4, 1, 128, 1e-6, None))
     with pytest.raises(sfq.SfqError, match="row pitch"):
         sfq.check(sfq.lib.sfq_head_norm_rope(sfq.ptr(t), 64, sfq.ptr(t), None, None, 4, 1, 128, 1e-6, None))
+
+
+@pytest.mark.parametrize("rows,heads", [(1, 7), (5, 8), (3, 9), (2, 17)])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_head_groups_and_table_alignment(rows, heads, aligned):
+    # a warp takes eight heads of a row: fewer, exactly eight, one over, two and one; tables that allow 16-byte loads and not
+    x = oracle.to_bf16(oracle.make_data(rows * heads * 128, 91 + heads, 2.0)).reshape(rows, heads * 128)
+    x[0, 128 * (heads - 1):128 * heads - 64] = 0  # a head with zeros among its rotated channels: the step-by-step path
+    w = oracle.to_bf16(1.0 + oracle.make_data(128, 5, 0.2))
+    cos, sin = tables(rows, 13)
+    want = oracle.head_norm_rope(x, heads, w, cos, sin, 1e-6)
+    t, dw = bf16_tensor(x), dev(w)
+    off = 0 if aligned else 1
+    dc, ds = (torch.empty(rows * 96 + off, dtype=torch.float32, device="cuda") for _ in range(2))
+    dc[off:].copy_(dev(cos).view(-1))
+    ds[off:].copy_(dev(sin).view(-1))
+    sfq.check(sfq.lib.sfq_head_norm_rope(sfq.ptr(t), heads * 128, sfq.ptr(dw), dc.data_ptr() + 4 * off, ds.data_ptr() + 4 * off, rows, heads,
+                                         128, 1e-6, sfq.stream_ptr()))
+    assert np.array_equal(bits(t), want)
