@@ -8,9 +8,9 @@
 // and quantize_act_kernel (src/cuda/nvfp4_gemm.cu:107-158). The activation is read
 // once (2 bytes/element, 128-bit loads) and only the quantized form is written.
 //
-// Work split: one CTA per token row, one thread per 16 consecutive elements (one
-// fp4 scale block; 16 threads = one 256-wide rotation group, always inside one
-// warp). The rotation runs two radix-4 stages in registers, transposes the group
+// Work split of the int8 form: one CTA per token row, one thread per 16 consecutive
+// elements (16 threads = one 256-wide rotation group, always inside one
+// warp); the norm without a rotation behind it has a kernel of its own. The rotation runs two radix-4 stages in registers, transposes the group
 // through a padded, conflict-free shared-memory tile, and runs the other two.
 //
 // Bit-exactness notes. The sum of squares is accumulated in the order of the
@@ -34,7 +34,8 @@
 namespace sfq {
 namespace {
 
-enum Mode { kModeInt8 = 0, kModeFp4Ref = 1, kModeFp4Feed = 2, kModeNormOnly = 3, kModeRotOnly = 4 };
+enum Mode { kModeInt8 = 0, kModeRotOnly = 1 };
+enum NormMode { kNormOnly = 0, kNormFp4Ref = 1, kNormFp4Feed = 2 };
 
 struct FusedArgs {
   const __nv_bfloat16* x;
@@ -140,13 +141,6 @@ __device__ __forceinline__ void process_row(const FusedArgs& a, const int row, u
   const int chunks = a.dim >> 4;
   const bool active = tid < chunks;
 
-  if constexpr (MODE == kModeFp4Feed) {
-    if (row >= a.rows) {  // padding rows of the last 128-row scale tile: zero scales
-      if (active) a.scales[nvfp4_scale_offset(row, tid, chunks)] = 0;
-      return;
-    }
-  }
-
   float v[16];
   {
     const __nv_bfloat162* h0 = reinterpret_cast<const __nv_bfloat162*>(&r0);
@@ -236,9 +230,7 @@ __device__ __forceinline__ void process_row(const FusedArgs& a, const int row, u
       dst[1] = o[1];
     }
   }
-  if constexpr (MODE == kModeNormOnly) return;
-
-  if constexpr (MODE == kModeInt8 || MODE == kModeRotOnly) {
+  {
     // ------------------------------------------------------------ ConvRot-256
     if (a.apply_convrot) {
       // Element i = 16*T + e of the group sits at word 17*T + e of the group's tile: a thread's own 16
@@ -318,31 +310,6 @@ __device__ __forceinline__ void process_row(const FusedArgs& a, const int row, u
       }
       reinterpret_cast<uint4*>(a.q + size_t(row) * a.dim)[tid] = make_uint4(o[0], o[1], o[2], o[3]);
     }
-  } else {
-    // ------------------------------------------------------------ per-16 fp4 (src/cuda/nvfp4_gemm.cu:107-158)
-    if (!active) return;
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-    const uint8_t s8 = __nv_cvt_float_to_fp8(amax * (1.0f / 6.0f), __NV_SATFINITE, __NV_E4M3);
-    const float decoded = e4m3_decode(s8);
-    const float inv = decoded > 0.0f ? __fdiv_rn(1.0f, decoded) : 0.0f;
-    uint32_t words[2] = {0, 0};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float even = v[2 * i] * inv, odd = v[2 * i + 1] * inv;
-      // The conversion puts its first component in the low nibble. The reference layout wants the even
-      // element there; the GEMM feed wants it in the high nibble, like the weight files.
-      const __nv_fp4x2_storage_t b = MODE == kModeFp4Ref
-                                         ? __nv_cvt_float2_to_fp4x2(make_float2(even, odd), __NV_E2M1, cudaRoundNearest)
-                                         : __nv_cvt_float2_to_fp4x2(make_float2(odd, even), __NV_E2M1, cudaRoundNearest);
-      words[i >> 2] |= uint32_t(b) << (8 * (i & 3));
-    }
-    reinterpret_cast<uint2*>(a.packed + size_t(row) * (a.dim >> 1))[tid] = make_uint2(words[0], words[1]);
-    if constexpr (MODE == kModeFp4Ref)
-      a.scales[size_t(row) * chunks + tid] = s8;
-    else
-      a.scales[nvfp4_scale_offset(row, tid, chunks)] = s8;
   }
 }
 
@@ -354,7 +321,6 @@ __global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int chunks = a.dim >> 4;
   const bool active = int(threadIdx.x) < chunks;
-  const int total_rows = MODE == kModeFp4Feed ? (a.rows + 127) / 128 * 128 : a.rows;
   auto load = [&](int row, uint4& r0, uint4& r1) {
     r0 = make_uint4(0, 0, 0, 0);
     r1 = r0;
@@ -367,12 +333,204 @@ __global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
   uint4 r0, r1, n0, n1;
   int row = blockIdx.x;
   load(row, r0, r1);
-  for (; row < total_rows; row += gridDim.x) {
+  for (; row < a.rows; row += gridDim.x) {
     load(row + gridDim.x, n0, n1);
     process_row<MODE>(a, row, r0, r1, smem);
     __syncthreads();  // shared memory is reused by the next row
     r0 = n0;
     r1 = n1;
+  }
+}
+
+// ---- RMSNorm [+ modulate], alone or in front of the per-16-block fp4 quantizer ---------------------------------------
+// In the reference's 256-thread block thread v accumulates the squares of the 8-element packs v, v + 256, ... in that order.
+// Here thread t of 128 owns packs t, t + 128, ..., i.e. the virtual threads t and t + 128, and keeps them in registers: the
+// row never goes through shared memory, and a 16-element fp4 block is the packs of two neighbouring threads (one shuffle for
+// its maximum). Bound by instruction issue (3600 warp instructions per 5120-wide row) and by the row's serial part - tree,
+// integer reciprocal, barrier -, not by HBM (2.56 bytes per element). Hence 128 threads, not 256 (the reciprocal is computed
+// by every warp, and 640 packs at dim = 5120 divide evenly), and two rows per CTA: their loads are in flight together, their
+// trees run side by side, their reciprocals are computed in different lanes behind ONE barrier, and the modulation tables
+// (8 bytes per element, from L1 / L2) are read once for rows of the same index. A CTA leaves after its rows; the next one's
+// loads run under the arithmetic of the others on the SM. Measured with modulation, 5120 wide, fp4 out: 75600 rows 375 us
+// (2.64 TB/s), 4747 rows 30 us; the one-row kernel with the row in shared memory took 1018 and 58 us. Not faster: 256 threads
+// (555 us), CTAs that stay with the next rows prefetched and the tables in shared memory (469 us, fewer warps per SM), the
+// reciprocal in warp 0 alone behind a second barrier (407 us).
+constexpr int kNormThreads = 128;
+// Rows a CTA takes at a time: two while a thread's share of a row is at most six packs (dim <= 6144), one beyond that.
+template <int MAXP> constexpr int kNormRows = MAXP <= 6 ? 2 : 1;
+
+// 1 / decode(s8) correctly rounded for the positive e4m3 scales, 0 for scale 0 (and for the NaN code, which is never produced).
+struct E4m3Reciprocals {
+  float v[128];
+  constexpr E4m3Reciprocals() : v() {
+    for (int i = 1; i < 127; ++i) {
+      const int e = i >> 3, m = i & 7;
+      float d = e == 0 ? float(m) : float(8 + m);  // decode = d * 2^(max(e, 1) - 10), exact at every step
+      for (int k = (e == 0 ? 1 : e); k < 10; ++k) d *= 0.5f;
+      for (int k = 10; k < e; ++k) d *= 2.0f;
+      v[i] = 1.0f / d;
+    }
+  }
+};
+__device__ const E4m3Reciprocals kE4m3Reciprocal;
+
+// Eight values -> four bytes of e2m1 pairs. HIGH_EVEN: the even element in the high nibble (GEMM feed), else in the low one.
+template <bool HIGH_EVEN> __device__ __forceinline__ uint32_t e2m1_word(const float (&v)[8]) {
+  uint32_t w;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %1, %2;\n\tcvt.rn.satfinite.e2m1x2.f32 b1, %3, %4;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %5, %6;\n\tcvt.rn.satfinite.e2m1x2.f32 b3, %7, %8;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(w)
+      : "f"(v[HIGH_EVEN ? 0 : 1]), "f"(v[HIGH_EVEN ? 1 : 0]), "f"(v[HIGH_EVEN ? 2 : 3]), "f"(v[HIGH_EVEN ? 3 : 2]),
+        "f"(v[HIGH_EVEN ? 4 : 5]), "f"(v[HIGH_EVEN ? 5 : 4]), "f"(v[HIGH_EVEN ? 6 : 7]), "f"(v[HIGH_EVEN ? 7 : 6]));
+  return w;
+}
+__device__ __forceinline__ uint32_t habs2(uint32_t a) {
+  uint32_t d;
+  asm("abs.bf16x2 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
+__device__ __forceinline__ uint32_t hmax2(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+
+template <int MODE, int MAXP>
+__global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_kernel(const FusedArgs a, int total_rows) {
+  constexpr int R = kNormRows<MAXP>;
+  __shared__ float warp_tot[R][8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int packs = a.dim >> 3, chunks = a.dim >> 4;
+  const int row0 = blockIdx.x * R;
+  if (MODE == kNormFp4Feed && row0 >= a.rows) {  // padding rows of the last 128-row scale tile: zero scales
+    for (int r = 0; r < R && row0 + r < total_rows; ++r)
+      for (int c = tid; c < chunks; c += kNormThreads) a.scales[nvfp4_scale_offset(row0 + r, c, chunks)] = 0;
+    return;
+  }
+  uint4 raw[R][MAXP];
+#pragma unroll
+  for (int j = 0; j < MAXP; ++j)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int p = tid + j * kNormThreads;
+      raw[r][j] = make_uint4(0, 0, 0, 0);
+      if (p < packs && row0 + r < a.rows) raw[r][j] = reinterpret_cast<const uint4*>(a.x + size_t(row0 + r) * a.dim)[p];
+    }
+  int index[R] = {};
+  if (a.mod_scale != nullptr) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) index[r] = __ldg(a.mod_index + min(row0 + r, a.rows - 1));
+  }
+  // sum of squares: the chains of virtual threads t (even packs) and t + 128 (odd ones), the shfl_down tree of their virtual
+  // warps, then the tree over the eight warps' totals
+  float sum[R][2];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    sum[r][0] = sum[r][1] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < MAXP; ++j) {  // absent packs are zeros: fma(0, 0, s) = s
+      const uint32_t u[4] = {raw[r][j].x, raw[r][j].y, raw[r][j].z, raw[r][j].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float lo = __uint_as_float(u[i] << 16), hi = __uint_as_float(u[i] & 0xFFFF0000u);
+        sum[r][j & 1] = __fmaf_rn(lo, lo, sum[r][j & 1]);
+        sum[r][j & 1] = __fmaf_rn(hi, hi, sum[r][j & 1]);
+      }
+    }
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) sum[r][k] = __fadd_rn(sum[r][k], __shfl_down_sync(0xFFFFFFFFu, sum[r][k], off));
+  if (lane == 0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) warp_tot[r][warp] = sum[r][0], warp_tot[r][warp + 4] = sum[r][1];
+  }
+  __syncthreads();
+  // Every warp folds the totals itself: lanes 8 r .. 8 r + 7 hold row r (the reference's steps 16 and 8 add zeros).
+  float tot = warp_tot[(lane >> 3) % R][lane & 7];
+#pragma unroll
+  for (int off = 4; off > 0; off >>= 1) tot = __fadd_rn(tot, __shfl_down_sync(0xFFFFFFFFu, tot, off));
+  const float inv_mine = norm_rsqrt(tot, a.dim, a.eps);
+  float inv[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) inv[r] = __shfl_sync(0xFFFFFFFFu, inv_mine, 8 * r);
+
+#pragma unroll
+  for (int j = 0; j < MAXP; ++j) {
+    const int p = tid + j * kNormThreads;
+    const bool active = p < packs;
+    if (!__any_sync(0xFFFFFFFFu, active)) break;
+    uint4 wr = make_uint4(0, 0, 0, 0);
+    if (active) wr = __ldg(reinterpret_cast<const uint4*>(a.norm_w) + p);
+    const uint32_t wu[4] = {wr.x, wr.y, wr.z, wr.w};
+    ptx::f32x2 sc[4], sh[4];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int row = row0 + r;
+      if (a.mod_scale != nullptr && (r == 0 || index[r] != index[r - 1])) {
+        const size_t at = size_t(index[r]) * a.dim + size_t(active ? p : 0) * 8;
+        const float4* sp = reinterpret_cast<const float4*>(a.mod_scale + at);
+        const float4* hp = reinterpret_cast<const float4*>(a.mod_shift + at);
+        const ptx::f32x2 one = ptx::pack2(1.0f, 1.0f);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float4 s4 = __ldg(sp + i), h4v = __ldg(hp + i);
+          sc[2 * i] = ptx::add2(one, ptx::pack2(s4.x, s4.y)), sc[2 * i + 1] = ptx::add2(one, ptx::pack2(s4.z, s4.w));
+          sh[2 * i] = ptx::pack2(h4v.x, h4v.y), sh[2 * i + 1] = ptx::pack2(h4v.z, h4v.w);
+        }
+      }
+      const uint32_t u[4] = {raw[r][j].x, raw[r][j].y, raw[r][j].z, raw[r][j].w};
+      const ptx::f32x2 inv2 = ptx::pack2(inv[r], inv[r]);
+      uint32_t n[4];  // the normed row rounded to bf16, as the reference stores it
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const ptx::f32x2 x2 = ptx::pack2(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xFFFF0000u));
+        ptx::f32x2 v = ptx::mul2(ptx::mul2(x2, inv2), ptx::pack2(__uint_as_float(wu[i] << 16), __uint_as_float(wu[i] & 0xFFFF0000u)));
+        if (a.mod_scale != nullptr) v = ptx::fma2(v, sc[i], sh[i]);
+        float lo, hi;
+        ptx::unpack2(v, lo, hi);
+        const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
+        n[i] = *reinterpret_cast<const uint32_t*>(&b);
+      }
+      const bool write = active && row < a.rows;
+      if (a.bf16_out != nullptr && write) reinterpret_cast<uint4*>(a.bf16_out + size_t(row) * a.dim)[p] = make_uint4(n[0], n[1], n[2], n[3]);
+      if constexpr (MODE != kNormOnly) {
+        // per-16 fp4 (src/cuda/nvfp4_gemm.cu:107-158): this thread's eight elements and its neighbour's share a scale
+        uint32_t m = hmax2(hmax2(habs2(n[0]), habs2(n[1])), hmax2(habs2(n[2]), habs2(n[3])));
+        m = hmax2(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+        m = hmax2(m, m >> 16);
+        uint32_t s8 = row < a.rows ? uint32_t(__nv_cvt_float_to_fp8(__uint_as_float(m << 16) * (1.0f / 6.0f), __NV_SATFINITE, __NV_E4M3)) : 0u;
+        const float rcp = __ldg(kE4m3Reciprocal.v + s8);
+        const ptx::f32x2 rcp2 = ptx::pack2(rcp, rcp);
+        float q[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          ptx::unpack2(ptx::mul2(ptx::pack2(__uint_as_float(n[i] << 16), __uint_as_float(n[i] & 0xFFFF0000u)), rcp2), q[2 * i], q[2 * i + 1]);
+        if (write) reinterpret_cast<uint32_t*>(a.packed + size_t(row) * (a.dim >> 1))[p] = e2m1_word<MODE == kNormFp4Feed>(q);
+        if constexpr (MODE == kNormFp4Ref) {
+          if (write && (lane & 1) == 0) a.scales[size_t(row) * chunks + (p >> 1)] = uint8_t(s8);
+        } else {
+          // four neighbouring blocks are the four bytes of one word of the tiled layout (dim % 64 == 0: whole words);
+          // the second row of the last pair may be a padding row, whose scales are zero
+          s8 <<= 8 * ((lane >> 1) & 3);
+          s8 |= __shfl_xor_sync(0xFFFFFFFFu, s8, 2);
+          s8 |= __shfl_xor_sync(0xFFFFFFFFu, s8, 4);
+          if (active && (lane & 7) == 0 && row < total_rows) {
+            // 64 blocks further on are 16 tiles of 512 bytes
+            uint8_t* dst = a.scales + nvfp4_scale_offset(row, tid >> 1, chunks) + size_t(j) * (16 * 512);
+            if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0)
+              *reinterpret_cast<uint32_t*>(dst) = s8;
+            else  // an array that starts off a word boundary
+              for (int i = 0; i < 4; ++i) dst[i] = uint8_t(s8 >> (8 * i));
+          }
+        }
+      }
+    }
   }
 }
 
@@ -410,13 +568,17 @@ inline void check_launch(const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-template <int MODE> void launch_fused(const FusedArgs& a, int grid_rows, cudaStream_t stream, const char* what) {
+void check_row_args(const FusedArgs& a, const char* what) {
   if (a.dim % 16 != 0 || a.dim > 16384)
     throw std::invalid_argument(std::string(what) + ": dim must be a multiple of 16 and at most 16384");
   if (reinterpret_cast<uintptr_t>(a.x) % 16 != 0)
     throw std::invalid_argument(std::string(what) + ": activation pointer must be 16-byte aligned");
   if (a.norm_w != nullptr && a.mod_scale != nullptr && (a.mod_shift == nullptr || a.mod_index == nullptr))
     throw std::invalid_argument(std::string(what) + ": modulation needs scale, shift and the row index");
+}
+
+template <int MODE> void launch_fused(const FusedArgs& a, cudaStream_t stream, const char* what) {
+  check_row_args(a, what);
   const int threads = ((a.dim / 16 + 31) / 32) * 32;
   const size_t smem = size_t(threads) * 17 * 4 + (256 + 16) * 4 + (a.norm_w ? size_t(a.dim) * 2 : 0);
   reserve_dynamic_smem(reinterpret_cast<const void*>(&fused_act_kernel<MODE>), smem, what);
@@ -424,8 +586,24 @@ template <int MODE> void launch_fused(const FusedArgs& a, int grid_rows, cudaStr
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_act_kernel<MODE>, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
-  const int grid = std::min(grid_rows, per_sm * device_sm_count());
+  const int grid = std::min(a.rows, per_sm * device_sm_count());
   fused_act_kernel<MODE><<<grid, threads, smem, stream>>>(a);
+  check_launch(what);
+}
+
+// A thread's packs per row decide the registers of the kernel.
+template <int MODE> void launch_norm(const FusedArgs& a, int total_rows, cudaStream_t stream, const char* what) {
+  check_row_args(a, what);
+  const int per_thread = (a.dim / 8 + kNormThreads - 1) / kNormThreads;
+  const auto grid = [&](int r) { return (total_rows + r - 1) / r; };
+  if (per_thread <= 2)
+    norm_rows_kernel<MODE, 2><<<grid(kNormRows<2>), kNormThreads, 0, stream>>>(a, total_rows);
+  else if (per_thread <= 5)
+    norm_rows_kernel<MODE, 5><<<grid(kNormRows<5>), kNormThreads, 0, stream>>>(a, total_rows);
+  else if (per_thread <= 6)
+    norm_rows_kernel<MODE, 6><<<grid(kNormRows<6>), kNormThreads, 0, stream>>>(a, total_rows);
+  else
+    norm_rows_kernel<MODE, 16><<<grid(kNormRows<16>), kNormThreads, 0, stream>>>(a, total_rows);
   check_launch(what);
 }
 
@@ -449,7 +627,7 @@ void rmsnorm(const __nv_bfloat16* x, const NormArgs& norm, __nv_bfloat16* out, i
   if (!x || !out || !norm.weight) throw std::invalid_argument("rmsnorm: null buffer");
   FusedArgs a = base_args(x, norm, rows, dim);
   a.bf16_out = out;
-  launch_fused<kModeNormOnly>(a, rows, stream, "rmsnorm");
+  launch_norm<kNormOnly>(a, rows, stream, "rmsnorm");
 }
 
 void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int group, cudaStream_t stream) {
@@ -463,7 +641,7 @@ void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int 
     FusedArgs a = base_args(x, NormArgs{}, rows, dim);
     a.apply_convrot = 1;
     a.bf16_out = out;
-    launch_fused<kModeRotOnly>(a, rows, stream, "convrot");
+    launch_fused<kModeRotOnly>(a, stream, "convrot");
     return;
   }
   if (group > 256) throw std::runtime_error("convrot: groups above 256 are not supported");
@@ -484,7 +662,7 @@ void quantize_int8_token(const __nv_bfloat16* x, const NormArgs& norm, int8_t* q
   a.row_scale = row_scale;
   a.apply_convrot = apply_convrot ? 1 : 0;
   a.bf16_out = norm.weight ? normed_out : nullptr;
-  launch_fused<kModeInt8>(a, rows, stream, "quantize_int8_token");
+  launch_fused<kModeInt8>(a, stream, "quantize_int8_token");
 }
 
 size_t nvfp4_act_scale_bytes(int rows, int dim) {
@@ -500,17 +678,6 @@ size_t nvfp4_act_scale_bytes(int rows, int dim) {
 // bf16x2 words and the products on packed fp32 pairs. FEED: high nibble = even element, scales in the 128x4-tiled layout
 // with the rows padded to a multiple of 128 (the pad rows' scales are written as zero).
 namespace {
-__device__ __forceinline__ uint32_t habs2(uint32_t a) {
-  uint32_t d;
-  asm("abs.bf16x2 %0, %1;" : "=r"(d) : "r"(a));
-  return d;
-}
-__device__ __forceinline__ uint32_t hmax2(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
-
 template <bool FEED>
 __device__ __forceinline__ void quantize_block16(const uint4 r0, const uint4 r1, uint2& codes, uint8_t& s8) {
   const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};  // element 2i in the low half of word i
@@ -610,14 +777,10 @@ void quantize_nvfp4_block(const __nv_bfloat16* x, const NormArgs& norm, uint8_t*
   a.packed = packed;
   a.scales = scales;
   a.bf16_out = norm.weight ? normed_out : nullptr;
-  if (layout == SFQ_NVFP4_ACT_REFERENCE) {
-    launch_fused<kModeFp4Ref>(a, rows, stream, "quantize_nvfp4_block");
-  } else if (layout == SFQ_NVFP4_ACT_GEMM_FEED) {
-    if (dim % 64 != 0) throw std::invalid_argument("quantize_nvfp4_block: the tiled scale layout needs dim % 64 == 0");
-    launch_fused<kModeFp4Feed>(a, (rows + 127) / 128 * 128, stream, "quantize_nvfp4_block");
-  } else {
-    throw std::invalid_argument("quantize_nvfp4_block: unknown layout");
-  }
+  if (layout == SFQ_NVFP4_ACT_REFERENCE)
+    launch_norm<kNormFp4Ref>(a, rows, stream, "quantize_nvfp4_block");
+  else
+    launch_norm<kNormFp4Feed>(a, (rows + 127) / 128 * 128, stream, "quantize_nvfp4_block");
 }
 
 // ---- head-wise q/k RMSNorm and MM-RoPE, the two steps between the fused projection and attention ----

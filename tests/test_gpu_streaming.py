@@ -312,3 +312,38 @@ def test_pointwise_kernels_match_reference():
     want = x.copy()
     oracle.lib.orc_add_gated_bf16(P(want), P(br), P(gate), P(a), rows, inner)
     assert np.array_equal(bits(dx), want)
+
+
+@pytest.mark.parametrize("rows,dim", [(1, 64), (3, 192), (2, 2048), (131, 2112), (5, 5120), (4, 6144), (3, 6208), (1, 16384)])
+@pytest.mark.parametrize("modulate", [False, True])
+def test_norm_in_front_of_the_fp4_quantizer(rows, dim, modulate):
+    # rows per CTA and packs per thread of the norm kernel at their edges: one, three and more packs, odd row counts, padding rows
+    rng = np.random.default_rng(rows + dim)
+    x = gaussian_bf16((rows, dim), seed=rows + dim, outliers=True)
+    w = oracle.to_bf16((1.0 + 0.1 * rng.standard_normal(dim)).astype(np.float32))
+    scale, shift = (0.1 * rng.standard_normal((2, 3, dim))).astype(np.float32)
+    a = (np.arange(rows) // 2 % 3).astype(np.int32)  # rows of one CTA with the same index and with different ones
+    d = [bf16_tensor(w), dev(scale), dev(shift), dev(a)]
+    norm = sfq.Norm(sfq.ptr(d[0]), *([sfq.ptr(t) for t in d[1:]] if modulate else [None] * 3), 1e-5)
+    dx = bf16_tensor(x)
+    n = oracle.rmsnorm_bf16(x, w, 1e-5, *((scale, shift, a) if modulate else ()))
+    wp, ws, _ = oracle.nvfp4_quantize_act(n)
+    packed = torch.empty((rows, dim // 2), dtype=torch.uint8, device="cuda")
+    scales = torch.empty((rows, dim // 16), dtype=torch.uint8, device="cuda")
+    normed = torch.empty_like(dx)
+    sfq.check(sfq.lib.sfq_quantize_nvfp4_block(sfq.ptr(dx), C.byref(norm), sfq.ptr(packed), sfq.ptr(scales), sfq.ptr(normed), rows, dim,
+                                               sfq.NVFP4_ACT_REFERENCE, S))
+    assert np.array_equal(bits(normed), n) and np.array_equal(_u8(packed), wp) and np.array_equal(_u8(scales), ws)
+    nb = sfq.lib.sfq_nvfp4_act_scale_bytes(rows, dim)
+    for shift_bytes in (0, 1):
+        fs = torch.full((nb + 4,), 0x55, dtype=torch.uint8, device="cuda")
+        sfq.check(sfq.lib.sfq_quantize_nvfp4_block(sfq.ptr(dx), C.byref(norm), sfq.ptr(packed), fs.data_ptr() + shift_bytes, None, rows, dim,
+                                                   sfq.NVFP4_ACT_GEMM_FEED, S))
+        assert np.array_equal(_u8(packed), ((wp << 4) | (wp >> 4)).astype(np.uint8))
+        tiled = np.zeros(nb, np.uint8)
+        for r in range(rows):
+            for b in range(dim // 16):
+                tiled[oracle.lib.orc_nvfp4_scale_slot(r, b, dim // 16)] = ws[r, b]
+        got = _u8(fs)
+        assert np.array_equal(got[shift_bytes:shift_bytes + nb], tiled)
+        assert (got[:shift_bytes] == 0x55).all() and (got[shift_bytes + nb:] == 0x55).all()
