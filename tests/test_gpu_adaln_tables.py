@@ -89,6 +89,26 @@ def test_forward_f32_against_the_fp64_product(fmt, rows, n, k):
         assert np.abs(ry.cpu().numpy() - got).max() <= 2e-6 * k * np.abs(x).max() * np.abs(w).max() + 1e-6
 
 
+@pytest.mark.parametrize("fmt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,n,k", [(1, 5, 4), (3, 2368, 516), (4, 2371, 5120), (5, 3000, 1000), (8, 30, 512), (9, 2400, 516), (16, 2369, 2052),
+                                      (17, 2500, 132), (64, 2500, 1024), (65, 300, 256), (3, 300, 258)])
+def test_forward_f32_row_tiles(fmt, rows, n, k):
+    """Every row tile (1, 4, 8, 16), one and four features per CTA, ragged ends of all three extents, and the tiled kernel behind
+    them (more than 64 rows, K not in fours). Bound: (K / 256 + 16) additions of fp32 terms, each rounding by 2^-24 of the sum of
+    the terms' magnitudes at most."""
+    g = torch.Generator("cuda").manual_seed(rows + n)
+    x = torch.randn((rows, k), device="cuda", generator=g)
+    w = torch.randn((n, k), device="cuda", generator=g).mul_(0.05).to(fmt)
+    bias = torch.randn(n, device="cuda", generator=g)
+    weight = sfq.new_weight(format=sfq.F32 if fmt == torch.float32 else sfq.BF16, data=sfq.ptr(w), out_features=n, in_features=k,
+                            bias=sfq.ptr(bias), bias_format=sfq.F32)
+    got = sfq.LinearRunner().forward_f32(weight, x)
+    want = x.double() @ w.double().T + bias.double()
+    terms = x.double().abs() @ w.double().abs().T + bias.double().abs()
+    steps = (k / 256 + 16) if rows <= 64 and k % 4 == 0 else k + 1
+    assert bool(((got.double() - want).abs() <= steps * 2.0 ** -24 * terms).all())
+
+
 def test_forward_f32_refuses_what_it_does_not_build():
     t = torch.zeros(256 * 256, dtype=torch.float32, device="cuda")
     runner = sfq.LinearRunner()
