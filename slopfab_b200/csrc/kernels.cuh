@@ -89,6 +89,11 @@ void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k,
                        int seq_q, int seq_kv, int heads, int kv_heads, int head_dim, float scale, void* workspace, size_t workspace_bytes,
                        cudaStream_t stream);
 
+// LoRA side branch in one launch (lora_kernel.cu): y[rows,out] += bf16(bf16(x a^T) b^T), a [rank,in], b [out,rank]; false,
+// with nothing launched, when rank > 128, a width is no multiple of 8 or an operand is not 16-byte aligned.
+bool lora_fused(const __nv_bfloat16* x, const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* y, int rows, int in, int out, int rank,
+                cudaStream_t stream);
+
 // Head-wise RMSNorm (norm_weight [128], may be null) and MM-RoPE (cos / sin fp32 [rows, 96], may be null) in place on
 // x [rows, heads, 128] with a row pitch of ld elements.
 void head_norm_rope(__nv_bfloat16* x, int ld, const __nv_bfloat16* norm_weight, const float* cos_tab, const float* sin_tab, int rows,

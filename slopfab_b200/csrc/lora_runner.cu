@@ -12,6 +12,7 @@
 
 #include "codec.cuh"
 #include "gemm_tc.cuh"
+#include "kernels.cuh"
 #include "runtime.h"
 
 namespace slopfab::cuda {
@@ -114,6 +115,7 @@ void LoraRunner::apply(const void* key, const __nv_bfloat16* input, int rows, __
   if (found == factors_.end() || rows <= 0) return;
   if (input == nullptr || output == nullptr) throw std::invalid_argument("LoRA: null activation");
   for (const auto& f : found->second) {
+    if (sfq::lora_fused(input, f.a_ptr, f.b_ptr, output, rows, f.in, f.out, f.rank, stream)) continue;
     for (int row = 0; row < rows; row += kRows) {
       const int count = std::min(kRows, rows - row);
       sfq::GemmArgs down;  // hidden = x A^T

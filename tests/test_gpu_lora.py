@@ -52,6 +52,32 @@ def test_lora_apply_matches_the_reference_statement(rows, k, rank, out_total, of
     assert sfq.device_status() == 0
 
 
+@pytest.mark.parametrize("rows,k,rank,out", [
+    (1, 512, 4, 512), (31, 520, 32, 40), (33, 1032, 33, 1000), (64, 4104, 64, 520), (95, 2048, 65, 2056), (300, 512, 128, 13824),
+    (4737, 520, 16, 264),   # more row tiles than SMs: no split of the features
+    (200, 512, 136, 512),   # past the one-launch kernel: two GEMMs
+    (200, 512, 8, 500),     # an output width that is no multiple of 8: two GEMMs
+])
+def test_lora_in_one_launch(rows, k, rank, out):
+    """Ragged rows, widths and ranks against fp64 on the stored factors. Three bf16 roundings, each by 2^-8 of its value at most:
+    the hidden row and the delta (both within the sum of the delta's terms) and the result."""
+    g = torch.Generator("cuda").manual_seed(rows + k)
+    x = torch.randn((rows, k), device="cuda", generator=g).to(torch.bfloat16)
+    a = (torch.randn((rank, k), generator=torch.Generator().manual_seed(1)) / k ** 0.5).float().numpy()
+    b = (0.1 * torch.randn((out, rank), generator=torch.Generator().manual_seed(2))).float().numpy()
+    y0 = torch.randn((rows, out), device="cuda", generator=g).to(torch.bfloat16)
+    runner = LoraRunner()
+    runner.attach(1, a, b)
+    y = y0.clone()
+    runner.apply(1, x, y)
+    da, db = (torch.from_numpy(t).cuda().to(torch.bfloat16).double() for t in (a, b))
+    hidden = x.double() @ da.T
+    want = y0.double() + hidden @ db.T
+    slack = 1.01 * 2.0 ** -8 * (2 * hidden.abs() @ db.abs().T + want.abs()) + 1e-5
+    assert bool(((y.double() - want).abs() <= slack).all())
+    assert sfq.device_status() == 0
+
+
 def test_two_factor_pairs_and_staged_upload():
     rows, k, out = 200, 256, 256
     x, a1, b1 = case(rows, k, 16, out, 1)
