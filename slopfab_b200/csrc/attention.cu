@@ -10,12 +10,12 @@
 //               [128 d x 128 keys]; V is transposed once per call by transpose_v_kernel so that both products are
 //               K-major x K-major, the operand form the GEMM kernels already use
 //   warp 1      issues, per key tile j: O0 += P0(j) V(j), S0 = Q0 K(j+1)^T, O1 += P1(j) V(j), S1 = Q1 K(j+1)^T (8 MMAs
-//               128x128x16 each). S and O of both query tiles live in TMEM (4 x 128 columns); P is read by the second
+//               128x128x16 each; the product with V in two parts, as its probabilities arrive). S and O of both query tiles live in TMEM (4 x 128 columns); P is read by the second
 //               product straight from TMEM, where it overwrites the first 64 columns of the scores it was computed from
 //   warps 4-7   softmax of query tile 0, warps 8-11 of query tile 1 (warps 2-3 only hand their registers over: the
 //               softmax warpgroups run with 216 registers, the first warpgroup with 56), one query row per thread with all 128 keys of the
 //               tile: S from TMEM, P = exp2(s - m) as bf16 pairs back into TMEM, the running sum, and - only when the
-//               tile's probabilities sum to more than 2^15, i.e. the row has outgrown the reference maximum m the
+//               part's probabilities sum to more than 2^15, i.e. the row has outgrown the reference maximum m the
 //               accumulator was last scaled to - the true running maximum, a rescale of O in TMEM and the tile's
 //               probabilities again. A stale reference changes nothing in exact arithmetic (numerator and denominator
 //               carry the same factor); the limit keeps every p far inside the range of bf16 and fp32, and no maximum over
@@ -48,7 +48,7 @@ constexpr int kAttnRegsLean = 56, kAttnRegsSoftmax = 216;  // after setmaxnreg: 
 constexpr float kTileSumLimit = 32768.0f;  // a key tile's 128 probabilities may sum to this before the reference maximum moves
 
 struct AttnShared {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_full[2], pv_done[2];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_part[2], p_full[2], pv_part[2], pv_done[2];
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -115,6 +115,11 @@ __device__ __forceinline__ f32x2 exp2_pair_fma(f32x2 x) {
   unpack2(t, t0, t1);
   return pack2(__int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23)), __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23)));
 }
+// A query tile's probabilities are handed to the second product in two parts: the first kFirstChunks chunks of 32 keys, then
+// the rest, so that most of O += P V runs under the last chunk's exponentials instead of behind them. A query tile's own chain
+// (scores -> softmax -> product -> next scores) is what bounds the kernel, not the tensor pipe. 40 heads, 18900 / 4747 tokens:
+// one part 6.00 / 0.534 ms, three chunks first 5.83 / 0.505 ms, two chunks first 5.93 / 0.517 ms.
+constexpr int kFirstChunks = 3;
 constexpr int kFmaPairsOfFour = 1;  // of every four pairs of probabilities, how many take the FMA-pipe exponential
 
 __global__ void __launch_bounds__(kAttnThreads, 1)
@@ -141,8 +146,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       mbar_init(smem_u32(&sh->v_full[i]), 1);
       mbar_init(smem_u32(&sh->v_empty[i]), 1);
       mbar_init(smem_u32(&sh->s_full[i]), 1);   // per query tile: the scores of the current key tile are in TMEM
-      mbar_init(smem_u32(&sh->p_full[i]), 4);   // per query tile: its four softmax warps have written P (and rescaled O)
-      mbar_init(smem_u32(&sh->pv_done[i]), 1);  // per query tile: O += P V of the current key tile has completed
+      mbar_init(smem_u32(&sh->p_part[i]), 4);   // per query tile: its four softmax warps have written P of the first chunks (and rescaled O)
+      mbar_init(smem_u32(&sh->p_full[i]), 4);   // per query tile: ... of the remaining chunks
+      mbar_init(smem_u32(&sh->pv_part[i]), 1);  // per query tile: O += P V over the first chunks' keys has completed
+      mbar_init(smem_u32(&sh->pv_done[i]), 1);  // per query tile: O += P V of the last key tile has completed
     }
     sh->abort = 0;
     fence_barrier_init();
@@ -208,21 +215,39 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       __syncwarp();
       return true;
     };
-    auto issue_pv = [&](int t, int j) {  // O_t += P_t V_j: A = P_t in tensor memory [queries x keys], B = V^T [d x keys]
+    // O_t += P_t V_j in two parts: the keys of the first chunks of probabilities as soon as those are written, the rest
+    // when the last chunk is. A = P_t in tensor memory [queries x keys], 16 keys (eight 32-bit columns of bf16 pairs) per
+    // MMA; B = V^T [d x keys].
+    auto issue_pv = [&](int t, int j, bool more) {
       const int st = j & 1;
+      const uint32_t d = tmem + 2 * kTile + t * kTile, a = tmem + t * kTile;
+      const uint64_t b0 = smem_desc_sw128(smem_u32(v_s + st * kTileBytes)), b1 = b0 + (kSlab >> 4);
       if (t == 0 && !wait(&sh->v_full[st], (j >> 1) & 1, 16)) return false;
-      if (!wait(&sh->p_full[t], j & 1, 17)) return false;
+      if (!wait(&sh->p_part[t], j & 1, 17)) return false;
       tc_fence_after_sync();
-      if (elect_one())  // 16 keys per MMA: eight 32-bit columns of bf16 pairs
-        mma_f16_ts_x8_commit(tmem + 2 * kTile + t * kTile, tmem + t * kTile, smem_desc_sw128(smem_u32(v_s + st * kTileBytes)), idesc,
-                             j ? 1u : 0u, kSlab >> 4, smem_u32(&sh->pv_done[t]), smem_u32(&sh->v_empty[st]), t == 1 ? 1u : 0u);
+      if (elect_one()) {
+        mma_f16_ts_x4(d, a, b0, idesc, j ? 1u : 0u);
+        if (kFirstChunks == 3) mma_f16_ts_x2(d, a + 32, b1, idesc, 1u);
+        tc_commit(smem_u32(&sh->pv_part[t]));
+      }
+      __syncwarp();
+      if (!wait(&sh->p_full[t], j & 1, 19)) return false;
+      tc_fence_after_sync();
+      if (elect_one()) {
+        if (kFirstChunks == 3)
+          mma_f16_ts_x2(d, a + 48, b1 + 4, idesc, 1u);
+        else
+          mma_f16_ts_x4(d, a + 32, b1, idesc, 1u);
+        if (t == 1) tc_commit(smem_u32(&sh->v_empty[st]));
+        if (!more) tc_commit(smem_u32(&sh->pv_done[t]));
+      }
       __syncwarp();
       return true;
     };
     if (ok) ok = issue_s(0, 0) && issue_s(1, 0);
     for (int j = 0; j < tiles && ok; ++j) {
       const bool more = j + 1 < tiles;
-      ok = issue_pv(0, j) && (!more || issue_s(0, j + 1)) && issue_pv(1, j) && (!more || issue_s(1, j + 1));
+      ok = issue_pv(0, j, more) && (!more || issue_s(0, j + 1)) && issue_pv(1, j, more) && (!more || issue_s(1, j + 1));
     }
   }
   } else {
@@ -243,7 +268,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     uint32_t r[4][32];
     const f32x2 scale2 = pack2(g.scale_log2, g.scale_log2);
     // p = 2^(s * scale - m) for the 32 keys of chunk c as bf16 pairs, written over columns [16 c, 16 c + 16) of the
-    // scores they came from (those columns belong to chunks 0 and 1, which are in registers by then); returns their sum.
+    // scores they came from (chunk 0's columns or, later, ones that are in registers by then); returns their sum.
     auto emit_chunk = [&](int c, float m, f32x2 sum2) {
       const f32x2 negm2 = pack2(-m, -m);
       uint32_t pk[16];
@@ -280,62 +305,96 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         for (int k = 0; k < 4; ++k) m4[k] = max3(m4[k], __uint_as_float(r[c][i + 2 * k]), __uint_as_float(r[c][i + 2 * k + 1]));
       return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
     };
+    // The reference maximum becomes m_new in the rows that outgrew it; O and the running sum follow (the TMEM accesses are
+    // warp-wide; rows within their limit use a factor of 1). O_t has to be at rest.
+    auto move_reference = [&](float m_new, bool rescale) {
+      if (rescale) {
+        const float f = m_new == m_used ? 1.0f : fast_exp2(m_used - m_new);
+        l *= f;
+        uint32_t o[32];
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          tmem_ld_32x32(tmem_o + c * 32, o);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+          tmem_st_32x32(tmem_o + c * 32, o);
+        }
+      }
+      m_used = m_new;
+    };
+    auto publish = [&](uint64_t* bar) {
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(bar));
+    };
+    auto total = [&](f32x2 sum2) {
+      float a, b;
+      unpack2(sum2, a, b);
+      return a + b;
+    };
     for (int j = 0; j < tiles; ++j) {
       if (!(ok = __all_sync(0xffffffffu, attn_wait<40>(smem_u32(&sh->s_full[t]), j & 1, sh, g.status, 18)))) break;
       tc_fence_after_sync();
       const int valid = g.seq_kv - j * kTile;  // keys of this tile that exist
       // The probabilities are computed against the reference maximum the accumulator was last scaled to, which is known
-      // before the tile arrives: chunk c is exponentiated while chunk c + 1 is still on its way out of tensor memory. No
+      // before the tile arrives: chunk 0 is exponentiated while the others are still on their way out of tensor memory. No
       // maximum is taken on this path: that the reference is still good enough is read off the tile's sum of probabilities.
       f32x2 sum2 = pack2(0.0f, 0.0f);
       tmem_ld_32x32(tmem_s, r[0]);
+      tmem_ld_wait();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        tmem_ld_wait();
-        if (c + 1 < 4) tmem_ld_32x32(tmem_s + (c + 1) * 32, r[c + 1]);
+      for (int c = 1; c < 4; ++c) tmem_ld_32x32(tmem_s + c * 32, r[c]);
+      if (valid < kTile) mask_chunk(0, valid);
+      if (j > 0) sum2 = emit_chunk(0, m_used, sum2);
+      tmem_ld_wait();  // every score is in registers, so P may overwrite any of the columns they came from
+#pragma unroll
+      for (int c = 1; c < 4; ++c)
         if (valid < kTile) mask_chunk(c, valid);
-        if (j > 0) sum2 = emit_chunk(c, m_used, sum2);
-      }
-      float sum0, sum1;
-      unpack2(sum2, sum0, sum1);
-      float tile_sum = sum0 + sum1;
-      const bool over = j == 0 || !(tile_sum <= kTileSumLimit);  // the first tile; a row that outgrew its reference; inf or NaN
+      if (j > 0)
+#pragma unroll
+        for (int c = 1; c < kFirstChunks; ++c) sum2 = emit_chunk(c, m_used, sum2);
+      float part_sum = total(sum2);
+      bool over = j == 0 || !(part_sum <= kTileSumLimit);  // the first tile; a row that outgrew its reference; inf or NaN
       if (__any_sync(0xffffffffu, over)) {
         // Rare after the first tiles. The reference becomes the running maximum. S_t(j) was issued behind O_t += P_t V(j-1),
-        // so its completion says that O_t is at rest. The warp rescales its 32 rows together (the TMEM accesses are
-        // warp-wide; rows within their limit use a factor of 1) and computes the tile's probabilities again against the new
-        // reference -- every score is still in registers -- over the ones just written.
+        // so its completion says that O_t is at rest. The probabilities are computed again against the new reference --
+        // every score is still in registers -- over the ones just written.
         float mx = -INFINITY;
 #pragma unroll
         for (int c = 0; c < 4; ++c) mx = fmaxf(mx, chunk_max(c));
-        const float m_new = over ? fmaxf(m_used, mx * g.scale_log2) : m_used;  // scale > 0: the maximum commutes with it
-        if (j > 0) {
-          const float f = over ? fast_exp2(m_used - m_new) : 1.0f;
-          l *= f;
-          uint32_t o[32];
-#pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            tmem_ld_32x32(tmem_o + c * 32, o);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-            tmem_st_32x32(tmem_o + c * 32, o);
-          }
-        }
-        m_used = m_new;
+        move_reference(over ? fmaxf(m_used, mx * g.scale_log2) : m_used, j > 0);  // scale > 0: the maximum commutes with it
         sum2 = pack2(0.0f, 0.0f);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) sum2 = emit_chunk(c, m_used, sum2);
-        unpack2(sum2, sum0, sum1);
-        tile_sum = sum0 + sum1;
+        for (int c = 0; c < kFirstChunks; ++c) sum2 = emit_chunk(c, m_used, sum2);
+        part_sum = total(sum2);
       }
-      l += tile_sum;
-      tmem_st_wait();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sh->p_full[t]));
+      l += part_sum;
+      publish(&sh->p_part[t]);
+      sum2 = pack2(0.0f, 0.0f);
+#pragma unroll
+      for (int c = kFirstChunks; c < 4; ++c) sum2 = emit_chunk(c, m_used, sum2);
+      part_sum = total(sum2);
+      over = !(part_sum <= kTileSumLimit);
+      if (__any_sync(0xffffffffu, over)) {
+        // The last keys outgrew the reference after the first part's product was released: O_t is at rest again when that
+        // product has completed (the issuer waits for the rest of P before it touches O_t).
+        if (!(ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_part[t]), j & 1, sh, g.status, 21)))) break;
+        tc_fence_after_sync();
+        float mx = -INFINITY;
+#pragma unroll
+        for (int c = kFirstChunks; c < 4; ++c) mx = fmaxf(mx, chunk_max(c));
+        move_reference(over ? fmaxf(m_used, mx * g.scale_log2) : m_used, true);
+        sum2 = pack2(0.0f, 0.0f);
+#pragma unroll
+        for (int c = kFirstChunks; c < 4; ++c) sum2 = emit_chunk(c, m_used, sum2);
+        part_sum = total(sum2);
+      }
+      l += part_sum;
+      publish(&sh->p_full[t]);
     }
-    if (ok && (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_done[t]), (tiles - 1) & 1, sh, g.status, 20)))) {
+    if (ok && (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_done[t]), 0, sh, g.status, 20)))) {
       tc_fence_after_sync();
       const float inv = 1.0f / l;
       const int qrow = q0 + t * kTile + row;

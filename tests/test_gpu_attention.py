@@ -95,6 +95,18 @@ def test_running_maximum_that_keeps_growing():
     assert sfq.device_status() == 0
 
 
+@pytest.mark.parametrize("spike", [0, 33, 95, 96, 127, 128 + 31, 128 + 95, 128 + 96, 128 + 127, 256 + 110, 399])
+def test_one_key_that_outgrows_the_reference(spike):
+    """One key raises some rows' scores by more than 2^15 in base-2 units of probability: the reference maximum moves inside that
+    key tile, before the tile's first part of probabilities is handed over or after it, with the accumulator rescaled either way."""
+    seq, heads = 400, 2
+    q, k, v = data(seq, heads, 81, 1.0), data(seq, heads, 82, 0.3), data(seq, heads, 83, 1.0)
+    k[spike] = oracle.from_bf16(oracle.to_bf16((4.0 * np.where(q[spike // 2] < 0, -1.0, 1.0)).astype(np.float32)))
+    scores = (q[:, :D] @ k[:, :D].T) / np.sqrt(D) * np.log2(np.e)
+    assert scores[spike // 2, spike] - np.delete(scores[spike // 2], spike).max() > 16
+    run_case(q, k, v, heads, heads)
+
+
 def test_against_torch_on_a_longer_sequence():
     torch.manual_seed(5)
     seq, heads = 4096 + 77, 4
