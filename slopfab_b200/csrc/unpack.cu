@@ -265,11 +265,80 @@ unpack_nf4_kernel(const uint8_t* __restrict__ src, const uint8_t* __restrict__ a
   }
 }
 
+// The same for block sizes that are a multiple of 16 over an even count of whole 16s (every real file: 64 and 4096): one scale
+// per thread, an 8-byte load, two 16-byte stores, where the kernel above moves one byte and two elements per thread. The 16
+// table entries lie in 16 different banks, so the lookups are conflict-free whatever the codes.
+template <class T>
+__global__ void __launch_bounds__(kThreads)
+unpack_nf4_vec_kernel(const uint8_t* __restrict__ src, const uint8_t* __restrict__ absmax, const float* __restrict__ map,
+                      const float* __restrict__ nested_map, const float* __restrict__ nested_absmax, unsigned chunks_per_block,
+                      unsigned nested_block, float offset, T* __restrict__ dst, unsigned chunks) {
+  __shared__ float lut[16];
+  if (threadIdx.x < 16) lut[threadIdx.x] = map[threadIdx.x];
+  __syncthreads();
+  const unsigned c = blockIdx.x * unsigned(kThreads) + threadIdx.x;  // 16 elements
+  if (c >= chunks) return;
+  const unsigned b = c / chunks_per_block;
+  const float scale = __fmaf_rn(__ldg(nested_map + __ldg(absmax + b)), __ldg(nested_absmax + b / nested_block), offset);
+  const uint2 raw = __ldg(reinterpret_cast<const uint2*>(src) + c);
+  const uint32_t words[2] = {raw.x, raw.y};
+  alignas(16) T o[16];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t byte = (words[i >> 2] >> (8 * (i & 3))) & 0xFFu;
+    o[2 * i] = narrow_to<T>(lut[byte >> 4] * scale);
+    o[2 * i + 1] = narrow_to<T>(lut[byte & 15u] * scale);
+  }
+  uint4* d = reinterpret_cast<uint4*>(dst) + size_t(c) * 2;
+  d[0] = *reinterpret_cast<const uint4*>(o);
+  d[1] = *reinterpret_cast<const uint4*>(o + 8);
+}
+
+// Eight elements per thread for aligned buffers; the tail of a count that is no multiple of eight goes through to_bf16_kernel.
+// 13824 x 5120 fp16: 45 us (one element per thread 180).
+template <class T> __global__ void __launch_bounds__(kThreads) to_bf16_vec_kernel(const T* __restrict__ src, uint4* __restrict__ dst, size_t packs) {
+  const size_t p = size_t(blockIdx.x) * kThreads + threadIdx.x;
+  if (p >= packs) return;
+  constexpr int kLoads = sizeof(T) / 2;
+  uint4 raw[kLoads];
+#pragma unroll
+  for (int i = 0; i < kLoads; ++i) raw[i] = __ldg(reinterpret_cast<const uint4*>(src) + p * kLoads + i);
+  const T* v = reinterpret_cast<const T*>(raw);
+  uint4 o;
+  __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) op[i] = __floats2bfloat162_rn(float(v[2 * i]), float(v[2 * i + 1]));
+  dst[p] = o;
+}
+
 template <class T> __global__ void __launch_bounds__(kThreads) to_bf16_kernel(const T* __restrict__ src, __nv_bfloat16* __restrict__ dst, size_t n) {
   const size_t i = size_t(blockIdx.x) * kThreads + threadIdx.x;
   if (i < n) dst[i] = __float2bfloat16(float(src[i]));
 }
 
+}  // namespace
+
+namespace {
+template <class T>
+void launch_nf4(const uint8_t* src, const uint8_t* absmax, const float* map, const float* nested_map, const float* nested_absmax, int block,
+                int nested_block, float offset, T* dst, size_t n, cudaStream_t stream) {
+  const bool aligned = reinterpret_cast<uintptr_t>(src) % 8 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0;
+  if (block % 16 == 0 && n % 16 == 0 && n / 16 < (size_t(1) << 32) - kThreads && aligned)
+    unpack_nf4_vec_kernel<T><<<blocks_for(n / 16, kThreads), kThreads, 0, stream>>>(src, absmax, map, nested_map, nested_absmax, unsigned(block / 16),
+                                                                                   unsigned(nested_block), offset, dst, unsigned(n / 16));
+  else
+    unpack_nf4_kernel<T><<<blocks_for((n + 1) / 2, kThreads), kThreads, 0, stream>>>(src, absmax, map, nested_map, nested_absmax, block, nested_block,
+                                                                                     offset, dst, n);
+}
+
+template <class T> void launch_to_bf16(const T* src, __nv_bfloat16* dst, size_t n, cudaStream_t stream) {
+  size_t done = 0;
+  if (reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0 && n >= 8) {
+    to_bf16_vec_kernel<T><<<blocks_for(n / 8, kThreads), kThreads, 0, stream>>>(src, reinterpret_cast<uint4*>(dst), n / 8);
+    done = n / 8 * 8;
+  }
+  if (done < n) to_bf16_kernel<T><<<blocks_for(n - done, kThreads), kThreads, 0, stream>>>(src + done, dst + done, n - done);
+}
 }  // namespace
 
 void unpack_f8e4m3_bf16(const uint8_t* src, const float* scale, __nv_bfloat16* dst, size_t n, cudaStream_t stream) {
@@ -287,8 +356,7 @@ void unpack_nf4_bf16(const uint8_t* src, const uint8_t* absmax, const float* map
     throw std::runtime_error("linear: nf4 weight without complete double-quant state");
   if (block <= 0 || nested_block <= 0) throw std::invalid_argument("unpack_nf4: block sizes must be positive");
   const size_t n = size_t(out_features) * in_features;
-  unpack_nf4_kernel<__nv_bfloat16><<<blocks_for((n + 1) / 2, kThreads), kThreads, 0, stream>>>(src, absmax, map, nested_map, nested_absmax,
-                                                                                              block, nested_block, offset, dst, n);
+  launch_nf4(src, absmax, map, nested_map, nested_absmax, block, nested_block, offset, dst, n, stream);
   check_launch("unpack_nf4");
 }
 
@@ -300,20 +368,19 @@ void unpack_nf4_f16(const uint8_t* src, const uint8_t* absmax, const float* map,
   if (!src || !absmax || !map || !nested_map || !nested_absmax || !dst)
     throw std::runtime_error("linear: nf4 weight without complete double-quant state");
   if (block <= 0 || nested_block <= 0) throw std::invalid_argument("unpack_nf4: block sizes must be positive");
-  unpack_nf4_kernel<__half><<<blocks_for((n + 1) / 2, kThreads), kThreads, 0, stream>>>(src, absmax, map, nested_map, nested_absmax, block,
-                                                                                       nested_block, offset, dst, n);
+  launch_nf4(src, absmax, map, nested_map, nested_absmax, block, nested_block, offset, dst, n, stream);
   check_launch("unpack_nf4_f16");
 }
 
 void convert_f16_bf16(const __half* src, __nv_bfloat16* dst, size_t n, cudaStream_t stream) {
   if (n == 0) return;
-  to_bf16_kernel<__half><<<blocks_for(n, kThreads), kThreads, 0, stream>>>(src, dst, n);
+  launch_to_bf16(src, dst, n, stream);
   check_launch("convert_f16_bf16");
 }
 
 void convert_f32_bf16(const float* src, __nv_bfloat16* dst, size_t n, cudaStream_t stream) {
   if (n == 0) return;
-  to_bf16_kernel<float><<<blocks_for(n, kThreads), kThreads, 0, stream>>>(src, dst, n);
+  launch_to_bf16(src, dst, n, stream);
   check_launch("convert_f32_bf16");
 }
 

@@ -82,6 +82,39 @@ def test_nf4_unpack_bit_exact(out_f, in_f, block, nested):
         assert np.array_equal(bits(r), want)
 
 
+@pytest.mark.parametrize("shift", [0, 1])  # elements off a 16-byte boundary: the wide kernels, and the narrow ones behind them
+@pytest.mark.parametrize("n", [1, 7, 8, 1000, 4096 * 8 + 5])
+def test_float_conversion_and_pre_scale_at_odd_sizes_and_offsets(n, shift):
+    g = torch.Generator("cuda").manual_seed(n)
+    src = torch.randn(n + 8, device="cuda", generator=g)
+    for fmt, t in ((sfq.F16, src.half()), (sfq.F32, src)):
+        w = sfq.new_weight(format=fmt, data=sfq.ptr(t) + shift * t.element_size(), out_features=1, in_features=n)
+        runner = sfq.LinearRunner()
+        prepared, used = runner.prepare(w, 1)
+        assert used >= 2 * n and prepared == sfq.ptr(runner._ws) + (-sfq.ptr(runner._ws)) % 256
+        got = runner._ws[prepared - sfq.ptr(runner._ws):][:2 * n].view(torch.bfloat16)
+        assert torch.equal(got, t[shift:shift + n].to(torch.bfloat16))
+    x, s = (torch.randn(3 * n + 8, device="cuda", generator=g).to(torch.bfloat16) for _ in range(2))
+    out = torch.zeros(3 * n + 8, dtype=torch.bfloat16, device="cuda")
+    sfq.check(sfq.lib.sfq_pre_quant_scale(sfq.ptr(x) + 2 * shift, sfq.ptr(s), sfq.ptr(out), 3, n, None))
+    want = (x[shift:shift + 3 * n].view(3, n).float() * s[:n].float()).to(torch.bfloat16)
+    assert torch.equal(out[:3 * n].view(3, n), want) and not out[3 * n:].any()
+
+
+@pytest.mark.parametrize("out_f,in_f,block,shift", [(8, 64, 16, 0), (16, 128, 32, 0), (128, 512, 4096, 0), (16, 128, 64, 1), (3, 24, 8, 0)])
+def test_nf4_unpack_wide_and_narrow_blocks(out_f, in_f, block, shift):
+    """Blocks of a multiple of 16 take the wide kernel, an output off its 16-byte boundary or other blocks the narrow one."""
+    n, nested = out_f * in_f, 4
+    rng = np.random.default_rng(n + block)
+    packed, absmax, qmap, nmap, nabs = _nf4_state(rng, n, block, nested)
+    want = np.empty(n, np.uint16)
+    oracle.lib.orc_nf4_dequant_bf16(P(packed), P(absmax), P(qmap), P(nmap), P(nabs), block, nested, 0.031, n, P(want))
+    d = [dev(a) for a in (packed, absmax, qmap, nmap, nabs)]
+    out = torch.empty(n + 8, dtype=torch.bfloat16, device="cuda")
+    sfq.check(sfq.lib.sfq_unpack_nf4_bf16(*[sfq.ptr(t) for t in d], block, nested, 0.031, sfq.ptr(out) + 2 * shift, out_f, in_f, None))
+    assert np.array_equal(bits(out[shift:shift + n].contiguous()), want)
+
+
 @pytest.mark.parametrize("rows,dim", [(1, 1), (3, 257), (64, 5120)])
 def test_pre_quant_scale_bit_exact(rows, dim):
     x = gaussian_bf16((rows, dim), seed=rows)
