@@ -8,7 +8,7 @@
 //          (replaces nvfp4_gemm_kernel, src/cuda/nvfp4_gemm.cu:346-485)
 //   kBf16  bf16 x bf16 -> fp32 (the dequantize-then-GEMM arm, src/cuda/linear.cu:243-246)
 //
-// Layout of the work: a CTA owns one SM and walks output tiles of 128 x BN.
+// Layout of the work: a CTA owns one SM and walks output tiles of 128 x BN (at few rows a cluster shares one, see SPLIT).
 // Warp 0 (one lane) streams K-slabs of 128 bytes per row into a ring of shared
 // memory stages with TMA (128-byte swizzle, no multicast). Warp 1 (one lane)
 // issues tcgen05.mma from shared-memory descriptors into a TMEM accumulator;
@@ -28,7 +28,7 @@
 namespace sfq {
 namespace {
 
-template <int KIND, int BN, int ACC> struct Cfg {
+template <int KIND, int BN, int ACC, int SPLIT = 1> struct Cfg {
   static constexpr int kStageA = kBM * kSlabBytes;
   static constexpr int kStageB = BN * kSlabBytes;
   // nvfp4: per stage 4 k-blocks of 64 elements; one 512-byte scale atom per (128 rows, k-block)
@@ -37,21 +37,29 @@ template <int KIND, int BN, int ACC> struct Cfg {
   static constexpr int kStageBytes = kStageA + kStageB + kStageSfa + kStageSfb;
   static constexpr int kBarrierBytes = 5120;   // barriers + the epilogue's column operands
   static constexpr int kStagingBytes = 8 * 2048;  // one 32x32 bf16 transpose block per epilogue warp
-  static constexpr int kRingBudget = 227 * 1024 - 1024 - kBarrierBytes - kStagingBytes;
+  // K split over a cluster: fp32 / int32 partial sums of this CTA's columns from the other SPLIT - 1 CTAs, 128 rows x 32 columns each
+  static constexpr int kOwnChunks = BN / 32 / SPLIT;
+  static constexpr int kExchangeBytes = (SPLIT - 1) * kOwnChunks * kBM * 128;
+  static constexpr int kRingBudget = 227 * 1024 - 1024 - kBarrierBytes - kStagingBytes - kExchangeBytes;
   static constexpr int kStages = kRingBudget / kStageBytes > 8 ? 8 : kRingBudget / kStageBytes;
   static constexpr int kAccCols = BN * ACC;
   static constexpr int kSfSlotCols = KIND == kNvfp4 ? 4 * 4 + 4 * (BN / 32) : 0;  // SFA 4 cols, SFB BN/32 cols per k-block
   static constexpr int kTmemCols = 512;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + kStagingBytes + 1024;  // +1024 alignment slack
+  static constexpr int kSmemBytes = kStages * kStageBytes + kBarrierBytes + kStagingBytes + kExchangeBytes + 1024;  // +1024 alignment slack
   // one TMEM scale slot per shared-memory stage, so a stage and its scales are released together
   static_assert(kAccCols + kStages * kSfSlotCols <= 512, "TMEM budget");
   static_assert(kStages >= 2, "pipeline needs at least two stages");
 };
 
-template <int KIND, int BN, int ACC, bool GATED>
+// SPLIT > 1: a cluster of SPLIT CTAs shares one output tile and divides K, for launches whose tiles alone leave most SMs
+// idle. Each CTA accumulates its share of the K-slabs; then every CTA sends its partial sums of the other CTAs' columns to
+// them through distributed shared memory, and each finishes (sums in rank order, epilogue, store) its own BN / SPLIT
+// columns. One tile per cluster.
+template <int KIND, int BN, int ACC, bool GATED, int SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, GemmArgs g) {
-  using C = Cfg<KIND, BN, ACC>;
+  static_assert(SPLIT == 1 || (!GATED && BN == 128 && 4 % SPLIT == 0), "the K split is built for the plain 128-wide tile");
+  using C = Cfg<KIND, BN, ACC, SPLIT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Shared* sh = reinterpret_cast<Shared*>(smem + C::kStages * C::kStageBytes);
@@ -64,6 +72,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   const int row_bytes = KIND == kNvfp4 ? g.K / 2 : (KIND == kBf16 ? g.K * 2 : g.K);
   const int k_stages = (row_bytes + kSlabBytes - 1) / kSlabBytes;
   const int band = g.band_m > 0 ? g.band_m : 16;  // m-tiles per raster band
+  const int rank = int(blockIdx.x) % SPLIT, first_tile = int(blockIdx.x) / SPLIT, tile_step = int(gridDim.x) / SPLIT;
+  const int ks_begin = k_stages * rank / SPLIT, ks_end = k_stages * (rank + 1) / SPLIT;
 
   auto tile_coords = [&](int t, int& tm, int& tn) {
     // Bands of `band` row-tiles sweep all column tiles, row-tile fastest inside
@@ -101,6 +111,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   tc_fence_after_sync();
   const uint32_t tmem = sh->tmem_base;
 
+  if constexpr (SPLIT > 1) cluster_arrive();  // awaited before the first store into another CTA: all CTAs of the cluster have started
+
   // Each role's code sits directly under its warpgroup's setmaxnreg, so the compiler budgets it accordingly.
   //
   // The producer, MMA and scale-copy roles run as CONVERGED warps: all 32 lanes walk the loop and poll the
@@ -114,10 +126,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       // ------------------------------------------------------------ producer
       uint32_t it = 0;  // running stage counter
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
+      for (int t = first_tile; t < num_tiles && ok; t += tile_step) {
         int tm, tn;
         tile_coords(t, tm, tn);
-        for (int ks = 0; ks < k_stages; ++ks, ++it) {
+        for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
           const int s = it % C::kStages;  // kStages is a compile-time constant
           const uint32_t ph = (it / C::kStages) & 1;
           if (!(ok = wait_barrier_warp(smem_u32(&sh->empty[s]), ph ^ 1, sh, g.status, 1))) break;
@@ -173,12 +185,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       const int last_valid = min(4, (row_bytes - (k_stages - 1) * kSlabBytes + kMmaKBytes - 1) / kMmaKBytes);
       int s = 0;
       uint32_t ph = 0, tile_it = 0;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_it) {
+      for (int t = first_tile; t < num_tiles && ok; t += tile_step, ++tile_it) {
         const int a = tile_it % ACC;
         if (!(ok = wait_barrier_warp(smem_u32(&sh->acc_empty[a]), ((tile_it / ACC) & 1) ^ 1, sh, g.status, 2))) break;
         tc_fence_after_sync();
         const uint32_t d = tmem + a * BN;
-        for (int ks = 0; ks < k_stages; ++ks) {
+        for (int ks = ks_begin; ks < ks_end; ++ks) {
           // nvfp4: the scale-copy warps arrive on sf_full[s] after they have seen full[s] themselves and their
           // copies into TMEM slot s have landed, so that one barrier stands for operands and scales alike.
           if constexpr (KIND == kNvfp4) {
@@ -195,7 +207,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
 #pragma unroll
             for (int kb = 0; kb < 4; ++kb) {
               if (kb < kb_valid) {
-                const uint32_t acc = (ks | kb) ? 1u : 0u;
+                const uint32_t acc = (ks > ks_begin || kb) ? 1u : 0u;
                 const uint64_t adv = uint64_t(kb * (kMmaKBytes >> 4));
                 if constexpr (KIND == kI8)
                   mma_i8(d, da + adv, db + adv, idesc, acc);
@@ -207,7 +219,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
             }
             // One commit frees the stage's shared memory for the producer and its scale slot for the copy warps.
             tc_commit(smem_u32(&sh->empty[s]));
-            if (ks == k_stages - 1) tc_commit(smem_u32(&sh->acc_full[a]));
+            if (ks == ks_end - 1) tc_commit(smem_u32(&sh->acc_full[a]));
           }
           __syncwarp();
           if (++s == C::kStages) s = 0, ph ^= 1;
@@ -229,8 +241,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        for (int ks = 0; ks < k_stages; ++ks) {
+      for (int t = first_tile; t < num_tiles && ok; t += tile_step) {
+        for (int ks = ks_begin; ks < ks_end; ++ks) {
           // full[s] of this round completes only after the producer has seen empty[s] of the previous round, so the
           // loads having landed also says that the MMAs which read this stage's scale slot are done: one wait, not two
           if (!(ok = wait_barrier_warp(smem_u32(&sh->full[s]), ph, sh, g.status, 6))) break;
@@ -265,7 +277,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     bool ok = true;
     const bool vec_ok = (g.N % 8 == 0) && ((reinterpret_cast<uintptr_t>(g.y) & 15) == 0) && (g.ldy % 8 == 0);
     const bool has_bias = g.bias != nullptr;
-    for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_it) {
+    for (int t = first_tile; t < num_tiles && ok; t += tile_step, ++tile_it) {
       int tm, tn;
       tile_coords(t, tm, tn);
       const int a = tile_it % ACC;
@@ -296,7 +308,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (!(ok = wait_barrier(smem_u32(&sh->acc_full[a]), aph, sh, g.status, 4))) break;
+      if (!(ok = wait_barrier(smem_u32(&sh->acc_full[a]), aph, sh, g.status, 4))) {
+        if constexpr (SPLIT > 1) cluster_wait(), cluster_sync_all();  // the other CTAs are not left waiting
+        break;
+      }
       tc_fence_after_sync();
       const int row = tm * kBM + quad * 32 + lane;
       const bool row_ok = row < g.M;
@@ -326,11 +341,54 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[a]));
+      if constexpr (SPLIT > 1) {
+        // [source among the others][chunk of the owner][row][32 columns]: 16-byte units XOR-swizzled with the row, so that the
+        // 32 lanes of a warp (rows 128 bytes apart) spread over the banks
+        uint8_t* exchange = smem + C::kStages * C::kStageBytes + C::kBarrierBytes + C::kStagingBytes;
+        const int lrow = quad * 32 + lane;
+        auto slot = [&](int src, int owner, int c) {
+          return uint32_t((((src < owner ? src : src - 1) * C::kOwnChunks + c - owner * C::kOwnChunks) * kBM + lrow) * 128);
+        };
+        cluster_wait();
+#pragma unroll
+        for (int j = 0; j < kMaxJ; ++j) {
+          const int c = half + 2 * j, owner = c / C::kOwnChunks;
+          if (owner == rank) continue;
+          const uint32_t dst = map_to_rank(smem_u32(exchange) + slot(rank, owner, c), uint32_t(owner));
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            st_cluster_v4(dst + uint32_t((u ^ (lane & 7)) * 16), r[j][4 * u], r[j][4 * u + 1], r[j][4 * u + 2], r[j][4 * u + 3]);
+        }
+        cluster_sync_all();
+#pragma unroll
+        for (int j = 0; j < kMaxJ; ++j) {
+          const int c = half + 2 * j;
+          if (c / C::kOwnChunks != rank) continue;
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            uint32_t sum[4] = {0, 0, 0, 0};  // in rank order, this CTA's own share in its place
+#pragma unroll
+            for (int src = 0; src < SPLIT; ++src) {
+              uint32_t v[4] = {r[j][4 * u], r[j][4 * u + 1], r[j][4 * u + 2], r[j][4 * u + 3]};
+              if (src != rank) {
+                const uint4 got = *reinterpret_cast<const uint4*>(exchange + slot(src, rank, c) + (u ^ (lane & 7)) * 16);
+                v[0] = got.x, v[1] = got.y, v[2] = got.z, v[3] = got.w;
+              }
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                sum[i] = src == 0 ? v[i] : (KIND == kI8 ? sum[i] + v[i] : __float_as_uint(__uint_as_float(sum[i]) + __uint_as_float(v[i])));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[j][4 * u + i] = sum[i];
+          }
+        }
+      }
 #pragma unroll
       for (int j = 0; j < kMaxJ; ++j) {
         const int c = half + 2 * j;
         const int col0 = tn * BN + c * 32;
         if (c >= kTileChunks || col0 >= g.N) continue;  // warp-uniform
+        if (SPLIT > 1 && c / C::kOwnChunks != rank) continue;
         const int lc0 = c * 32;
         uint4 packed[4];
         if (!has_bias && g.act == SFQ_ACT_NONE)
@@ -364,6 +422,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
     }
   }
 
+  if constexpr (SPLIT > 1)
+    if (warp < 4 || warp >= 12) cluster_wait(), cluster_sync_all();  // the epilogue warps have been through both
   tc_fence_before_sync();
   __syncthreads();
   if (warp == 1) {
@@ -372,16 +432,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   }
 }
 
-template <int KIND, int BN, int ACC, bool GATED>
+template <int KIND, int BN, int ACC, bool GATED, int SPLIT = 1>
 void launch_epi(const void* a, const void* w, size_t row_bytes, const GemmArgs& g, cudaStream_t stream) {
-  using C = Cfg<KIND, BN, ACC>;
-  reserve_dynamic_smem(reinterpret_cast<const void*>(&gemm_kernel<KIND, BN, ACC, GATED>), C::kSmemBytes, "sfq gemm");
+  using C = Cfg<KIND, BN, ACC, SPLIT>;
+  auto kernel = gemm_kernel<KIND, BN, ACC, GATED, SPLIT>;
+  reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), C::kSmemBytes, "sfq gemm");
   const CUtensorMap ma = make_map(a, size_t(g.M), row_bytes, kBM);
   const CUtensorMap mb = make_map(w, size_t(g.N), row_bytes, BN);
   const int tiles = ((g.M + kBM - 1) / kBM) * ((g.N + BN - 1) / BN);
-  const int grid = g.max_ctas > 0 ? std::min(tiles, g.max_ctas) : std::min(tiles, sm_count());
-  gemm_kernel<KIND, BN, ACC, GATED><<<grid, kThreads, C::kSmemBytes, stream>>>(ma, mb, g);
-  const cudaError_t e = cudaGetLastError();
+  const int grid = SPLIT > 1 ? tiles * SPLIT : (g.max_ctas > 0 ? std::min(tiles, g.max_ctas) : std::min(tiles, sm_count()));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = SPLIT;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mb, g);
   if (e != cudaSuccess) throw std::runtime_error(std::string("sfq gemm: launch failed: ") + cudaGetErrorString(e));
 }
 
@@ -392,6 +464,25 @@ void launch(const void* a, const void* w, size_t row_bytes, const GemmArgs& g, c
     launch_epi<KIND, BN, ACC, true>(a, w, row_bytes, g, stream);
   else
     launch_epi<KIND, BN, ACC, false>(a, w, row_bytes, g, stream);
+}
+
+// At most 128 rows: the launch is bound by reading the weight, and an SM takes in no more than about 100 GB/s, so what counts
+// is how many SMs read. 128-wide tiles where 256-wide ones would leave SMs idle; and K split two or four ways where even
+// those do, as long as each CTA keeps kMinSplitStages slabs (below that the exchange of the partial sums costs more than the
+// shorter loop saves). 77 x 5120 -> 13824 nvfp4, quantizer and launch gaps included: 20.5 us, 29.0 with 256-wide tiles.
+constexpr int kMinSplitStages = 8;
+template <int KIND, int ACC256>
+void launch_few_rows(const void* a, const void* w, size_t row_bytes, const GemmArgs& g, cudaStream_t stream) {
+  const int tiles = (g.N + 127) / 128, sms = sm_count();
+  const int stages = int((row_bytes + kSlabBytes - 1) / kSlabBytes);
+  if (tiles > sms || g.gate != nullptr)
+    launch<KIND, 256, ACC256>(a, w, row_bytes, g, stream);
+  else if (4 * tiles <= sms && stages >= 4 * kMinSplitStages)
+    launch_epi<KIND, 128, 2, false, 4>(a, w, row_bytes, g, stream);
+  else if (2 * tiles <= sms && stages >= 2 * kMinSplitStages)
+    launch_epi<KIND, 128, 2, false, 2>(a, w, row_bytes, g, stream);
+  else
+    launch<KIND, 128, 2>(a, w, row_bytes, g, stream);
 }
 
 }  // namespace
@@ -408,7 +499,9 @@ void gemm_int8(const int8_t* a, const int8_t* w, const GemmArgs& g, cudaStream_t
     return;
   }
   if (g.tile_n == 0 && g.M > kBM && gemm_pair_int8(a, w, g, stream)) return;
-  if (g.tile_n == 128)
+  if (g.tile_n == 0 && g.max_ctas == 0 && g.M <= kBM)
+    launch_few_rows<kI8, 2>(a, w, size_t(g.K), g, stream);
+  else if (g.tile_n == 128)
     launch<kI8, 128, 2>(a, w, size_t(g.K), g, stream);
   else
     launch<kI8, 256, 2>(a, w, size_t(g.K), g, stream);
@@ -427,7 +520,9 @@ void gemm_nvfp4(const uint8_t* a, const uint8_t* w, const GemmArgs& g, cudaStrea
     return;
   }
   if (g.tile_n == 0 && g.M > kBM && gemm_pair_nvfp4(a, w, g, stream)) return;
-  if (g.tile_n == 128)
+  if (g.tile_n == 0 && g.max_ctas == 0 && g.M <= kBM)
+    launch_few_rows<kNvfp4, 1>(a, w, size_t(g.K) / 2, g, stream);
+  else if (g.tile_n == 128)
     launch<kNvfp4, 128, 2>(a, w, size_t(g.K) / 2, g, stream);
   else
     launch<kNvfp4, 256, 1>(a, w, size_t(g.K) / 2, g, stream);
@@ -442,7 +537,9 @@ void gemm_bf16(const __nv_bfloat16* a, const __nv_bfloat16* w, const GemmArgs& g
     return;
   }
   if (g.tile_n == 0 && g.M > kBM && gemm_pair_bf16(a, w, g, stream)) return;
-  if (g.tile_n == 128)
+  if (g.tile_n == 0 && g.max_ctas == 0 && g.M <= kBM)
+    launch_few_rows<kBf16, 2>(a, w, size_t(g.K) * 2, g, stream);
+  else if (g.tile_n == 128)
     launch<kBf16, 128, 2>(a, w, size_t(g.K) * 2, g, stream);
   else
     launch<kBf16, 256, 2>(a, w, size_t(g.K) * 2, g, stream);

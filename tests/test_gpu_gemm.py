@@ -132,6 +132,66 @@ def test_gemm_bf16_within_reference_tolerance(M, N, K):
     assert torch.all((y.float() - want).abs() <= 1e-3 + 1e-2 * want.abs())
 
 
+@pytest.mark.parametrize("kind", ["int8", "bf16", "nvfp4"])
+@pytest.mark.parametrize("M,N,slabs", [
+    (1, 128, 32),      # one tile, K four ways
+    (77, 136, 35),     # ragged N, unequal shares of K
+    (128, 4736, 33),   # the most tiles that K is still split four ways for on 148 SMs
+    (128, 4864, 17),   # two ways
+    (100, 9472, 16),   # the most tiles with two ways
+    (128, 9600, 16),   # 128-wide tiles, no split
+    (64, 640, 9),      # too few slabs for a split
+    (33, 18944, 3),    # the most 128-wide tiles
+    (33, 19072, 3),    # 256-wide tiles
+])
+def test_gemm_of_few_rows_equals_the_256_wide_kernel(M, N, slabs, kind):
+    """At most 128 rows: narrower tiles and K divided over a cluster. int8 sums are exact; in fp32 only the order of the sums
+    differs, which moves at most the last bit of the bf16 result."""
+    rng = np.random.default_rng(M + N + slabs)
+    bias = dev((0.01 * rng.standard_normal(N)).astype(np.float32))
+    if kind == "nvfp4":
+        N = (N + 127) // 128 * 128
+        K = slabs * 256 - 64  # the last slab is not full
+        a = dev(rng.integers(0, 256, size=(M, K // 2), dtype=np.uint8))
+        w = dev(rng.integers(0, 256, size=(N, K // 2), dtype=np.uint8))
+        rows = (M + 127) // 128 * 128
+        sa, sw = (dev(rng.integers(0x30, 0x40, size=n * K // 16, dtype=np.uint8)) for n in (rows, N))
+        bias = dev((0.01 * rng.standard_normal(N)).astype(np.float32))
+        run = lambda y, ep: sfq.lib.sfq_gemm_nvfp4(sfq.ptr(a), sfq.ptr(sa), sfq.ptr(w), sfq.ptr(sw), C.byref(ep), sfq.ptr(y), M, N, K, S)  # noqa: E731
+        ep = sfq.Epilogue(None, None, 0.001, sfq.ptr(bias), sfq.F32, sfq.ACT_NONE)
+    elif kind == "int8":
+        K = slabs * 128 - 48
+        a = dev(rng.integers(-128, 128, size=(M, K), dtype=np.int8))
+        w = dev(rng.integers(-127, 128, size=(N, K), dtype=np.int8))
+        rs, cs = dev((rng.random(M) * 0.05 + 1e-3).astype(np.float32)), dev((rng.random(N) * 0.01 + 1e-4).astype(np.float32))
+        run = lambda y, ep: sfq.lib.sfq_gemm_int8(sfq.ptr(a), sfq.ptr(w), C.byref(ep), sfq.ptr(y), M, N, K, S)  # noqa: E731
+        ep = sfq.Epilogue(sfq.ptr(rs), sfq.ptr(cs), 1.0, sfq.ptr(bias), sfq.F32, sfq.ACT_NONE)
+    else:
+        K = slabs * 64 - 8
+        a = bf16_tensor(gaussian_bf16((M, K), seed=M))
+        w = torch.randn((N, K), device="cuda", generator=torch.Generator("cuda").manual_seed(N)).mul_(0.02).to(torch.bfloat16)
+        run = lambda y, ep: sfq.lib.sfq_gemm_bf16(sfq.ptr(a), sfq.ptr(w), C.byref(ep), sfq.ptr(y), M, N, K, S)  # noqa: E731
+        ep = sfq.Epilogue(None, None, 1.0, sfq.ptr(bias), sfq.F32, sfq.ACT_NONE)
+    got = []
+    for tile_n in (0, 0, 256):
+        y = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+        sfq.lib.sfq_test_gemm_variant(tile_n, 0, 0)
+        try:
+            sfq.check(run(y, ep))
+        finally:
+            sfq.lib.sfq_test_gemm_variant(0, 0, 0)
+        _status_clean()
+        got.append(y)
+    assert torch.equal(got[0], got[1])  # the order of the sums is fixed
+    if kind == "int8":
+        assert torch.equal(got[0], got[2])
+    else:
+        f, want = got[0].float(), got[2].float()
+        # fp32 sums a few ulps apart, rounded to bf16 twice: the product (|product| <= |result| + |bias|) and the sum with the bias may
+        # each land one bf16 step (2^-7 of the value at most) apart
+        assert bool(((f - want).abs() <= 2.0 ** -7 * (2 * want.abs() + bias.abs()) + 1e-5 * want.abs().max()).all())
+
+
 def _nvfp4_case(M, N, K, seed):
     rng = np.random.default_rng(seed)
     w = (0.02 * rng.standard_normal((N, K))).astype(np.float32)
