@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
     }
 }
 
-// The same product for few rows, which is how the DiT calls it: bound by reading the weight once. A CTA of four warps
+// The same product with the rows in tiles of at most 16, for the few rows the DiT calls it with: bound by reading the weight once. A CTA of four warps
 // takes F output features and R rows and splits K between its 128 threads, 16 bytes of fp32 weight (8 of bf16) per thread,
 // feature and step, so a warp reads 512 contiguous bytes of each weight row and 2 F such loads are in flight per thread;
 // the products run as packed pairs (even and odd k in the two halves of an f32x2 accumulator). x is small and shared by
@@ -492,13 +492,15 @@ void launch_rows_for(const float* x, const WT* w, const void* bias, bool bias_is
     launch_rows<WT, 16, F>(x, w, bias, bias_is_bf16, y, rows, out_features, in_features, stream);
 }
 
-constexpr int kFewRows = 64;
-
 template <typename WT>
 void launch_linear_f32(const float* x, const WT* w, const void* bias, bool bias_is_bf16, float* y, int rows, int out_features, int in_features,
                        cudaStream_t stream) {
+  const dim3 grid((out_features + 63) / 64, (rows + 63) / 64);
+  if (grid.y > 65535) throw std::invalid_argument("linear_f32: too many rows for one launch");
+  // The row kernel wherever its loads are aligned and its flat grid fits: 5120 -> 15360 in fp32, it against the tiled kernel, 1 row
+  // 48 / 1052 us, 64 rows 580 / 1323, 512 rows 4243 / 4383; 200 rows of 1024 -> 512 29 / 147.
   const bool wide = in_features % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % (4 * sizeof(WT)) == 0;
-  if (rows <= kFewRows && wide) {
+  if (wide && size_t(out_features) * ((rows + 15) / 16) <= size_t(0x7FFFFFFF)) {
     // four features per CTA while that leaves every SM its four CTAs, one otherwise
     if (out_features >= 4 * 4 * device_sm_count())
       launch_rows_for<WT, 4>(x, w, bias, bias_is_bf16, y, rows, out_features, in_features, stream);
@@ -506,8 +508,6 @@ void launch_linear_f32(const float* x, const WT* w, const void* bias, bool bias_
       launch_rows_for<WT, 1>(x, w, bias, bias_is_bf16, y, rows, out_features, in_features, stream);
     return;
   }
-  const dim3 grid((out_features + 63) / 64, (rows + 63) / 64);
-  if (grid.y > 65535) throw std::invalid_argument("linear_f32: too many rows for one launch");
   linear_f32_kernel<WT><<<grid, 256, 0, stream>>>(x, w, bias, bias_is_bf16 ? 1 : 0, y, rows, out_features, in_features);
 }
 

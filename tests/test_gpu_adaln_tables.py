@@ -94,7 +94,7 @@ def test_forward_f32_against_the_fp64_product(fmt, rows, n, k):
                                       (17, 2500, 132), (64, 2500, 1024), (65, 300, 256), (3, 300, 258)])
 def test_forward_f32_row_tiles(fmt, rows, n, k):
     """Every row tile (1, 4, 8, 16), one and four features per CTA, ragged ends of all three extents, and the tiled kernel behind
-    them (more than 64 rows, K not in fours). Bound: (K / 256 + 16) additions of fp32 terms, each rounding by 2^-24 of the sum of
+    them (K not in fours). Bound: (K / 256 + 16) additions of fp32 terms, each rounding by 2^-24 of the sum of
     the terms' magnitudes at most."""
     g = torch.Generator("cuda").manual_seed(rows + n)
     x = torch.randn((rows, k), device="cuda", generator=g)
@@ -105,7 +105,7 @@ def test_forward_f32_row_tiles(fmt, rows, n, k):
     got = sfq.LinearRunner().forward_f32(weight, x)
     want = x.double() @ w.double().T + bias.double()
     terms = x.double().abs() @ w.double().abs().T + bias.double().abs()
-    steps = (k / 256 + 16) if rows <= 64 and k % 4 == 0 else k + 1
+    steps = (k / 256 + 16) if k % 4 == 0 else k + 1
     assert bool(((got.double() - want).abs() <= steps * 2.0 ** -24 * terms).all())
 
 
