@@ -180,7 +180,8 @@ private:
   const void* cached_arena_ = nullptr;
   size_t cached_end_ = 0;
   uint64_t cached_epoch_ = 0;
-  // A plain forward() of a W4A8/W6A8 layer expands the weight on this second stream while the activation is
+  bool beside_ = false;  // inside forward(): the dense weight's launch is the last one in the stream
+  // A plain forward() of a W4A8/W6A8 layer whose weight is not small expands it on this second stream while the activation is
   // quantized on the caller's; the GEMM waits for both. Created on first use.
   cudaStream_t side_ = nullptr;
   cudaEvent_t fork_ = nullptr;

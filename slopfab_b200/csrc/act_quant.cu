@@ -51,6 +51,7 @@ struct FusedArgs {
   uint8_t* packed;
   uint8_t* scales;
   __nv_bfloat16* bf16_out;  // normed activation (optional) or the rotated one (rot-only mode)
+  int beside;  // rotation only: wait for the kernel in front at the end instead of at the start (see kernels.cuh)
 };
 
 // ---- integer-exact norm reciprocal (include/slopfab/cuda/deterministic_math.cuh:26-197) ----
@@ -319,6 +320,8 @@ __device__ __forceinline__ void process_row(const FusedArgs& a, const int row, u
 template <int MODE>
 __global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
+  ptx::grid_dependency_release();
+  if (MODE != kModeRotOnly || !a.beside) a.x = ptx::grid_dependency_wait(a.x);
   const int chunks = a.dim >> 4;
   const bool active = int(threadIdx.x) < chunks;
   auto load = [&](int row, uint4& r0, uint4& r1) {
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
     r0 = n0;
     r1 = n1;
   }
+  if (MODE == kModeRotOnly && a.beside) ptx::grid_dependency_wait();
 }
 
 // ---- RMSNorm [+ modulate], alone or in front of the per-16-block fp4 quantizer ---------------------------------------
@@ -398,8 +402,11 @@ __device__ __forceinline__ uint32_t hmax2(uint32_t a, uint32_t b) {
 }
 
 template <int MODE, int MAXP>
-__global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_kernel(const FusedArgs a, int total_rows) {
+__global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_kernel(const FusedArgs args, int total_rows) {
   constexpr int R = kNormRows<MAXP>;
+  FusedArgs a = args;
+  ptx::grid_dependency_release();
+  a.x = ptx::grid_dependency_wait(a.x);
   __shared__ float warp_tot[R][8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int packs = a.dim >> 3, chunks = a.dim >> 4;
@@ -563,8 +570,7 @@ convrot_small_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __rest
   for (int i = t; i < n; i += 64) out[base + i] = __float2bfloat16(v[i + (i >> 2)] * norm);
 }
 
-inline void check_launch(const char* what) {
-  const cudaError_t e = cudaGetLastError();
+inline void check_launch(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -587,8 +593,7 @@ template <int MODE> void launch_fused(const FusedArgs& a, cudaStream_t stream, c
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_act_kernel<MODE>, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   const int grid = std::min(a.rows, per_sm * device_sm_count());
-  fused_act_kernel<MODE><<<grid, threads, smem, stream>>>(a);
-  check_launch(what);
+  check_launch(launch_overlapped(size_t(a.rows) * a.dim * 4, fused_act_kernel<MODE>, dim3(grid), dim3(threads), smem, stream, a), what);
 }
 
 // A thread's packs per row decide the registers of the kernel.
@@ -596,15 +601,17 @@ template <int MODE> void launch_norm(const FusedArgs& a, int total_rows, cudaStr
   check_row_args(a, what);
   const int per_thread = (a.dim / 8 + kNormThreads - 1) / kNormThreads;
   const auto grid = [&](int r) { return (total_rows + r - 1) / r; };
+  const size_t bytes = size_t(a.rows) * a.dim * 3;
+  cudaError_t e = cudaSuccess;
   if (per_thread <= 2)
-    norm_rows_kernel<MODE, 2><<<grid(kNormRows<2>), kNormThreads, 0, stream>>>(a, total_rows);
+    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 2>, dim3(grid(kNormRows<2>)), dim3(kNormThreads), 0, stream, a, total_rows);
   else if (per_thread <= 5)
-    norm_rows_kernel<MODE, 5><<<grid(kNormRows<5>), kNormThreads, 0, stream>>>(a, total_rows);
+    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 5>, dim3(grid(kNormRows<5>)), dim3(kNormThreads), 0, stream, a, total_rows);
   else if (per_thread <= 6)
-    norm_rows_kernel<MODE, 6><<<grid(kNormRows<6>), kNormThreads, 0, stream>>>(a, total_rows);
+    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 6>, dim3(grid(kNormRows<6>)), dim3(kNormThreads), 0, stream, a, total_rows);
   else
-    norm_rows_kernel<MODE, 16><<<grid(kNormRows<16>), kNormThreads, 0, stream>>>(a, total_rows);
-  check_launch(what);
+    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 16>, dim3(grid(kNormRows<16>)), dim3(kNormThreads), 0, stream, a, total_rows);
+  check_launch(e, what);
 }
 
 FusedArgs base_args(const __nv_bfloat16* x, const NormArgs& n, int rows, int dim) {
@@ -630,7 +637,7 @@ void rmsnorm(const __nv_bfloat16* x, const NormArgs& norm, __nv_bfloat16* out, i
   launch_norm<kNormOnly>(a, rows, stream, "rmsnorm");
 }
 
-void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int group, cudaStream_t stream) {
+void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int group, cudaStream_t stream, bool beside) {
   if (rows <= 0 || dim <= 0) return;
   if (!x || !out) throw std::invalid_argument("convrot: null buffer");
   int stages = 0, n = 1;
@@ -640,23 +647,24 @@ void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int 
   if (group == 256 && dim <= 16384) {
     FusedArgs a = base_args(x, NormArgs{}, rows, dim);
     a.apply_convrot = 1;
+    a.beside = beside ? 1 : 0;
     a.bf16_out = out;
     launch_fused<kModeRotOnly>(a, stream, "convrot");
     return;
   }
   if (group > 256) throw std::runtime_error("convrot: groups above 256 are not supported");
   convrot_small_kernel<<<dim3(rows, (dim + 255) / 256), 64, 0, stream>>>(x, out, dim, stages, 1.0f / float(1 << stages));
-  check_launch("convrot");
+  check_launch(cudaGetLastError(), "convrot");
 }
 
 void quantize_int8_token(const __nv_bfloat16* x, const NormArgs& norm, int8_t* q, float* row_scale,
-                         __nv_bfloat16* normed_out, int rows, int dim, bool apply_convrot, cudaStream_t stream) {
+                         __nv_bfloat16* normed_out, int rows, int dim, bool apply_convrot, cudaStream_t stream, bool overlap) {
   if (rows <= 0 || dim <= 0) throw std::invalid_argument("W4A8 activation shape");
   if (!x || !q || !row_scale) throw std::invalid_argument("quantize_int8_token: null buffer");
   if (apply_convrot && dim % 256 != 0) throw std::invalid_argument("W4A8 activation requires K divisible by 256");
   if (reinterpret_cast<uintptr_t>(q) % 16 != 0) throw std::invalid_argument("quantize_int8_token: output must be 16-byte aligned");
   // The Linear's own case (rotation on, nothing fused in front, K <= 6144) has a two-rows-per-step kernel.
-  if (apply_convrot && norm.weight == nullptr && quantize_int8_rot_pairs(x, q, row_scale, rows, dim, stream)) return;
+  if (apply_convrot && norm.weight == nullptr && quantize_int8_rot_pairs(x, q, row_scale, rows, dim, stream, overlap)) return;
   FusedArgs a = base_args(x, norm, rows, dim);
   a.q = q;
   a.row_scale = row_scale;
@@ -706,6 +714,8 @@ __device__ __forceinline__ void quantize_block16(const uint4 r0, const uint4 r1,
 template <bool FEED>
 __global__ void __launch_bounds__(256) quantize_nvfp4_flat_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ packed,
                                                                   uint8_t* __restrict__ scales, int rows, int padded_rows, int chunks) {
+  ptx::grid_dependency_release();
+  x = ptx::grid_dependency_wait(x);
   // item g = (row, chunk): advance by the grid's stride without a division per item
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
@@ -750,8 +760,8 @@ void launch_nvfp4_flat(const __nv_bfloat16* x, uint8_t* packed, uint8_t* scales,
   const size_t items = size_t(padded) * chunks;
   if (items >= (size_t(1) << 31)) throw std::invalid_argument("quantize_nvfp4_block: too many 16-element blocks for one launch");
   const int ctas = int(std::min<size_t>((items + 511) / 512, size_t(device_sm_count()) * 8));  // two items per thread and trip
-  quantize_nvfp4_flat_kernel<FEED><<<ctas, 256, 0, stream>>>(x, packed, scales, rows, padded, chunks);
-  check_launch("quantize_nvfp4_block");
+  check_launch(launch_overlapped(items * 41, quantize_nvfp4_flat_kernel<FEED>, dim3(ctas), dim3(256), 0, stream, x, packed, scales, rows, padded, chunks),
+               "quantize_nvfp4_block");
 }
 }  // namespace
 
@@ -836,6 +846,8 @@ __global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __re
                                                              const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
                                                              int tables_vec, int rows, int heads, float eps) {
   constexpr int kPer = kHeadsPerWarp / 2;  // heads per half warp
+  ptx::grid_dependency_release();
+  ptx::grid_dependency_wait();
   const int lane = threadIdx.x & 31, l = lane & 15, half = lane >> 4;
   const int groups = (heads + kHeadsPerWarp - 1) / kHeadsPerWarp;
   const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);  // (row, group of heads)
@@ -951,13 +963,15 @@ void head_norm_rope(__nv_bfloat16* x, int ld, const __nv_bfloat16* norm_weight, 
   const long long units = (long long)rows * ((heads + kHeadsPerWarp - 1) / kHeadsPerWarp);
   const int tables_vec = ((reinterpret_cast<uintptr_t>(cos_tab) | reinterpret_cast<uintptr_t>(sin_tab)) & 15) == 0;
   const unsigned grid = unsigned((units + 7) / 8);
+  const size_t bytes = size_t(rows) * heads * 512;
+  cudaError_t e = cudaSuccess;
   if (norm_weight != nullptr && cos_tab != nullptr)
-    head_norm_rope_kernel<true, true><<<grid, 256, 0, stream>>>(x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
+    e = launch_overlapped(bytes, head_norm_rope_kernel<true, true>, dim3(grid), dim3(256), 0, stream, x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
   else if (norm_weight != nullptr)
-    head_norm_rope_kernel<true, false><<<grid, 256, 0, stream>>>(x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
+    e = launch_overlapped(bytes, head_norm_rope_kernel<true, false>, dim3(grid), dim3(256), 0, stream, x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
   else
-    head_norm_rope_kernel<false, true><<<grid, 256, 0, stream>>>(x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
-  check_launch("head_norm_rope");
+    e = launch_overlapped(bytes, head_norm_rope_kernel<false, true>, dim3(grid), dim3(256), 0, stream, x, ld, norm_weight, cos_tab, sin_tab, tables_vec, rows, heads, eps);
+  check_launch(e, "head_norm_rope");
 }
 
 }  // namespace sfq

@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
+  grid_dependency_release();
+  grid_dependency_wait();  // q, k and the transposed v
   const uint32_t tmem = sh->tmem_base;  // columns: S/P of tile 0 [0,128), of tile 1 [128,256), O of tile 0 [256,384), of tile 1 [384,512)
 
   // Each role's code sits directly under its warpgroup's setmaxnreg, so the compiler budgets it accordingly.
@@ -439,6 +441,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
 __global__ void __launch_bounds__(256) transpose_v_kernel(const __nv_bfloat16* __restrict__ v, int ld_v, __nv_bfloat16* __restrict__ vt, int ld_t,
                                                           int seq, int width) {
   __shared__ __nv_bfloat16 tile[64][66];
+  grid_dependency_release();
+  v = grid_dependency_wait(v);
   const int s0 = blockIdx.x * 64, w0 = blockIdx.y * 64;
   for (int i = threadIdx.x; i < 64 * 64; i += 256) {
     const int rs = i >> 6, cw = i & 63;
@@ -494,8 +498,7 @@ void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k,
   const int ld_t = padded_keys(seq_kv);
   __nv_bfloat16* vt = static_cast<__nv_bfloat16*>(workspace);
   const int width = kv_heads * kTile;
-  transpose_v_kernel<<<dim3((ld_t + 63) / 64, (width + 63) / 64), 256, 0, stream>>>(v, ld_kv, vt, ld_t, seq_kv, width);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_overlapped(size_t(seq_kv) * width * 4, transpose_v_kernel, dim3((ld_t + 63) / 64, (width + 63) / 64), dim3(256), 0, stream, v, ld_kv, vt, ld_t, seq_kv, width);
   if (e != cudaSuccess) throw std::runtime_error(std::string("sfq attention: launch failed: ") + cudaGetErrorString(e));
 
   const CUtensorMap mq = make_attn_map(q, size_t(seq_q), size_t(heads) * kTile, size_t(ld_q));
@@ -505,8 +508,7 @@ void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k,
   a.out = out, a.ld_out = ld_out, a.seq_q = seq_q, a.seq_kv = seq_kv, a.group = heads / kv_heads;
   a.scale_log2 = (scale > 0.0f ? scale : 1.0f / sqrtf(float(head_dim))) * 1.4426950408889634f;
   a.status = device_status_word();
-  attention_kernel<<<dim3((seq_q + 2 * kTile - 1) / (2 * kTile), heads), kAttnThreads, kAttnSmem, stream>>>(mq, mk, mv, a);
-  e = cudaGetLastError();
+  e = launch_overlapped(size_t(seq_kv) * width * 4, attention_kernel, dim3((seq_q + 2 * kTile - 1) / (2 * kTile), heads), dim3(kAttnThreads), kAttnSmem, stream, mq, mk, mv, a);
   if (e != cudaSuccess) throw std::runtime_error(std::string("sfq attention: launch failed: ") + cudaGetErrorString(e));
 }
 

@@ -111,6 +111,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   tc_fence_after_sync();
   const uint32_t tmem = sh->tmem_base;
 
+  // The set-up above ran beside the end of the kernel that writes the activation; the next kernel's may run beside this one's end.
+  grid_dependency_release();
+  grid_dependency_wait();
   if constexpr (SPLIT > 1) cluster_arrive();  // awaited before the first store into another CTA: all CTAs of the cluster have started
 
   // Each role's code sits directly under its warpgroup's setmaxnreg, so the compiler budgets it accordingly.
@@ -446,13 +449,15 @@ void launch_epi(const void* a, const void* w, size_t row_bytes, const GemmArgs& 
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = SPLIT;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_overlapped()
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = g.serial_launch ? 1 : 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, ma, mb, g);
   if (e != cudaSuccess) throw std::runtime_error(std::string("sfq gemm: launch failed: ") + cudaGetErrorString(e));
 }

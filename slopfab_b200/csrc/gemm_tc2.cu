@@ -141,6 +141,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   cluster_sync_all();  // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after_sync();
   const uint32_t tmem = sh->tmem_base;
+  // The set-up above ran beside the end of the kernel that writes the activation; the next kernel's may run beside this one's end.
+  grid_dependency_release();
+  grid_dependency_wait();
 
   if (warp < 4) {
     reg_dec<kRegsLean>();
@@ -592,13 +595,15 @@ bool launch_pair_epi(const void* a, const void* w, size_t row_bytes, const GemmA
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = C::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 2;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_overlapped()
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g.serial_launch || tiles > 4 * pairs_cap ? 1 : 2;  // long launches the plain way, see launch_overlapped()
   const cudaError_t e = ga.tail_split > 0
                             ? cudaLaunchKernelEx(&cfg, gemm_pair_kernel<KIND, ACC, EPI, true>, ma, mb, msa, msb, mbn, msbn, ga)
                             : cudaLaunchKernelEx(&cfg, gemm_pair_kernel<KIND, ACC, EPI, false>, ma, mb, msa, msb, mbn, msbn, ga);

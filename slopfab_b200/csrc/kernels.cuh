@@ -45,9 +45,12 @@ struct NormArgs {  // null weight = stage disabled
   float eps = 1e-5f;
 };
 void rmsnorm(const __nv_bfloat16* x, const NormArgs& norm, __nv_bfloat16* out, int rows, int dim, cudaStream_t stream);
-void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int group, cudaStream_t stream);
+// `beside`: the kernel directly in front in the stream (a weight unpacker, itself launched behind everything older) neither
+// writes x nor touches out, so this one runs beside it and waits for it only before it ends. Whatever is launched next then
+// follows both.
+void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int group, cudaStream_t stream, bool beside = false);
 void quantize_int8_token(const __nv_bfloat16* x, const NormArgs& norm, int8_t* q, float* row_scale,
-                         __nv_bfloat16* normed_out, int rows, int dim, bool apply_convrot, cudaStream_t stream);
+                         __nv_bfloat16* normed_out, int rows, int dim, bool apply_convrot, cudaStream_t stream, bool overlap = true);
 void quantize_nvfp4_block(const __nv_bfloat16* x, const NormArgs& norm, uint8_t* packed, uint8_t* scales,
                           __nv_bfloat16* normed_out, int rows, int dim, int layout, cudaStream_t stream);
 size_t nvfp4_act_scale_bytes(int rows, int dim);
@@ -70,7 +73,7 @@ void narrow_to_bf16(const float* src, __nv_bfloat16* dst, size_t n, cudaStream_t
 void nvfp4_act_to_feed(const uint8_t* xq, const uint8_t* xs, uint8_t* feed_q, uint8_t* feed_scale_tiled, int rows, int dim,
                        cudaStream_t stream);
 // quant_int8_pairs.cu: ConvRot-256 + per-token int8 without a norm in front; false when the shape is not covered.
-bool quantize_int8_rot_pairs(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, cudaStream_t stream);
+bool quantize_int8_rot_pairs(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, cudaStream_t stream, bool overlap = true);
 void add_gated(__nv_bfloat16* x, const __nv_bfloat16* branch, const float* gate, const int32_t* index, int rows,
                int dim, cudaStream_t stream);
 

@@ -41,6 +41,8 @@ void validate_packed_int8(const QuantWeight& w) {
         "W4A8/W6A8 requires group scales, channel scales, compatible codebook and ConvRot-256");
 }
 
+constexpr size_t kDecodeInFront = size_t(8) << 20;  // weights of a W4A8 / W6A8 layer
+
 bool has_dense_form(const QuantWeight& w) {
   switch (w.format) {
     case QuantFormat::kW4A8:
@@ -312,7 +314,14 @@ void LinearRunner::forward(const QuantWeight& w, const __nv_bfloat16* x, int row
     forward_prepared(w, nullptr, x, rows, y, ws);
     return;
   }
-  forward_prepared(w, prepare(w, ws), x, rows, y, ws);
+  const __nv_bfloat16* weight = prepare(w, ws);
+  // the dense form was launched just now (unless the weight is one already): the rotation, if it comes first, runs beside it
+  beside_ = weight != nullptr && w.format != QuantFormat::kBF16;
+  struct Reset {
+    bool& flag;
+    ~Reset() { flag = false; }
+  } reset{beside_};
+  forward_prepared(w, weight, x, rows, y, ws);
 }
 
 void LinearRunner::forward_prepared(const QuantWeight& w, const __nv_bfloat16* weight, const __nv_bfloat16* x,
@@ -327,7 +336,12 @@ void LinearRunner::forward_prepared(const QuantWeight& w, const __nv_bfloat16* w
       run_packed_int8(w, cached_codes_, x, rows, y, ws, nullptr);  // expansion kept by prepare()
       return;
     }
-    // No expansion at hand: decode the weight on the side stream while this one quantizes the activation.
+    // No expansion at hand. A small weight is decoded in front, in a microsecond or two; a larger one on the side stream while
+    // this one quantizes the activation, which costs a fork and a join between streams (about 4 us).
+    if (size_t(w.out_features) * w.in_features <= kDecodeInFront) {
+      run_packed_int8(w, expanded_weight(w, ws, /*keep=*/false, stream_), x, rows, y, ws, nullptr);
+      return;
+    }
     ensure_side_stream();
     auto check = [](cudaError_t e) {
       if (e != cudaSuccess) throw std::runtime_error(std::string("LinearRunner: stream fork failed: ") + cudaGetErrorString(e));
@@ -364,7 +378,7 @@ void LinearRunner::forward_prepared(const QuantWeight& w, const __nv_bfloat16* w
   }
   if (convrot_applies(w)) {
     __nv_bfloat16* xr = ws.alloc_n<__nv_bfloat16>(size_t(rows) * w.in_features);
-    sfq::convrot(xin, xr, rows, w.in_features, w.convrot_group, stream_);
+    sfq::convrot(xin, xr, rows, w.in_features, w.convrot_group, stream_, /*beside=*/beside_ && xin == x);
     xin = xr;
   }
   sfq::GemmArgs g = epilogue_for(w, rows, y, activation_);
@@ -386,7 +400,7 @@ void LinearRunner::run_packed_int8(const QuantWeight& w, const int8_t* codes, co
   int8_t* q = ws.alloc_n<int8_t>(size_t(rows) * w.in_features);
   float* scales = ws.alloc_n<float>(size_t(rows));
   sfq::quantize_int8_token(x, sfq::NormArgs{}, q, scales, nullptr, rows, w.in_features, /*apply_convrot=*/true,
-                           stream_);
+                           stream_, /*overlap=*/codes_ready == nullptr);  // early blocks would take the SMs from the decoder beside it
   if (codes_ready != nullptr) {
     const cudaError_t e = cudaStreamWaitEvent(stream_, codes_ready, 0);
     if (e != cudaSuccess) throw std::runtime_error(std::string("LinearRunner: stream join failed: ") + cudaGetErrorString(e));
@@ -394,6 +408,7 @@ void LinearRunner::run_packed_int8(const QuantWeight& w, const int8_t* codes, co
   sfq::GemmArgs g = epilogue_for(w, rows, y, activation_);
   g.row_scale = scales;
   g.col_scale = w.weight_scale;
+  g.serial_launch = codes_ready != nullptr;
   sfq::gemm_int8(q, codes, g, stream_);
 }
 

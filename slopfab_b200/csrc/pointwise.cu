@@ -54,6 +54,8 @@ __global__ void add_gated_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloa
 // Eight elements per thread, 128-bit accesses; same arithmetic as add_gated_kernel.
 __global__ void add_gated_vec_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,
                                      const float* __restrict__ gate, const int32_t* __restrict__ a, int packs) {
+  grid_dependency_release();
+  branch = grid_dependency_wait(branch);
   const size_t row = blockIdx.x;
   const int p = blockIdx.y * blockDim.x + threadIdx.x;
   if (p >= packs) return;
@@ -140,10 +142,12 @@ void add_gated(__nv_bfloat16* x, const __nv_bfloat16* branch, const float* gate,
   if (!x || !branch || !gate || !index) throw std::invalid_argument("add_gated: null buffer");
   const bool vec = dim % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(branch) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(gate) % 16 == 0;
-  if (vec)
-    add_gated_vec_kernel<<<dim3(rows, (dim / 8 + 127) / 128), 128, 0, stream>>>(x, branch, gate, index, dim / 8);
-  else
+  if (vec) {
+    const cudaError_t e = launch_overlapped(size_t(rows) * dim * 6, add_gated_vec_kernel, dim3(rows, (dim / 8 + 127) / 128), dim3(128), 0, stream, x, branch, gate, index, dim / 8);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("add_gated: ") + cudaGetErrorString(e));
+  } else {
     add_gated_kernel<<<dim3(rows, (dim + 255) / 256), 256, 0, stream>>>(x, branch, gate, index, dim);
+  }
   check_launch("add_gated");
 }
 

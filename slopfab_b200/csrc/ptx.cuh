@@ -31,6 +31,21 @@ __device__ __forceinline__ bool elect_one() {
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
+// ---------------------------------------------------------------- overlapped launches
+// A kernel launched with launch_overlapped() may start while the kernel in front of it in the stream is still running. The
+// first of these returns when everything in front has completed and its writes are visible: it stands before the kernel's
+// first access to memory that an earlier kernel may write or still read. The second lets the next kernel's blocks start
+// once every block of this one has executed it (or left).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The same with a pointer that the loads behind it use: read-only (non-coherent) loads are not ordered by a memory clobber,
+// an address that comes out of the wait is.
+template <class T> __device__ __forceinline__ const T* grid_dependency_wait(const T* p) {
+  grid_dependency_wait();
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));

@@ -16,6 +16,7 @@
 //     NEXT row pair, 92 registers, two CTAs per SM -- was built and measured: 3.04 TB/s against 3.2 for this form at
 //     32768 x 5120, same bits. The kernel is bound by its instruction count, not by warps idling at the barrier.)
 #include "kernels.cuh"
+#include "ptx.cuh"
 #include "runtime.h"
 
 #include <algorithm>
@@ -100,6 +101,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
 quantize_int8_pairs_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ row_scale,
                            int rows, int dim) {
   extern __shared__ __align__(16) uint8_t smem[];
+  ptx::grid_dependency_release();
+  x = ptx::grid_dependency_wait(x);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
   const int chunks = dim >> 4;
@@ -225,6 +228,8 @@ __global__ void __launch_bounds__(wide_max_threads(NC), 2)
 quantize_int8_pairs_wide_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ row_scale,
                                 int rows, int dim) {
   extern __shared__ __align__(16) uint8_t smem[];
+  ptx::grid_dependency_release();
+  x = ptx::grid_dependency_wait(x);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
   f2* tile = reinterpret_cast<f2*>(smem) + (tid >> 4) * kGroupTile;
@@ -324,40 +329,38 @@ quantize_int8_pairs_wide_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __r
 }
 
 template <int NC>
-void launch_pairs_wide(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, int threads, cudaStream_t stream) {
+void launch_pairs_wide(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, int threads, cudaStream_t stream, bool overlap) {
   const size_t smem = size_t(threads / 16) * (kGroupTile * 8 + kGroupBytesOut) + 2 * 32 * sizeof(uint32_t);
   reserve_dynamic_smem(reinterpret_cast<const void*>(&quantize_int8_pairs_wide_kernel<NC>), smem, "quantize_int8_token");
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quantize_int8_pairs_wide_kernel<NC>, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   const int grid = std::min((rows + 1) / 2, per_sm * device_sm_count());
-  quantize_int8_pairs_wide_kernel<NC><<<grid, threads, smem, stream>>>(x, q, row_scale, rows, dim);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_overlapped(overlap ? size_t(rows) * dim * 3 : kNoOverlap, quantize_int8_pairs_wide_kernel<NC>, dim3(grid), dim3(threads), smem, stream, x, q, row_scale, rows, dim);
   if (e != cudaSuccess) throw std::runtime_error(std::string("quantize_int8_token: ") + cudaGetErrorString(e));
 }
 
 template <int MAXT, int MINB>
-void launch_pairs(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, int threads, cudaStream_t stream) {
+void launch_pairs(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, int threads, cudaStream_t stream, bool overlap) {
   const size_t smem = size_t(threads / 16) * (kGroupTile * 8 + kGroupBytesOut) + 2 * 32 * sizeof(uint32_t);
   reserve_dynamic_smem(reinterpret_cast<const void*>(&quantize_int8_pairs_kernel<MAXT, MINB>), smem, "quantize_int8_token");
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quantize_int8_pairs_kernel<MAXT, MINB>, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   const int grid = std::min((rows + 1) / 2, per_sm * device_sm_count());
-  quantize_int8_pairs_kernel<MAXT, MINB><<<grid, threads, smem, stream>>>(x, q, row_scale, rows, dim);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_overlapped(overlap ? size_t(rows) * dim * 3 : kNoOverlap, quantize_int8_pairs_kernel<MAXT, MINB>, dim3(grid), dim3(threads), smem, stream, x, q, row_scale, rows, dim);
   if (e != cudaSuccess) throw std::runtime_error(std::string("quantize_int8_token: ") + cudaGetErrorString(e));
 }
 
 }  // namespace
 
-bool quantize_int8_rot_pairs(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, cudaStream_t stream) {
+bool quantize_int8_rot_pairs(const __nv_bfloat16* x, int8_t* q, float* row_scale, int rows, int dim, cudaStream_t stream, bool overlap) {
   if (dim % 256 != 0 || rows <= 0) return false;
   if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(q) % 16 != 0) return false;
   if (dim > 6144 && dim / 16 <= 1024 && (dim / 16) % 32 == 0) {
     // One chunk per thread in ONE large CTA per SM (864 threads at K = 13824): 3.2 TB/s against 2.9 for the form below with
     // three chunks per thread in two CTAs of 288, whose rotated values of all chunks stay in registers across the barrier.
-    launch_pairs<1024, 1>(x, q, row_scale, rows, dim, dim / 16, stream);
+    launch_pairs<1024, 1>(x, q, row_scale, rows, dim, dim / 16, stream, overlap);
     return true;
   }
   if (dim > 6144) {
@@ -365,18 +368,18 @@ bool quantize_int8_rot_pairs(const __nv_bfloat16* x, int8_t* q, float* row_scale
     const int chunks = dim / 16;
     for (int nc = 2; nc <= 4; ++nc) {
       if (chunks % nc != 0 || (chunks / nc) % 32 != 0 || chunks / nc > wide_max_threads(nc)) continue;
-      if (nc == 2) launch_pairs_wide<2>(x, q, row_scale, rows, dim, chunks / nc, stream);
-      if (nc == 3) launch_pairs_wide<3>(x, q, row_scale, rows, dim, chunks / nc, stream);
-      if (nc == 4) launch_pairs_wide<4>(x, q, row_scale, rows, dim, chunks / nc, stream);
+      if (nc == 2) launch_pairs_wide<2>(x, q, row_scale, rows, dim, chunks / nc, stream, overlap);
+      if (nc == 3) launch_pairs_wide<3>(x, q, row_scale, rows, dim, chunks / nc, stream, overlap);
+      if (nc == 4) launch_pairs_wide<4>(x, q, row_scale, rows, dim, chunks / nc, stream, overlap);
       return true;
     }
     return false;  // the one-row kernel takes it
   }
   const int threads = ((dim / 16 + 31) / 32) * 32;
   if (threads <= 320)
-    launch_pairs<320, 3>(x, q, row_scale, rows, dim, threads, stream);
+    launch_pairs<320, 3>(x, q, row_scale, rows, dim, threads, stream, overlap);
   else
-    launch_pairs<384, 2>(x, q, row_scale, rows, dim, threads, stream);
+    launch_pairs<384, 2>(x, q, row_scale, rows, dim, threads, stream, overlap);
   return true;
 }
 

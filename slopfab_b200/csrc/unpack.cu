@@ -8,6 +8,7 @@
 #include <string>
 
 #include "codec.cuh"
+#include "ptx.cuh"
 
 namespace sfq {
 namespace {
@@ -28,6 +29,7 @@ inline void check_launch(const char* what) {
 __global__ void __launch_bounds__(kThreads)
 unpack_nvfp4_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ scale, float global,
                     __nv_bfloat16* __restrict__ out, int rows, int blocks_per_row) {
+  ptx::grid_dependency_release();
   const size_t g = size_t(blockIdx.x) * kThreads + threadIdx.x;  // one 16-element block
   const size_t total = size_t(rows) * blocks_per_row;
   if (g >= total) return;
@@ -59,6 +61,7 @@ unpack_nvfp4_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict_
 __global__ void __launch_bounds__(kThreads)
 unpack_w4a8_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict__ gscale,
                    const float* __restrict__ codebook, int8_t* __restrict__ out, size_t groups) {
+  ptx::grid_dependency_release();
   __shared__ __align__(16) uint8_t table[256 * 16];
   {
     // thread t builds the row of scale byte t (kThreads == 256): decode the scale once, sixteen products
@@ -116,6 +119,7 @@ unpack_w4a8_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict
 __global__ void __launch_bounds__(kThreads)
 unpack_w6a8_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict__ gscale, int8_t* __restrict__ out,
                    int rows, int width, int group) {
+  ptx::grid_dependency_release();
   const int chunks_per_row = width / 16;
   const size_t c = size_t(blockIdx.x) * kThreads + threadIdx.x;  // 16 consecutive columns of one row
   if (c >= size_t(rows) * chunks_per_row) return;
@@ -157,6 +161,7 @@ unpack_int8_bf16_kernel(const int8_t* __restrict__ src, const float* __restrict_
 __global__ void __launch_bounds__(kThreads)
 unpack_int8_bf16_vec_kernel(const int8_t* __restrict__ src, const float* __restrict__ scale,
                             __nv_bfloat16* __restrict__ dst, size_t packs, int packs_per_row) {
+  ptx::grid_dependency_release();
   const size_t p = size_t(blockIdx.x) * kThreads + threadIdx.x;  // 16 elements
   if (p >= packs) return;
   const float s = __ldg(scale + p / packs_per_row);
@@ -216,6 +221,7 @@ unpack_int8_f16_kernel(const int8_t* __restrict__ codes, const float* __restrict
 // bf16(f8_e4m3(v) * scale), scale a device scalar (dequant_f8_kernel, src/cuda/linear_weights.cu:150-172).
 __global__ void __launch_bounds__(kThreads)
 unpack_f8_kernel(const uint8_t* __restrict__ src, const float* __restrict__ scale, __nv_bfloat16* __restrict__ dst, size_t n) {
+  ptx::grid_dependency_release();
   const size_t i = (size_t(blockIdx.x) * kThreads + threadIdx.x) * 8;
   if (i >= n) return;
   const float s = __ldg(scale);
@@ -273,6 +279,7 @@ __global__ void __launch_bounds__(kThreads)
 unpack_nf4_vec_kernel(const uint8_t* __restrict__ src, const uint8_t* __restrict__ absmax, const float* __restrict__ map,
                       const float* __restrict__ nested_map, const float* __restrict__ nested_absmax, unsigned chunks_per_block,
                       unsigned nested_block, float offset, T* __restrict__ dst, unsigned chunks) {
+  ptx::grid_dependency_release();
   __shared__ float lut[16];
   if (threadIdx.x < 16) lut[threadIdx.x] = map[threadIdx.x];
   __syncthreads();
@@ -297,6 +304,7 @@ unpack_nf4_vec_kernel(const uint8_t* __restrict__ src, const uint8_t* __restrict
 // Eight elements per thread for aligned buffers; the tail of a count that is no multiple of eight goes through to_bf16_kernel.
 // 13824 x 5120 fp16: 45 us (one element per thread 180).
 template <class T> __global__ void __launch_bounds__(kThreads) to_bf16_vec_kernel(const T* __restrict__ src, uint4* __restrict__ dst, size_t packs) {
+  ptx::grid_dependency_release();
   const size_t p = size_t(blockIdx.x) * kThreads + threadIdx.x;
   if (p >= packs) return;
   constexpr int kLoads = sizeof(T) / 2;
