@@ -267,6 +267,13 @@ SFQ_API int sfq_gemm_w4a8_fused(const int8_t* d_q, const uint8_t* d_w_packed, co
 SFQ_API int sfq_gemm_nvfp4(const uint8_t* d_a_packed, const uint8_t* d_a_scale_tiled, const uint8_t* d_w_packed,
                            const uint8_t* d_w_scale_tiled, const sfq_epilogue* ep, void* d_y_bf16,
                            int M, int N, int K, void* stream);
+/* The same product with its result quantized for the next one: what sfq_quantize_nvfp4_block(GEMM_FEED, no norm) makes of
+ * the bf16 y that sfq_gemm_nvfp4 would have stored, byte for byte, without that y. Columns C = N (SFQ_ACT_SWIGLU: N / 2);
+ * d_out_packed [M, C / 2] and d_out_scale_tiled (sfq_nvfp4_act_scale_bytes(M, C)), both 16-byte aligned and not the operand's
+ * buffers. No gated residual. No counterpart in the reference, which quantizes in a launch of its own. */
+SFQ_API int sfq_gemm_nvfp4_quantized(const uint8_t* d_a_packed, const uint8_t* d_a_scale_tiled, const uint8_t* d_w_packed,
+                                     const uint8_t* d_w_scale_tiled, const sfq_epilogue* ep, uint8_t* d_out_packed,
+                                     uint8_t* d_out_scale_tiled, int M, int N, int K, void* stream);
 /* nvfp4_gemm_forward_q with its own operand convention (include/slopfab/cuda/nvfp4_gemm.cuh:101-113): activations as
  * launch_quantize_nvfp4_activations / sfq_quantize_nvfp4_block(REFERENCE) wrote them (low nibble = even element, scales
  * row-major), no bias, no activation. They are converted into the GEMM_FEED layout in stream-ordered scratch that the

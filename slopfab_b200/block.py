@@ -8,13 +8,14 @@ Order of operations of the reference's ``run_block`` (src/dit/transformer_execut
                                                                 fused projection as they lie (or a callable you pass)
     x += gate_msa * (attn Wo^T)                                 NVFP4 Linear, gated residual in its epilogue
     n2 = modulate(rmsnorm(x, norm2), scale_mlp, shift_mlp)      fused with the fp4 quantizer
-    x += gate_mlp * (act(n2 W1^T) W2^T)                         GELU-tanh fused in the first GEMM's epilogue
+    x += gate_mlp * (act(n2 W1^T) W2^T)                         the activation and the fp4 quantizer of the second GEMM's operand
+                                                                fused in the first GEMM's epilogue
 
 Head-wise q/k RMSNorm and MM-RoPE sit between the projections and attention (QK-norm first, then RoPE; v untouched):
 one in-place pass per third of the fused projection, run when the weights carry q_norm / k_norm or `rope` is given.
 The FFN is the plain GELU form of the benchmark configuration by default; `ffn_form="swiglu"` runs the reference's H3
 form instead (src/dit/transformer_execution.cpp:433-441): fc1 is the fused [gate | up] weight with 2 * ffn rows and the
-SwiGLU epilogue writes silu(gate) * up, ffn columns wide, so the [rows, 2 * ffn] intermediate never exists.
+SwiGLU epilogue makes silu(gate) * up, ffn columns wide, so the [rows, 2 * ffn] intermediate never exists.
 """
 from __future__ import annotations
 
@@ -62,12 +63,12 @@ class Nvfp4Block:
         if ffn_form not in ("gelu", "swiglu"):
             raise ValueError("ffn_form must be 'gelu' or 'swiglu'")
         self.rows, self.hidden, self.heads, self.ffn, self.ffn_form = rows, hidden, heads, ffn, ffn_form
-        kmax = max(hidden, ffn)
-        self.xq = torch.empty((rows, kmax // 2), dtype=torch.uint8, device=device)
-        self.xs = torch.empty(lib.sfq_nvfp4_act_scale_bytes(rows, kmax), dtype=torch.uint8, device=device)
+        self.xq = torch.empty((rows, hidden // 2), dtype=torch.uint8, device=device)
+        self.xs = torch.empty(lib.sfq_nvfp4_act_scale_bytes(rows, hidden), dtype=torch.uint8, device=device)
         self.qkv = torch.empty((rows, 3 * hidden), dtype=torch.bfloat16, device=device)
         self.branch = torch.empty((rows, hidden), dtype=torch.bfloat16, device=device)
-        self.h = torch.empty((rows, ffn), dtype=torch.bfloat16, device=device)
+        self.hq = torch.empty((rows, ffn // 2), dtype=torch.uint8, device=device)  # the FFN's hidden activation as fc2 reads it
+        self.hs = torch.empty(lib.sfq_nvfp4_act_scale_bytes(rows, ffn), dtype=torch.uint8, device=device)
         self.linear_ms = 0.0
         self.attn = torch.empty((rows, hidden), dtype=torch.bfloat16, device=device)
         self.attn_ws = None  # V transposed, allocated on first use of the library's own attention
@@ -79,12 +80,20 @@ class Nvfp4Block:
         check(lib.sfq_quantize_nvfp4_block(ptr(x), C.byref(norm) if norm is not None else None, ptr(self.xq), ptr(self.xs),
                                            None, self.rows, dim, NVFP4_ACT_GEMM_FEED, stream_ptr()))
 
-    def _gemm(self, w: Nvfp4Linear, y, act=ACT_NONE, gate=None, gate_index=None):
-        """y = act(x W^T), or with `gate`: y += gate[gate_index] * (x W^T) fused in the epilogue."""
+    def _gemm(self, w: Nvfp4Linear, y, act=ACT_NONE, gate=None, gate_index=None, operand=None):
+        """y = act(x W^T), or with `gate`: y += gate[gate_index] * (x W^T) fused in the epilogue. x is the quantized operand,
+        (self.xq, self.xs) unless given."""
+        xq, xs = operand or (self.xq, self.xs)
         ep = Epilogue(None, None, w.global_scale, None, F32, act, ptr(gate) if gate is not None else None,
                       ptr(gate_index) if gate is not None else None)
-        check(lib.sfq_gemm_nvfp4(ptr(self.xq), ptr(self.xs), ptr(w.data), ptr(w.scale), C.byref(ep), ptr(y), self.rows,
+        check(lib.sfq_gemm_nvfp4(ptr(xq), ptr(xs), ptr(w.data), ptr(w.scale), C.byref(ep), ptr(y), self.rows,
                                  w.out_features, w.in_features, stream_ptr()))
+
+    def _gemm_quantized(self, w: Nvfp4Linear, act):
+        """(self.hq, self.hs) = fp4(act(x W^T)), the operand of the next GEMM."""
+        ep = Epilogue(None, None, w.global_scale, None, F32, act, None, None)
+        check(lib.sfq_gemm_nvfp4_quantized(ptr(self.xq), ptr(self.xs), ptr(w.data), ptr(w.scale), C.byref(ep), ptr(self.hq), ptr(self.hs),
+                                           self.rows, w.out_features, w.in_features, stream_ptr()))
 
     def forward(self, x: torch.Tensor, w: BlockWeights, mod: dict, adaln_index: torch.Tensor, eps: float = 1e-5,
                 attention=None, time_linears: bool = False, rope=None) -> torch.Tensor:
@@ -133,14 +142,12 @@ class Nvfp4Block:
         if self.ffn_form == "swiglu":
             if w.fc1.out_features != 2 * self.ffn:
                 raise ValueError("the SwiGLU form needs fc1 = [gate | up] with 2 * ffn rows")
-            self._gemm(w.fc1, self.h, ACT_SWIGLU)
-        else:
-            self._gemm(w.fc1, self.h, ACT_GELU_TANH)
-        self._quantize(self.h, self.ffn, None)
+        self._gemm_quantized(w.fc1, ACT_SWIGLU if self.ffn_form == "swiglu" else ACT_GELU_TANH)
+        hidden_act = (self.hq, self.hs)
         if self.fuse_residual:
-            self._gemm(w.fc2, x, gate=mod["gate_mlp"], gate_index=adaln_index)
+            self._gemm(w.fc2, x, gate=mod["gate_mlp"], gate_index=adaln_index, operand=hidden_act)
         else:
-            self._gemm(w.fc2, self.branch)
+            self._gemm(w.fc2, self.branch, operand=hidden_act)
             check(lib.sfq_add_gated(ptr(x), ptr(self.branch), ptr(mod["gate_mlp"]), ptr(adaln_index), rows, hidden, stream_ptr()))
         if ev:
             ev[3].record()

@@ -29,6 +29,7 @@
 #include <string>
 
 #include "codec.cuh"
+#include "fp4_block.cuh"
 #include "ptx.cuh"
 
 namespace sfq {
@@ -390,16 +391,6 @@ template <bool HIGH_EVEN> __device__ __forceinline__ uint32_t e2m1_word(const fl
         "f"(v[HIGH_EVEN ? 4 : 5]), "f"(v[HIGH_EVEN ? 5 : 4]), "f"(v[HIGH_EVEN ? 6 : 7]), "f"(v[HIGH_EVEN ? 7 : 6]));
   return w;
 }
-__device__ __forceinline__ uint32_t habs2(uint32_t a) {
-  uint32_t d;
-  asm("abs.bf16x2 %0, %1;" : "=r"(d) : "r"(a));
-  return d;
-}
-__device__ __forceinline__ uint32_t hmax2(uint32_t a, uint32_t b) {
-  uint32_t d;
-  asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
-  return d;
-}
 
 template <int MODE, int MAXP>
 __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_kernel(const FusedArgs args, int total_rows) {
@@ -686,31 +677,6 @@ size_t nvfp4_act_scale_bytes(int rows, int dim) {
 // bf16x2 words and the products on packed fp32 pairs. FEED: high nibble = even element, scales in the 128x4-tiled layout
 // with the rows padded to a multiple of 128 (the pad rows' scales are written as zero).
 namespace {
-template <bool FEED>
-__device__ __forceinline__ void quantize_block16(const uint4 r0, const uint4 r1, uint2& codes, uint8_t& s8) {
-  const uint32_t w[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};  // element 2i in the low half of word i
-  uint32_t m = hmax2(hmax2(hmax2(habs2(w[0]), habs2(w[1])), hmax2(habs2(w[2]), habs2(w[3]))),
-                     hmax2(hmax2(habs2(w[4]), habs2(w[5])), hmax2(habs2(w[6]), habs2(w[7]))));
-  m = hmax2(m, m >> 16);
-  const float amax = __uint_as_float(m << 16);
-  s8 = uint8_t(__nv_cvt_float_to_fp8(amax * (1.0f / 6.0f), __NV_SATFINITE, __NV_E4M3));
-  const float decoded = __half2float(__half(__nv_cvt_fp8_to_halfraw(s8, __NV_E4M3)));
-  const float inv = decoded > 0.0f ? __frcp_rn(decoded) : 0.0f;  // the correctly rounded reciprocal, as 1.0f / decoded
-  const ptx::f32x2 inv2 = ptx::pack2(inv, inv);
-  uint32_t out[2] = {0, 0};
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float even, odd;
-    ptx::unpack2(ptx::mul2(ptx::pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u)), inv2), even, odd);
-    // The conversion puts its first component in the low nibble. The reference layout wants the even element there; the
-    // GEMM feed wants it in the high nibble, like the weight files.
-    const __nv_fp4x2_storage_t b = FEED ? __nv_cvt_float2_to_fp4x2(make_float2(odd, even), __NV_E2M1, cudaRoundNearest)
-                                        : __nv_cvt_float2_to_fp4x2(make_float2(even, odd), __NV_E2M1, cudaRoundNearest);
-    out[i >> 2] |= uint32_t(b) << (8 * (i & 3));
-  }
-  codes = make_uint2(out[0], out[1]);
-}
-
 template <bool FEED>
 __global__ void __launch_bounds__(256) quantize_nvfp4_flat_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ packed,
                                                                   uint8_t* __restrict__ scales, int rows, int padded_rows, int chunks) {

@@ -325,6 +325,19 @@ int sfq_gemm_nvfp4(const uint8_t* d_a_packed, const uint8_t* d_a_scale_tiled, co
     sfq::gemm_nvfp4(d_a_packed, d_w_packed, g, as_stream(stream));
   });
 }
+int sfq_gemm_nvfp4_quantized(const uint8_t* d_a_packed, const uint8_t* d_a_scale_tiled, const uint8_t* d_w_packed,
+                             const uint8_t* d_w_scale_tiled, const sfq_epilogue* ep, uint8_t* d_out_packed, uint8_t* d_out_scale_tiled,
+                             int M, int N, int K, void* stream) {
+  return guarded([&] {
+    if (!d_out_packed || !d_out_scale_tiled) throw std::invalid_argument("sfq_gemm_nvfp4_quantized: null output");
+    sfq::GemmArgs g = to_gemm(ep, nullptr, M, N, K);
+    g.a_scale_tiled = d_a_scale_tiled;
+    g.w_scale_tiled = d_w_scale_tiled;
+    g.q_out = d_out_packed;
+    g.q_scale_tiled = d_out_scale_tiled;
+    sfq::gemm_nvfp4(d_a_packed, d_w_packed, g, as_stream(stream));
+  });
+}
 int sfq_gemm_bf16(const void* d_x_bf16, const void* d_w_bf16, const sfq_epilogue* ep, void* d_y_bf16, int M, int N,
                   int K, void* stream) {
   return guarded([&] {

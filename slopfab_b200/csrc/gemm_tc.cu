@@ -516,8 +516,16 @@ void gemm_nvfp4(const uint8_t* a, const uint8_t* w, const GemmArgs& g, cudaStrea
   if (g.M <= 0 || g.N <= 0) return;
   if (g.K <= 0 || g.K % 64 != 0 || g.N % 128 != 0)
     throw std::invalid_argument("sfq gemm nvfp4: needs K % 64 == 0 and N % 128 == 0 (the scale tiling has no padded form)");
-  if (!a || !w || !g.a_scale_tiled || !g.w_scale_tiled || !g.y || !g.status)
+  if (!a || !w || !g.a_scale_tiled || !g.w_scale_tiled || (!g.y && !g.q_out) || !g.status)
     throw std::invalid_argument("sfq gemm nvfp4: null operand");
+  if (g.q_out != nullptr) {
+    if (g.gate != nullptr) throw std::invalid_argument("sfq gemm nvfp4: the quantized result cannot be combined with the gated residual");
+    if (!g.q_scale_tiled || reinterpret_cast<uintptr_t>(g.q_out) % 16 != 0 || reinterpret_cast<uintptr_t>(g.q_scale_tiled) % 16 != 0)
+      throw std::invalid_argument("sfq gemm nvfp4: the quantized result needs codes and scales, both 16-byte aligned");
+    if (g.q_out == a || g.q_scale_tiled == g.a_scale_tiled) throw std::invalid_argument("sfq gemm nvfp4: the quantized result may not overwrite the operand");
+    if (!gemm_pair_nvfp4(a, w, g, stream)) throw std::runtime_error("sfq gemm nvfp4: the quantized result needs the CTA-pair kernel, which this device cannot schedule");
+    return;
+  }
   // One-CTA form: a 256-wide tile has one accumulator (256 columns + the scale slots); 128-wide tiles have two
   // but feed the tensor pipe less efficiently.
   if (g.act == SFQ_ACT_SWIGLU) {  // only the CTA-pair kernel pairs gate and up columns in one tile

@@ -26,6 +26,10 @@ struct GemmArgs {
   // epilogue would otherwise have stored (launch_add_gated, include/slopfab/cuda/nn_kernels.cuh:64-69)
   const float* gate = nullptr;          // fp32 [*, N]
   const int32_t* gate_index = nullptr;  // int32 [M]
+  // nvfp4, instead of y: the result (behind bias and activation, rounded to bf16) quantized to fp4 per 16 columns in the
+  // GEMM_FEED layout, i.e. the next GEMM's activation operand
+  uint8_t* q_out = nullptr;        // [M, columns / 2], 16-byte aligned
+  uint8_t* q_scale_tiled = nullptr;
   // nvfp4 block scales, both in the 128x4-tiled layout (512-byte tiles, row tile major)
   const uint8_t* a_scale_tiled = nullptr;
   const uint8_t* w_scale_tiled = nullptr;

@@ -19,6 +19,7 @@
 // Every wait is bounded as in the one-CTA kernel; both CTAs meet at a cluster barrier before TMEM is freed, so
 // neither exits while its partner can still read its shared memory or signal its barriers.
 #include "codec.cuh"
+#include "fp4_block.cuh"
 #include "gemm_common.cuh"
 
 namespace sfq {
@@ -54,8 +55,34 @@ template <int KIND, int ACC, bool W4 = false> struct PairCfg {
 };
 
 // EPI selects the epilogue variant at compile time, so the plain store path carries none of the others' registers or
-// branches: 0 = scales / bias / GELU, 1 = + gated residual (read-modify-write of y), 2 = SwiGLU over [gate | up].
-enum { kEpiPlain = 0, kEpiGated = 1, kEpiSwiglu = 2 };
+// branches: 0 = scales / bias / GELU, 1 = + gated residual (read-modify-write of y), 2 = SwiGLU over [gate | up], 3 and 4 =
+// 0 and 2 with the result quantized to fp4 for the next GEMM instead of stored: a thread holds whole 16-column blocks of a row,
+// so the bf16 intermediate (2 x 131 MB of traffic at 4747 x 13824, and the quantizer's launch) never exists. A warp takes
+// neighbouring 32-column chunks there, so that a row's codes fill 32-byte sectors.
+enum { kEpiPlain = 0, kEpiGated = 1, kEpiSwiglu = 2, kEpiQuant = 3, kEpiSwigluQuant = 4 };
+
+// fp4 codes and scales of 32 bf16 columns of one row (two blocks).
+__device__ __forceinline__ void quantize_chunk(const uint4 (&v)[4], uint4& codes, uint32_t& scales) {
+  uint2 c0, c1;
+  uint8_t s0, s1;
+  quantize_block16<true>(v[0], v[1], c0, s0);
+  quantize_block16<true>(v[2], v[3], c1, s1);
+  codes = make_uint4(c0.x, c0.y, c1.x, c1.y);
+  scales = uint32_t(s0) | (uint32_t(s1) << 8);
+}
+
+// The codes of two neighbouring chunks (64 columns) of one row, 32 bytes, and their four scales, one aligned word of the 128x4
+// tiling. Rows past M, up to the end of their 128-row scale tile, get zero scales, as the stand-alone quantizer writes them.
+__device__ __forceinline__ void store_quantized(const GemmArgs& g, int row, int col, int cols, const uint4 (&codes)[2], const uint32_t (&scales)[2]) {
+  const bool row_ok = row < g.M;
+  if (row_ok) {
+    uint4* dst = reinterpret_cast<uint4*>(g.q_out + size_t(row) * (cols / 2) + col / 2);
+    dst[0] = codes[0];
+    dst[1] = codes[1];
+  }
+  if (row < (g.M + 127) / 128 * 128)
+    *reinterpret_cast<uint32_t*>(g.q_scale_tiled + nvfp4_scale_offset(row, col / 16, cols / 16)) = row_ok ? scales[0] | (scales[1] << 16) : 0;
+}
 
 // TAIL: the schedule ends with tiles cut into 128-column halves (see above); without it every tile is 256 wide at
 // compile time.
@@ -80,7 +107,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int tiles_m = (g.M + kPairBM - 1) / kPairBM;
   // SwiGLU epilogue: the weight rows are [gate | up], `inner` each, and a tile pairs 128 gate columns (the leader's
   // weight rows) with the 128 up columns of the same outputs (the peer's), so both meet in one accumulator row.
-  constexpr bool swiglu = EPI == kEpiSwiglu;
+  constexpr bool swiglu = EPI == kEpiSwiglu || EPI == kEpiSwigluQuant;
+  constexpr bool quant = EPI == kEpiQuant || EPI == kEpiSwigluQuant;
+  static_assert(!quant || KIND == kNvfp4, "only the fp4 GEMM emits an fp4 operand");
   const int inner = g.N / 2;
   const int tiles_n = swiglu ? inner / (BN / 2) : (g.N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
@@ -442,12 +471,52 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       }
       uint32_t r[kMaxJ][32];
 #pragma unroll
-      for (int j = 0; j < kMaxJ; ++j)
-        if (half + 2 * j < kTileChunks) tmem_ld_32x32(tbase + (half + 2 * j) * 32, r[j]);
+      for (int j = 0; j < kMaxJ; ++j) {
+        // this warp's j-th chunk; quantizing: neighbours, in the SwiGLU form two of the gate columns, then their up columns
+        const int c = !quant ? half + 2 * j : (swiglu ? (j >> 1) * 4 + half * 2 + (j & 1) : half * (kTileChunks / 2) + j);
+        if (quant && !swiglu ? j < kTileChunks / 2 : c < kTileChunks) tmem_ld_32x32(tbase + c * 32, r[j]);
+      }
       tmem_ld_wait();
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(acc_empty_leader[a]);
+      if constexpr (quant) {
+        uint4 codes[2];
+        uint32_t scales[2];
+        if constexpr (swiglu) {  // r[0], r[1]: gate chunks 2 half, 2 half + 1; r[2], r[3]: their up chunks
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const int c = half * 2 + j;
+            uint4 pg[4], pu[4], po[4];
+            if (has_bias) {
+              pack_chunk<KIND, true, false>(r[j], rs, cs_s + c * 32, bs_s + c * 32, pg);
+              pack_chunk<KIND, true, false>(r[j + 2], rs, cs_s + (c + 4) * 32, bs_s + (c + 4) * 32, pu);
+            } else {
+              pack_chunk<KIND, false, false>(r[j], rs, cs_s + c * 32, bs_s + c * 32, pg);
+              pack_chunk<KIND, false, false>(r[j + 2], rs, cs_s + (c + 4) * 32, bs_s + (c + 4) * 32, pu);
+            }
+            swiglu_chunk(pg, pu, po);
+            quantize_chunk(po, codes[j], scales[j]);
+          }
+          store_quantized(g, row, tn * (BN / 2) + half * 64, inner, codes, scales);
+        } else {
+#pragma unroll
+          for (int j = 0; j < kMaxJ; ++j) {
+            const int c = half * (kTileChunks / 2) + j;
+            if (j >= kTileChunks / 2 || col_base + c * 32 >= g.N) continue;  // N is a multiple of 128: two chunks go together
+            uint4 packed[4];
+            if (!has_bias && g.act == SFQ_ACT_NONE)
+              pack_chunk<KIND, false, false>(r[j], rs, cs_s + c * 32, bs_s + c * 32, packed);
+            else if (g.act == SFQ_ACT_NONE)
+              pack_chunk<KIND, true, false>(r[j], rs, cs_s + c * 32, bs_s + c * 32, packed);
+            else
+              pack_chunk<KIND, true, true>(r[j], rs, cs_s + c * 32, bs_s + c * 32, packed);
+            quantize_chunk(packed, codes[j & 1], scales[j & 1]);
+            if (j & 1) store_quantized(g, row, col_base + (c - 1) * 32, g.N, codes, scales);
+          }
+        }
+        continue;
+      }
       if constexpr (swiglu) {
         // this warp holds gate chunks half, half + 2 (r[0], r[1]) and their up chunks half + 4, half + 6 (r[2], r[3])
 #pragma unroll
@@ -573,7 +642,7 @@ bool launch_pair_epi(const void* a, const void* w, size_t row_bytes, const GemmA
   if (g.act == SFQ_ACT_SWIGLU) {
     if (g.N % kPairBN != 0) throw std::invalid_argument("sfq gemm: the SwiGLU epilogue needs N % 256 == 0 (gate and up halves in 128-column blocks)");
     if (g.gate != nullptr) throw std::invalid_argument("sfq gemm: the SwiGLU epilogue cannot be combined with the gated residual");
-    if (g.ldy != g.N / 2 || reinterpret_cast<uintptr_t>(g.y) % 16 != 0)
+    if (g.q_out == nullptr && (g.ldy != g.N / 2 || reinterpret_cast<uintptr_t>(g.y) % 16 != 0))
       throw std::invalid_argument("sfq gemm: the SwiGLU epilogue writes [M, N/2], 16-byte aligned");
   }
   const int tiles = ((g.M + kPairBM - 1) / kPairBM) * ((g.N + kPairBN - 1) / kPairBN);  // same count with or without SwiGLU
@@ -613,6 +682,11 @@ bool launch_pair_epi(const void* a, const void* w, size_t row_bytes, const GemmA
 
 template <int KIND, int ACC>
 bool launch_pair(const void* a, const void* w, size_t row_bytes, const GemmArgs& g, cudaStream_t stream) {
+  if constexpr (KIND == kNvfp4) {
+    if (g.q_out != nullptr)
+      return g.act == SFQ_ACT_SWIGLU ? launch_pair_epi<KIND, ACC, kEpiSwigluQuant>(a, w, row_bytes, g, stream)
+                                     : launch_pair_epi<KIND, ACC, kEpiQuant>(a, w, row_bytes, g, stream);
+  }
   if (g.act == SFQ_ACT_SWIGLU) return launch_pair_epi<KIND, ACC, kEpiSwiglu>(a, w, row_bytes, g, stream);
   if (g.gate != nullptr) return launch_pair_epi<KIND, ACC, kEpiGated>(a, w, row_bytes, g, stream);
   return launch_pair_epi<KIND, ACC, kEpiPlain>(a, w, row_bytes, g, stream);

@@ -235,6 +235,49 @@ def test_gemm_nvfp4_matches_fp4_activation_oracle(M, N, K, tile_n):
     assert np.all(np.abs(got - ref_) <= 1e-3 + 1e-2 * np.abs(ref_))
 
 
+@pytest.mark.parametrize("act", [sfq.ACT_NONE, sfq.ACT_GELU_TANH, sfq.ACT_SWIGLU])
+@pytest.mark.parametrize("M,N,K", [(1, 256, 64), (128, 256, 128), (129, 512, 320), (300, 384, 1024), (1000, 1280, 512), (4747, 2560, 256),
+                                   (2600, 4992, 192)])
+def test_gemm_nvfp4_quantized_result_equals_gemm_then_quantizer(M, N, K, act):
+    """Codes and scales byte for byte, the zero scales of the padding rows included; bytes past the outputs stay as they were."""
+    if act == sfq.ACT_SWIGLU and N % 256:
+        N += 128
+    g = torch.Generator("cuda").manual_seed(M + N + K)
+    a = torch.randint(0, 256, (M, K // 2), dtype=torch.uint8, device="cuda", generator=g)
+    w = torch.randint(0, 256, (N, K // 2), dtype=torch.uint8, device="cuda", generator=g)
+    pad = (M + 127) // 128 * 128
+    sa = torch.randint(0x30, 0x40, (pad * K // 16,), dtype=torch.uint8, device="cuda", generator=g)
+    sw = torch.randint(0x30, 0x40, (N * K // 16,), dtype=torch.uint8, device="cuda", generator=g)
+    bias = 0.01 * torch.randn(N, device="cuda", generator=g)
+    cols = N // 2 if act == sfq.ACT_SWIGLU else N
+    for db in (None, bias):
+        ep = sfq.Epilogue(None, None, 0.002, sfq.ptr(db) if db is not None else None, sfq.F32, act)
+        y = torch.empty((M, cols), dtype=torch.bfloat16, device="cuda")
+        sfq.check(sfq.lib.sfq_gemm_nvfp4(sfq.ptr(a), sfq.ptr(sa), sfq.ptr(w), sfq.ptr(sw), C.byref(ep), sfq.ptr(y), M, N, K, S))
+        want_q = torch.empty((M, cols // 2), dtype=torch.uint8, device="cuda")
+        want_s = torch.empty(sfq.lib.sfq_nvfp4_act_scale_bytes(M, cols), dtype=torch.uint8, device="cuda")
+        sfq.check(sfq.lib.sfq_quantize_nvfp4_block(sfq.ptr(y), None, sfq.ptr(want_q), sfq.ptr(want_s), None, M, cols, sfq.NVFP4_ACT_GEMM_FEED, S))
+        got_q = torch.full((M * cols // 2 + 256,), 0xA5, dtype=torch.uint8, device="cuda")
+        got_s = torch.full((want_s.numel() + 256,), 0xA5, dtype=torch.uint8, device="cuda")
+        sfq.check(sfq.lib.sfq_gemm_nvfp4_quantized(sfq.ptr(a), sfq.ptr(sa), sfq.ptr(w), sfq.ptr(sw), C.byref(ep), sfq.ptr(got_q), sfq.ptr(got_s),
+                                                   M, N, K, S))
+        _status_clean()
+        assert torch.equal(got_q[:-256].view(M, cols // 2), want_q) and torch.equal(got_s[:-256], want_s)
+        assert bool((got_q[-256:] == 0xA5).all()) and bool((got_s[-256:] == 0xA5).all())
+
+
+def test_gemm_nvfp4_quantized_refusals():
+    z = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
+    o = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda")
+    f = torch.zeros(256, dtype=torch.float32, device="cuda")
+    run = lambda ep, q, s: sfq.lib.sfq_gemm_nvfp4_quantized(sfq.ptr(z), sfq.ptr(z), sfq.ptr(z), sfq.ptr(z), C.byref(ep), q, s, 128, 256, 64, S)  # noqa: E731
+    plain = sfq.Epilogue(None, None, 1.0, None, sfq.F32, sfq.ACT_NONE)
+    assert run(plain, None, sfq.ptr(o)) != 0 and run(plain, sfq.ptr(o), None) != 0
+    assert run(plain, sfq.ptr(z), sfq.ptr(o)) != 0  # over its own operand
+    assert run(plain, sfq.ptr(o) + 8, sfq.ptr(o)) != 0
+    assert run(sfq.Epilogue(None, None, 1.0, None, sfq.F32, sfq.ACT_NONE, sfq.ptr(f), sfq.ptr(f)), sfq.ptr(o), sfq.ptr(o)) != 0
+
+
 @pytest.mark.parametrize("tile_n", [0, 256])
 @pytest.mark.parametrize("M,N,K", [(300, 512, 256), (129, 34, 256), (1000, 1280, 512)])
 def test_gemm_gated_residual_epilogue(M, N, K, tile_n):
