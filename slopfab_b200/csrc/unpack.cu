@@ -19,6 +19,14 @@ inline unsigned blocks_for(size_t n, int per_block) {
   return static_cast<unsigned>((n + per_block - 1) / per_block);
 }
 
+// Calls launch(uint32_t) when `count` items and a grid's overhang fit 32 bits, launch(size_t) otherwise.
+template <class F> void by_index(size_t count, F&& launch) {
+  if (count < (size_t(1) << 32) - kThreads)
+    launch(uint32_t(0));
+  else
+    launch(size_t(0));
+}
+
 inline void check_launch(const char* what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
@@ -26,15 +34,18 @@ inline void check_launch(const char* what) {
 
 // w = bf16( e2m1(nibble) * (e4m3(scale) * global) ), even element in the HIGH nibble,
 // scales in the 128x4-tiled layout (dequant_nvfp4_kernel, src/cuda/linear_weights.cu:216-245).
+// Index: 32 bits whenever the blocks can be counted in them (by_index below). The division by blocks_per_row is most of the
+// arithmetic in the 64-bit form.
+template <class Index>
 __global__ void __launch_bounds__(kThreads)
 unpack_nvfp4_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ scale, float global,
                     __nv_bfloat16* __restrict__ out, int rows, int blocks_per_row) {
   ptx::grid_dependency_release();
-  const size_t g = size_t(blockIdx.x) * kThreads + threadIdx.x;  // one 16-element block
-  const size_t total = size_t(rows) * blocks_per_row;
+  const Index g = Index(blockIdx.x) * kThreads + threadIdx.x;  // one 16-element block
+  const Index total = Index(rows) * Index(blocks_per_row);
   if (g >= total) return;
-  const int row = int(g / blocks_per_row);
-  const int blk = int(g - size_t(row) * blocks_per_row);
+  const int row = int(g / Index(blocks_per_row));
+  const int blk = int(g - Index(row) * Index(blocks_per_row));
   const uint2 raw = __ldg(reinterpret_cast<const uint2*>(data) + g);
   const float s = e4m3_decode(__ldg(scale + nvfp4_scale_offset(row, blk, blocks_per_row))) * global;
   const uint32_t words[2] = {raw.x, raw.y};
@@ -45,7 +56,7 @@ unpack_nvfp4_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict_
     const uint32_t byte = (words[b >> 2] >> (8 * (b & 3))) & 0xFFu;
     op[b] = __floats2bfloat162_rn(e2m1_decode(byte >> 4) * s, e2m1_decode(byte & 15u) * s);
   }
-  uint4* dst = reinterpret_cast<uint4*>(out + g * 16);
+  uint4* dst = reinterpret_cast<uint4*>(out + size_t(g) * 16);
   dst[0] = o[0];
   dst[1] = o[1];
 }
@@ -113,38 +124,51 @@ unpack_w4a8_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict
   for (; g < groups; g += stride) expand(__ldg(reinterpret_cast<const uint2*>(packed) + g), rows[__ldg(gscale + g)], g);
 }
 
+// Four codes (one per byte, 0 .. 63) -> four int8 of clamp(rint((code - 32) * s), -127, 127). No integer / float conversion, which
+// run at a quarter of the rate and bound the first form of this kernel (50 us at 13824 x 5120, 45 now): a byte becomes the float
+// 2^23 + code by a permute, the subtraction of 2^23 + 32 is exact, the product of a 6-bit and a 4-bit significand is exact too, so
+// adding it to 1.5 * 2^23 in one fused step rounds it to the nearest even integer once, which then is the low byte of the sum.
+__device__ __forceinline__ uint32_t expand_w6(uint32_t codes, ptx::f32x2 s2) {
+  const ptx::f32x2 bias = ptx::pack2(-8388640.0f, -8388640.0f), magic = ptx::pack2(12582912.0f, 12582912.0f);
+  uint32_t r[4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float x0 = __uint_as_float(__byte_perm(codes, 0x4B000000u, 0x7440 + 2 * h)), x1 = __uint_as_float(__byte_perm(codes, 0x4B000000u, 0x7441 + 2 * h));
+    float r0, r1;
+    ptx::unpack2(ptx::fma2(ptx::add2(ptx::pack2(x0, x1), bias), s2, magic), r0, r1);
+    r[2 * h] = __float_as_uint(fminf(fmaxf(r0, 12582785.0f), 12583039.0f));
+    r[2 * h + 1] = __float_as_uint(fminf(fmaxf(r1, 12582785.0f), 12583039.0f));
+  }
+  return __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+}
+
 // Row = K/2 low-nibble bytes then K/4 bytes of 2-bit highs (shifts 0,2,4,6);
 // level = code - 32; q = clamp(rint(level * e4m3(scale[(row*K + col) / group])), -127, 127)
 // (dequant_w6_kernel, src/cuda/w4a8.cu:15-29).
+template <class Index>
 __global__ void __launch_bounds__(kThreads)
 unpack_w6a8_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict__ gscale, int8_t* __restrict__ out,
                    int rows, int width, int group) {
   ptx::grid_dependency_release();
-  const int chunks_per_row = width / 16;
-  const size_t c = size_t(blockIdx.x) * kThreads + threadIdx.x;  // 16 consecutive columns of one row
-  if (c >= size_t(rows) * chunks_per_row) return;
+  const Index chunks_per_row = Index(width / 16);
+  const Index c = Index(blockIdx.x) * kThreads + threadIdx.x;  // 16 consecutive columns of one row
+  if (c >= Index(rows) * chunks_per_row) return;
   const int row = int(c / chunks_per_row);
-  const int col0 = int(c - size_t(row) * chunks_per_row) * 16;
+  const int col0 = int(c - Index(row) * chunks_per_row) * 16;
   const uint8_t* rowp = packed + size_t(row) * (size_t(width) * 3 / 4);
   const uint2 lo = __ldg(reinterpret_cast<const uint2*>(rowp + col0 / 2));
   const uint32_t hi = __ldg(reinterpret_cast<const uint32_t*>(rowp + width / 2 + col0 / 4));
-  const float s = e4m3_decode(__ldg(gscale + (size_t(row) * width + col0) / group));
-  const uint32_t words[2] = {lo.x, lo.y};
+  float s = e4m3_decode(__ldg(gscale + c / Index(group / 16)));
+  if (s != s) s = 0.0f;  // NaN scale bytes never occur in valid files; the reference's integer conversion makes them 0
+  const ptx::f32x2 s2 = ptx::pack2(s, s);
   uint32_t o[4];
 #pragma unroll
   for (int w = 0; w < 4; ++w) {
-    uint32_t acc = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int e = w * 4 + j;
-      const uint32_t byte = (words[e >> 3] >> (8 * ((e >> 1) & 3))) & 0xFFu;
-      const uint32_t low = (e & 1) ? (byte >> 4) : (byte & 15u);
-      const uint32_t high = (hi >> (2 * e)) & 3u;  // byte e/4, shift (e&3)*2
-      const int level = int(low | (high << 4)) - 32;
-      const int q = max(-127, min(127, __float2int_rn(float(level) * s)));
-      acc |= uint32_t(uint8_t(q)) << (8 * j);
-    }
-    o[w] = acc;
+    const uint32_t nib = (w & 1 ? (w & 2 ? lo.y : lo.x) >> 16 : (w & 2 ? lo.y : lo.x)) & 0xFFFFu;  // elements 4w .. 4w+3
+    const uint32_t low = __byte_perm(nib & 0x0F0Fu, (nib >> 4) & 0x0F0Fu, 0x5140);
+    const uint32_t h = (hi >> (8 * w)) & 0xFFu;
+    const uint32_t high = ((h << 4) & 0x30u) | ((h << 10) & 0x3000u) | ((h << 16) & 0x300000u) | ((h << 22) & 0x30000000u);
+    o[w] = expand_w6(low | high, s2);
   }
   *reinterpret_cast<uint4*>(out + size_t(row) * width + col0) = make_uint4(o[0], o[1], o[2], o[3]);
 }
@@ -158,11 +182,12 @@ unpack_int8_bf16_kernel(const int8_t* __restrict__ src, const float* __restrict_
   if (i >= total) return;
   dst[i] = __float2bfloat16(float(src[i]) * scale[i / cols]);
 }
+template <class Index>
 __global__ void __launch_bounds__(kThreads)
 unpack_int8_bf16_vec_kernel(const int8_t* __restrict__ src, const float* __restrict__ scale,
-                            __nv_bfloat16* __restrict__ dst, size_t packs, int packs_per_row) {
+                            __nv_bfloat16* __restrict__ dst, Index packs, Index packs_per_row) {
   ptx::grid_dependency_release();
-  const size_t p = size_t(blockIdx.x) * kThreads + threadIdx.x;  // 16 elements
+  const Index p = Index(blockIdx.x) * kThreads + threadIdx.x;  // 16 elements
   if (p >= packs) return;
   const float s = __ldg(scale + p / packs_per_row);
   const uint4 raw = __ldg(reinterpret_cast<const uint4*>(src) + p);
@@ -171,7 +196,7 @@ unpack_int8_bf16_vec_kernel(const int8_t* __restrict__ src, const float* __restr
   __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(o);
 #pragma unroll
   for (int j = 0; j < 8; ++j) op[j] = __floats2bfloat162_rn(float(b[2 * j]) * s, float(b[2 * j + 1]) * s);
-  uint4* d = reinterpret_cast<uint4*>(dst + p * 16);
+  uint4* d = reinterpret_cast<uint4*>(dst + size_t(p) * 16);
   d[0] = o[0];
   d[1] = o[1];
 }
@@ -401,8 +426,9 @@ void unpack_nvfp4_bf16(const uint8_t* data, const uint8_t* scale, float global, 
     throw std::runtime_error("unpack_nvfp4: " + std::to_string(out_features) + "x" + std::to_string(in_features) +
                              " does not tile the 128x4 block-scale layout (needs out % 128 == 0 and in % 64 == 0)");
   const size_t groups = size_t(out_features) * (in_features / 16);
-  unpack_nvfp4_kernel<<<blocks_for(groups, kThreads), kThreads, 0, stream>>>(data, scale, global, out, out_features,
-                                                                            in_features / 16);
+  by_index(groups, [&](auto index) {
+    unpack_nvfp4_kernel<decltype(index)><<<blocks_for(groups, kThreads), kThreads, 0, stream>>>(data, scale, global, out, out_features, in_features / 16);
+  });
   check_launch("unpack_nvfp4");
 }
 
@@ -426,8 +452,10 @@ void unpack_w6a8_int8(const int8_t* packed, const uint8_t* gscale, int8_t* out, 
       group % 16 || in_features % group)
     throw std::invalid_argument("W6A8 weight decode: invalid buffers or dimensions");
   const size_t chunks = size_t(out_features) * (in_features / 16);
-  unpack_w6a8_kernel<<<blocks_for(chunks, kThreads), kThreads, 0, stream>>>(reinterpret_cast<const uint8_t*>(packed),
-                                                                           gscale, out, out_features, in_features, group);
+  by_index(chunks, [&](auto index) {
+    unpack_w6a8_kernel<decltype(index)><<<blocks_for(chunks, kThreads), kThreads, 0, stream>>>(reinterpret_cast<const uint8_t*>(packed), gscale, out,
+                                                                                              out_features, in_features, group);
+  });
   check_launch("unpack_w6a8");
 }
 
@@ -437,8 +465,10 @@ void unpack_int8_bf16(const int8_t* codes, const float* scale, __nv_bfloat16* ou
   if (!codes || !scale || !out) throw std::invalid_argument("unpack_int8: null buffer");
   const size_t n = size_t(out_features) * in_features;
   if (in_features % 16 == 0 && reinterpret_cast<uintptr_t>(codes) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0)
-    unpack_int8_bf16_vec_kernel<<<blocks_for(n / 16, kThreads), kThreads, 0, stream>>>(codes, scale, out, n / 16,
-                                                                                     in_features / 16);
+    by_index(n / 16, [&](auto index) {
+      using Index = decltype(index);
+      unpack_int8_bf16_vec_kernel<Index><<<blocks_for(n / 16, kThreads), kThreads, 0, stream>>>(codes, scale, out, Index(n / 16), Index(in_features / 16));
+    });
   else
     unpack_int8_bf16_kernel<<<blocks_for(n, kThreads), kThreads, 0, stream>>>(codes, scale, out, out_features, in_features);
   check_launch("unpack_int8");
