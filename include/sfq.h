@@ -444,8 +444,8 @@ SFQ_API int sfq_head_norm_rope(void* d_x_bf16, int ld, const void* d_norm_weight
  * no causality. q and out may be a compact chunk of the sequence's rows (seq_q <= seq_kv is not required); k and v
  * are the whole sequence, [seq_kv, kv_heads*128]; query head h reads key/value head h / (heads / kv_heads). The
  * three leading dimensions are in elements, so the thirds of a fused QKV projection are passed as they lie
- * (ld = 3 * heads * 128). scale <= 0 selects 1/sqrt(128). The workspace (sfq_attention_workspace_bytes) holds V
- * transposed. out may not alias the inputs. Parity: the reference's own bound against a dense fp64 softmax,
+ * (ld = 3 * heads * 128). scale <= 0 selects 1/sqrt(128). The workspace (sfq_attention_workspace_bytes) takes V
+ * transposed when its rows do not start on 16 bytes. out may not alias the inputs. Parity: the reference's own bound against a dense fp64 softmax,
  * |err| <= 1e-3 + 1e-2 |want| (tests/test_nn_kernels_attention_synthetic.cu:40). */
 SFQ_API int sfq_attention_workspace_bytes(int seq_kv, int kv_heads, int head_dim, size_t* out);
 SFQ_API int sfq_attention_forward(const void* d_q_bf16, int ld_q, const void* d_k_bf16, const void* d_v_bf16, int ld_kv,

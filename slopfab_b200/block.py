@@ -71,7 +71,7 @@ class Nvfp4Block:
         self.hs = torch.empty(lib.sfq_nvfp4_act_scale_bytes(rows, ffn), dtype=torch.uint8, device=device)
         self.linear_ms = 0.0
         self.attn = torch.empty((rows, hidden), dtype=torch.bfloat16, device=device)
-        self.attn_ws = None  # V transposed, allocated on first use of the library's own attention
+        self.attn_ws = None  # the attention's workspace, allocated on its first use
         # True: x += gate * branch inside the out / fc2 GEMM epilogues (same bits; measured 3 % slower per block than the
         # separate add_gated kernel at 75600 tokens, because the single-accumulator nvfp4 epilogue then waits on x)
         self.fuse_residual = False

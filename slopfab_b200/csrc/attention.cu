@@ -6,14 +6,14 @@
 //
 // One CTA owns TWO tiles of 128 queries of one head and walks the keys in tiles of 128 with an online softmax, so that the
 // softmax of one query tile runs while the tensor pipe works on the other tile's products:
-//   warp 0      TMA producer: both Q tiles once, then a two-stage ring of K tiles [128 keys x 128 d] and V^T tiles
-//               [128 d x 128 keys]; V is transposed once per call by transpose_v_kernel so that both products are
-//               K-major x K-major, the operand form the GEMM kernels already use
+//   warp 0      TMA producer: both Q tiles once, then a two-stage ring of K and V tiles [128 keys x 128 d]. The second product
+//               reads V as it lies, as an N-major operand (its N is d, its K the keys), or - VT, where its rows are not aligned -
+//               V transposed once per call by transpose_v_kernel, [128 d x 128 keys], K-major like the other operands
 //   warp 1      issues, per key tile j: O0 += P0(j) V(j), S0 = Q0 K(j+1)^T, O1 += P1(j) V(j), S1 = Q1 K(j+1)^T (8 MMAs
 //               128x128x16 each; the product with V in two parts, as its probabilities arrive). S and O of both query tiles live in TMEM (4 x 128 columns); P is read by the second
 //               product straight from TMEM, where it overwrites the first 64 columns of the scores it was computed from
 //   warps 4-7   softmax of query tile 0, warps 8-11 of query tile 1 (warps 2-3 only hand their registers over: the
-//               softmax warpgroups run with 216 registers, the first warpgroup with 56), one query row per thread with all 128 keys of the
+//               softmax warpgroups run with 232 registers, the first warpgroup with 40), one query row per thread with all 128 keys of the
 //               tile: S from TMEM, P = exp2(s - m) as bf16 pairs back into TMEM, the running sum, and - only when the
 //               part's probabilities sum to more than 2^15, i.e. the row has outgrown the reference maximum m the
 //               accumulator was last scaled to - the true running maximum, a rescale of O in TMEM and the tile's
@@ -44,7 +44,8 @@ constexpr int kTile = 128;             // queries per query tile (two per CTA), 
 constexpr int kSlab = kTile * 128;     // 128 rows x 128 bytes: 64 bf16 columns of a tile
 constexpr int kTileBytes = 2 * kSlab;  // [128 x 128] bf16
 constexpr int kAttnThreads = 384;  // warpgroup 0: producer, MMA issuer, two idle warps; warpgroups 1 and 2: the softmax of query tiles 0 and 1
-constexpr int kAttnRegsLean = 56, kAttnRegsSoftmax = 216;  // after setmaxnreg: 128 x 56 + 256 x 216 <= 65536
+constexpr int kAttnRegsLean = 40, kAttnRegsSoftmax = 232;  // after setmaxnreg: 128 x 40 + 256 x 232 = 384 x 168, what the launch allocates (56 / 216: 1.3 % slower)
+constexpr int kTailWaves = 16;
 constexpr float kTileSumLimit = 32768.0f;  // a key tile's 128 probabilities may sum to this before the reference maximum moves
 
 struct AttnShared {
@@ -58,6 +59,8 @@ struct AttnArgs {
   __nv_bfloat16* out;
   int ld_out;
   int seq_q, seq_kv;
+  int q_blocks;  // blocks of 256 queries per head
+  int whole;     // the first `whole` CTAs take a (block, head) each; behind them a unit is two CTAs, one per query tile
   int group;         // query heads per key/value head
   float scale_log2;  // scale * log2(e)
   int* status;
@@ -122,9 +125,12 @@ __device__ __forceinline__ f32x2 exp2_pair_fma(f32x2 x) {
 constexpr int kFirstChunks = 3;
 constexpr int kFmaPairsOfFour = 1;  // of every four pairs of probabilities, how many take the FMA-pipe exponential
 
+// TAIL: the units of the last wave run as CTAs of one query tile each (see attention_forward). Without it every CTA has two
+// tiles at compile time and the grid is (blocks of 256 queries, heads).
+template <bool VT, bool TAIL>
 __global__ void __launch_bounds__(kAttnThreads, 1)
     attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                     const __grid_constant__ CUtensorMap map_vt, const AttnArgs g) {
+                     const __grid_constant__ CUtensorMap map_v, const AttnArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_s = smem;                    // two query tiles
@@ -133,8 +139,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   AttnShared* sh = reinterpret_cast<AttnShared*>(smem + 6 * kTileBytes);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q0 = blockIdx.x * (2 * kTile);
-  const int head = blockIdx.y;
+  const int tail_cta = TAIL ? int(blockIdx.x) - g.whole : -1;
+  const int unit = tail_cta < 0 ? int(blockIdx.x) : g.whole + (tail_cta >> 1);
+  const int q0 = (TAIL ? unit % g.q_blocks : unit) * (2 * kTile) + (tail_cta < 0 ? 0 : (tail_cta & 1) * kTile);
+  const int head = TAIL ? unit / g.q_blocks : int(blockIdx.y);
+  if (TAIL && q0 >= g.seq_q) return;  // the second half of a split block may have no queries
+  const bool two = !TAIL || (tail_cta < 0 && q0 + kTile < g.seq_q);  // otherwise query tile 0 alone
   const int kv_head = head / g.group;
   const int tiles = (g.seq_kv + kTile - 1) / kTile;
 
@@ -155,7 +165,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     fence_barrier_init();
     prefetch_tensormap(&map_q);
     prefetch_tensormap(&map_k);
-    prefetch_tensormap(&map_vt);
+    prefetch_tensormap(&map_v);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&sh->tmem_base), 512);
@@ -174,8 +184,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
-      mbar_arrive_expect_tx(smem_u32(&sh->q_full), 2 * kTileBytes);
-      for (int t = 0; t < 2; ++t) {
+      mbar_arrive_expect_tx(smem_u32(&sh->q_full), (two ? 2 : 1) * kTileBytes);
+      for (int t = 0; t < (two ? 2 : 1); ++t) {
         tma_load_2d(smem_u32(q_s + t * kTileBytes), &map_q, head * 256, q0 + t * kTile, smem_u32(&sh->q_full));
         tma_load_2d(smem_u32(q_s + t * kTileBytes + kSlab), &map_q, head * 256 + 128, q0 + t * kTile, smem_u32(&sh->q_full));
       }
@@ -188,9 +198,13 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         tma_load_2d(smem_u32(k_s + st * kTileBytes + kSlab), &map_k, kv_head * 256 + 128, j * kTile, smem_u32(&sh->k_full[st]));
         if (!attn_wait<200>(smem_u32(&sh->v_empty[st]), ph, sh, g.status, 12)) break;
         mbar_arrive_expect_tx(smem_u32(&sh->v_full[st]), kTileBytes);
-        // V^T: rows are (kv_head, d), columns are keys; 64 keys = 128 bytes per slab
-        tma_load_2d(smem_u32(v_s + st * kTileBytes), &map_vt, j * 256, kv_head * kTile, smem_u32(&sh->v_full[st]));
-        tma_load_2d(smem_u32(v_s + st * kTileBytes + kSlab), &map_vt, j * 256 + 128, kv_head * kTile, smem_u32(&sh->v_full[st]));
+        if (VT) {  // rows are (kv_head, d), columns are keys; 64 keys = 128 bytes per slab
+          tma_load_2d(smem_u32(v_s + st * kTileBytes), &map_v, j * 256, kv_head * kTile, smem_u32(&sh->v_full[st]));
+          tma_load_2d(smem_u32(v_s + st * kTileBytes + kSlab), &map_v, j * 256 + 128, kv_head * kTile, smem_u32(&sh->v_full[st]));
+        } else {
+          tma_load_2d(smem_u32(v_s + st * kTileBytes), &map_v, kv_head * 256, j * kTile, smem_u32(&sh->v_full[st]));
+          tma_load_2d(smem_u32(v_s + st * kTileBytes + kSlab), &map_v, kv_head * 256 + 128, j * kTile, smem_u32(&sh->v_full[st]));
+        }
       }
     }
   } else if (warp == 1) {
@@ -213,23 +227,27 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       tc_fence_after_sync();
       if (elect_one())  // eight MMAs, the commit for the softmax warps and, behind the second query tile, the one that frees K
         mma_f16_x8_commit(tmem + t * kTile, smem_desc_sw128(smem_u32(q_s + t * kTileBytes)), smem_desc_sw128(smem_u32(k_s + st * kTileBytes)),
-                          idesc, 0u, kSlab >> 4, smem_u32(&sh->s_full[t]), smem_u32(&sh->k_empty[st]), t == 1 ? 1u : 0u);
+                          idesc, 0u, kSlab >> 4, smem_u32(&sh->s_full[t]), smem_u32(&sh->k_empty[st]), t == int(two) ? 1u : 0u);
       __syncwarp();
       return true;
     };
     // O_t += P_t V_j in two parts: the keys of the first chunks of probabilities as soon as those are written, the rest
     // when the last chunk is. A = P_t in tensor memory [queries x keys], 16 keys (eight 32-bit columns of bf16 pairs) per
-    // MMA; B = V^T [d x keys].
+    // MMA; B = V [keys x d], N-major (16 keys are two groups of eight 128-byte rows), or V^T [d x keys] (four MMAs per slab of
+    // 64 keys, 32 bytes of each row apiece).
+    constexpr uint32_t idesc_pv = VT ? idesc : idesc | kIdescBMajorN;
+    constexpr uint64_t kStep = VT ? 2 : 16 * 128 >> 4;                    // 16 keys on
+    constexpr uint64_t kKeys64 = VT ? uint64_t(kSlab >> 4) : 4 * kStep;   // 64 keys on
     auto issue_pv = [&](int t, int j, bool more) {
       const int st = j & 1;
       const uint32_t d = tmem + 2 * kTile + t * kTile, a = tmem + t * kTile;
-      const uint64_t b0 = smem_desc_sw128(smem_u32(v_s + st * kTileBytes)), b1 = b0 + (kSlab >> 4);
+      const uint64_t b = VT ? smem_desc_sw128(smem_u32(v_s + st * kTileBytes)) : smem_desc_sw128_mn(smem_u32(v_s + st * kTileBytes), kSlab);
       if (t == 0 && !wait(&sh->v_full[st], (j >> 1) & 1, 16)) return false;
       if (!wait(&sh->p_part[t], j & 1, 17)) return false;
       tc_fence_after_sync();
       if (elect_one()) {
-        mma_f16_ts_x4(d, a, b0, idesc, j ? 1u : 0u);
-        if (kFirstChunks == 3) mma_f16_ts_x2(d, a + 32, b1, idesc, 1u);
+        mma_f16_ts_x4<kStep>(d, a, b, idesc_pv, j ? 1u : 0u);
+        if (kFirstChunks == 3) mma_f16_ts_x2<kStep>(d, a + 32, b + kKeys64, idesc_pv, 1u);
         tc_commit(smem_u32(&sh->pv_part[t]));
       }
       __syncwarp();
@@ -237,19 +255,19 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       tc_fence_after_sync();
       if (elect_one()) {
         if (kFirstChunks == 3)
-          mma_f16_ts_x2(d, a + 48, b1 + 4, idesc, 1u);
+          mma_f16_ts_x2<kStep>(d, a + 48, b + kKeys64 + 2 * kStep, idesc_pv, 1u);
         else
-          mma_f16_ts_x4(d, a + 32, b1, idesc, 1u);
-        if (t == 1) tc_commit(smem_u32(&sh->v_empty[st]));
+          mma_f16_ts_x4<kStep>(d, a + 32, b + kKeys64, idesc_pv, 1u);
+        if (t == int(two)) tc_commit(smem_u32(&sh->v_empty[st]));
         if (!more) tc_commit(smem_u32(&sh->pv_done[t]));
       }
       __syncwarp();
       return true;
     };
-    if (ok) ok = issue_s(0, 0) && issue_s(1, 0);
+    if (ok) ok = issue_s(0, 0) && (!two || issue_s(1, 0));
     for (int j = 0; j < tiles && ok; ++j) {
       const bool more = j + 1 < tiles;
-      ok = issue_pv(0, j, more) && (!more || issue_s(0, j + 1)) && issue_pv(1, j, more) && (!more || issue_s(1, j + 1));
+      ok = issue_pv(0, j, more) && (!more || issue_s(0, j + 1)) && (!two || (issue_pv(1, j, more) && (!more || issue_s(1, j + 1))));
     }
   }
   } else {
@@ -336,7 +354,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       unpack2(sum2, a, b);
       return a + b;
     };
-    for (int j = 0; j < tiles; ++j) {
+    const int my_tiles = t == 0 || two ? tiles : 0;
+    for (int j = 0; j < my_tiles; ++j) {
       if (!(ok = __all_sync(0xffffffffu, attn_wait<40>(smem_u32(&sh->s_full[t]), j & 1, sh, g.status, 18)))) break;
       tc_fence_after_sync();
       const int valid = g.seq_kv - j * kTile;  // keys of this tile that exist
@@ -396,7 +415,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       l += part_sum;
       publish(&sh->p_full[t]);
     }
-    if (ok && (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_done[t]), 0, sh, g.status, 20)))) {
+    if (ok && my_tiles > 0 && (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_done[t]), 0, sh, g.status, 20)))) {
       tc_fence_after_sync();
       const float inv = 1.0f / l;
       const int qrow = q0 + t * kTile + row;
@@ -492,23 +511,45 @@ void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k,
     throw std::invalid_argument("sfq attention: row pitches must cover heads * 128 columns and keep 16-byte alignment");
   if (workspace_bytes < attention_workspace_bytes(seq_kv, kv_heads, head_dim)) throw std::invalid_argument("sfq attention: workspace too small");
   if (out == q || out == k || out == v) throw std::invalid_argument("sfq attention: out may not alias q, k or v");
-  if ((seq_q + kTile - 1) / kTile > 0x7FFFFFFF / 2 || heads > 65535) throw std::invalid_argument("sfq attention: too many query tiles or heads");
-  reserve_dynamic_smem(reinterpret_cast<const void*>(&attention_kernel), kAttnSmem, "sfq attention");
+  if ((seq_q + kTile - 1) / kTile > 0x7FFFFFFF / 2 || heads > 65535 || (long long)((seq_q + 2 * kTile - 1) / (2 * kTile)) * heads > 0x3FFFFFFF) throw std::invalid_argument("sfq attention: too many query tiles or heads");
+  for (auto kernel : {attention_kernel<false, false>, attention_kernel<false, true>, attention_kernel<true, false>, attention_kernel<true, true>})
+    reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), kAttnSmem, "sfq attention");
 
-  const int ld_t = padded_keys(seq_kv);
+  // V is read as it lies, except one whose rows do not start on 16 bytes, which TMA cannot read: that one is transposed first.
+  // 40 heads in loops of 0.4 s, as it lies against transposed (pass included): 2048 tokens 0.106 / 0.136 ms, 4747 0.499 / 0.548,
+  // 18900 6.60 / 6.79, 75600 102.0 / 102.4.
+  const bool transposed = reinterpret_cast<uintptr_t>(v) % 16 != 0;
+  cudaError_t e = cudaSuccess;
+  const int width = kv_heads * kTile, ld_t = padded_keys(seq_kv);
+  const size_t kv_bytes = size_t(seq_kv) * width * 4;
   __nv_bfloat16* vt = static_cast<__nv_bfloat16*>(workspace);
-  const int width = kv_heads * kTile;
-  cudaError_t e = launch_overlapped(size_t(seq_kv) * width * 4, transpose_v_kernel, dim3((ld_t + 63) / 64, (width + 63) / 64), dim3(256), 0, stream, v, ld_kv, vt, ld_t, seq_kv, width);
-  if (e != cudaSuccess) throw std::runtime_error(std::string("sfq attention: launch failed: ") + cudaGetErrorString(e));
+  if (transposed) {
+    e = launch_overlapped(kv_bytes, transpose_v_kernel, dim3((ld_t + 63) / 64, (width + 63) / 64), dim3(256), 0, stream, v, ld_kv, vt, ld_t, seq_kv, width);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("sfq attention: launch failed: ") + cudaGetErrorString(e));
+  }
 
   const CUtensorMap mq = make_attn_map(q, size_t(seq_q), size_t(heads) * kTile, size_t(ld_q));
-  const CUtensorMap mk = make_attn_map(k, size_t(seq_kv), size_t(kv_heads) * kTile, size_t(ld_kv));
-  const CUtensorMap mv = make_attn_map(vt, size_t(width), size_t(ld_t), size_t(ld_t));
+  const CUtensorMap mk = make_attn_map(k, size_t(seq_kv), size_t(width), size_t(ld_kv));
+  const CUtensorMap mv = transposed ? make_attn_map(vt, size_t(width), size_t(ld_t), size_t(ld_t)) : make_attn_map(v, size_t(seq_kv), size_t(width), size_t(ld_kv));
   AttnArgs a;
   a.out = out, a.ld_out = ld_out, a.seq_q = seq_q, a.seq_kv = seq_kv, a.group = heads / kv_heads;
   a.scale_log2 = (scale > 0.0f ? scale : 1.0f / sqrtf(float(head_dim))) * 1.4426950408889634f;
   a.status = device_status_word();
-  e = launch_overlapped(size_t(seq_kv) * width * 4, attention_kernel, dim3((seq_q + 2 * kTile - 1) / (2 * kTile), heads), dim3(kAttnThreads), kAttnSmem, stream, mq, mk, mv, a);
+  // Units (256 queries of a head) run one per SM, all equally long, so a last wave that is nearly empty costs as much as a full
+  // one: 4747 tokens x 40 heads are 760 units = 5.14 waves of 148. When the last wave's units fit the SMs twice over, they run
+  // as two CTAs of one query tile each, which take about 0.6 of the time (a query tile alone has no other tile to share the
+  // tensor pipe with). A row's arithmetic is the same either way. Past kTailWaves waves there is less to gain than the
+  // bookkeeping costs (1.4 % at 75600 tokens x 40 heads, 80 waves).
+  a.q_blocks = (seq_q + 2 * kTile - 1) / (2 * kTile);
+  const int units = a.q_blocks * heads, sms = device_sm_count(), rest = units % sms;
+  const int split = 2 * rest <= sms && units < kTailWaves * sms && seq_q > kTile ? rest : 0;
+  a.whole = units - split;
+  if (split > 0)
+    e = launch_overlapped(kv_bytes, transposed ? attention_kernel<true, true> : attention_kernel<false, true>, dim3(units + split), dim3(kAttnThreads), kAttnSmem,
+                          stream, mq, mk, mv, a);
+  else
+    e = launch_overlapped(kv_bytes, transposed ? attention_kernel<true, false> : attention_kernel<false, false>, dim3(a.q_blocks, heads), dim3(kAttnThreads),
+                          kAttnSmem, stream, mq, mk, mv, a);
   if (e != cudaSuccess) throw std::runtime_error(std::string("sfq attention: launch failed: ") + cudaGetErrorString(e));
 }
 

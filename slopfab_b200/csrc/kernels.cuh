@@ -86,7 +86,7 @@ void adaln_expand(const float* w, const float* bias, const float* code, float* o
 
 // Full self-attention, head_dim 128 (attention.cu). q: [seq_q, heads*128] with row pitch ld_q; k, v: [seq_kv, kv_heads*128]
 // with row pitch ld_kv; out: [seq_q, heads*128] with row pitch ld_out. scale <= 0 selects 1/sqrt(head_dim). The workspace
-// holds V^T (attention_workspace_bytes).
+// takes V^T when V's rows do not start on 16 bytes (attention_workspace_bytes).
 size_t attention_workspace_bytes(int seq_kv, int kv_heads, int head_dim);
 void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k, const __nv_bfloat16* v, int ld_kv, __nv_bfloat16* out, int ld_out,
                        int seq_q, int seq_kv, int heads, int kv_heads, int head_dim, float scale, void* workspace, size_t workspace_bytes,

@@ -184,28 +184,28 @@ __device__ __forceinline__ void mma_f16_x8_commit(uint32_t d, uint64_t a, uint64
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate_first), "r"(slab16), "r"(bar1), "r"(bar2), "r"(commit2)
       : "memory");
 }
-// The `_ts` forms: A in tensor memory, COUNT (2 or 4) K = 16 steps inside one 128-byte slab of B, no commit.
-__device__ __forceinline__ void mma_f16_ts_x4(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate_first) {
+// The `_ts` forms: A in tensor memory, two or four K = 16 steps, B advancing by STEP 16-byte units, no commit.
+template <uint64_t STEP> __device__ __forceinline__ void mma_f16_ts_x4(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate_first) {
   asm volatile(
       "{\n\t.reg .pred p, pt;\n\t.reg .b64 b1, b2, b3;\n\t.reg .b32 a1, a2, a3;\n\t"
       "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
       "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
-      "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\t"
+      "add.s64 b1, %2, %5;\n\tadd.s64 b2, b1, %5;\n\tadd.s64 b3, b2, %5;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, pt;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, pt;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, pt;\n\t}" ::"r"(d),
-      "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate_first)
+      "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate_first), "n"(STEP)
       : "memory");
 }
-__device__ __forceinline__ void mma_f16_ts_x2(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate_first) {
+template <uint64_t STEP> __device__ __forceinline__ void mma_f16_ts_x2(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate_first) {
   asm volatile(
       "{\n\t.reg .pred p, pt;\n\t.reg .b64 b1;\n\t.reg .b32 a1;\n\t"
       "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
-      "add.u32 a1, %1, 8;\n\tadd.s64 b1, %2, 2;\n\t"
+      "add.u32 a1, %1, 8;\n\tadd.s64 b1, %2, %5;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, pt;\n\t}" ::"r"(d),
-      "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate_first)
+      "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate_first), "n"(STEP)
       : "memory");
 }
 // Block-scaled e2m1 x e2m1, one ue4m3 scale per 16 elements (four per K=64 instruction).
@@ -480,6 +480,12 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
   return uint64_t((saddr >> 4) & 0x3FFFu) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61);
 }
+// The same bytes -- rows of 128 bytes, 128-byte swizzle -- read with the rows along K: 64 consecutive 16-bit elements of N per
+// row, the next 64 one slab of `slab` bytes on (leading offset), groups of eight rows 1024 bytes apart (stride offset).
+__device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t saddr, uint32_t slab) {
+  return uint64_t((saddr >> 4) & 0x3FFFu) | (uint64_t(slab >> 4) << 16) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) | (uint64_t(2) << 61);
+}
+constexpr uint32_t kIdescBMajorN = 1u << 16;  // instruction descriptor: B is N-major
 // 32 rows x 16 bytes, unswizzled, rows contiguous (8-row groups 128 bytes apart): a scale-factor atom.
 __device__ __forceinline__ uint64_t smem_desc_sf(uint32_t saddr) {
   return uint64_t((saddr >> 4) & 0x3FFFu) | (uint64_t(128 >> 4) << 32) | (uint64_t(1) << 46);

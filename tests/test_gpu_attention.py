@@ -107,6 +107,30 @@ def test_one_key_that_outgrows_the_reference(spike):
     run_case(q, k, v, heads, heads)
 
 
+def test_values_that_do_not_start_on_sixteen_bytes():
+    """q, k and out need 16-byte rows, v never did: such a v is copied to the workspace first."""
+    seq, heads = 259, 2
+    q, k, v = data(seq, heads, 91, 0.3), data(seq, heads, 92, 0.3), data(seq, heads, 93, 1.0)
+    dq, dk, dv = (bf16_tensor(oracle.to_bf16(t)) for t in (q, k, v))
+    shifted = torch.empty(seq * heads * D + 8, dtype=torch.bfloat16, device="cuda")[3:3 + seq * heads * D].view(seq, heads * D)
+    shifted.copy_(dv)
+    assert torch.equal(attention(dq, dk, shifted, heads, heads), attention(dq, dk, dv, heads, heads))
+    assert sfq.device_status() == 0
+
+
+@pytest.mark.parametrize("seq,heads", [(130, 150), (256, 160), (385, 80), (513, 50)])
+def test_last_wave_as_single_query_tiles(seq, heads):
+    """Whole blocks of 256 queries and blocks run as two CTAs side by side in one launch (the last wave of 148 SMs): each head,
+    whichever form carried it, equals the same head computed alone."""
+    g = torch.Generator("cuda").manual_seed(seq)
+    q, k, v = (torch.randn((seq, heads * D), device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    out = attention(q, k, v, heads, heads)
+    for h in (0, heads // 2, heads - 1):
+        one = attention(*(t[:, h * D:(h + 1) * D].contiguous() for t in (q, k, v)), 1, 1)
+        assert torch.equal(out[:, h * D:(h + 1) * D], one)
+    assert sfq.device_status() == 0
+
+
 def test_against_torch_on_a_longer_sequence():
     torch.manual_seed(5)
     seq, heads = 4096 + 77, 4
