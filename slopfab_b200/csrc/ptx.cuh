@@ -45,6 +45,12 @@ template <class T> __device__ __forceinline__ const T* grid_dependency_wait(cons
   asm volatile("" : "+l"(p)::"memory");
   return p;
 }
+// ... or with an index, for a kernel that has no two registers to spare for a pointer it otherwise reads from the parameters.
+__device__ __forceinline__ int grid_dependency_wait(int i) {
+  grid_dependency_wait();
+  asm volatile("" : "+r"(i)::"memory");
+  return i;
+}
 
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {

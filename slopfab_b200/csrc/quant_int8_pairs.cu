@@ -102,8 +102,7 @@ quantize_int8_pairs_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restri
                            int rows, int dim) {
   extern __shared__ __align__(16) uint8_t smem[];
   ptx::grid_dependency_release();
-  x = ptx::grid_dependency_wait(x);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = ptx::grid_dependency_wait(int(threadIdx.x)), lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
   const int chunks = dim >> 4;
   const bool active = tid < chunks;
@@ -229,8 +228,7 @@ quantize_int8_pairs_wide_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __r
                                 int rows, int dim) {
   extern __shared__ __align__(16) uint8_t smem[];
   ptx::grid_dependency_release();
-  x = ptx::grid_dependency_wait(x);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = ptx::grid_dependency_wait(int(threadIdx.x)), lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
   f2* tile = reinterpret_cast<f2*>(smem) + (tid >> 4) * kGroupTile;
   uint8_t* bytes = smem + size_t(blockDim.x >> 4) * kGroupTile * 8 + (tid >> 4) * kGroupBytesOut;
