@@ -46,7 +46,7 @@ constexpr int kTileBytes = 2 * kSlab;  // [128 x 128] bf16
 constexpr int kAttnThreads = 384;  // warpgroup 0: producer, MMA issuer, two idle warps; warpgroups 1 and 2: the softmax of query tiles 0 and 1
 constexpr int kAttnRegsLean = 40, kAttnRegsSoftmax = 232;  // after setmaxnreg: 128 x 40 + 256 x 232 = 384 x 168, what the launch allocates (56 / 216: 1.3 % slower)
 constexpr int kTailWaves = 16;
-constexpr float kTileSumLimit = 32768.0f;  // a key tile's 128 probabilities may sum to this before the reference maximum moves
+constexpr float kTileSumLimit = 32768.0f;  // either part of a key tile's probabilities (96 and 32 keys) may sum to this before the reference maximum moves, so a tile to twice that
 
 struct AttnShared {
   uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_part[2], p_full[2], pv_part[2], pv_done[2];
@@ -391,13 +391,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         for (int c = 0; c < kFirstChunks; ++c) sum2 = emit_chunk(c, m_used, sum2);
         part_sum = total(sum2);
       }
-      l += part_sum;
       publish(&sh->p_part[t]);
-      sum2 = pack2(0.0f, 0.0f);
+      // The tile's probabilities are summed in one chain over all of its keys, as if they were handed over together.
 #pragma unroll
       for (int c = kFirstChunks; c < 4; ++c) sum2 = emit_chunk(c, m_used, sum2);
-      part_sum = total(sum2);
-      over = !(part_sum <= kTileSumLimit);
+      float tile_sum = total(sum2);
+      over = !(tile_sum - part_sum <= kTileSumLimit);
       if (__any_sync(0xffffffffu, over)) {
         // The last keys outgrew the reference after the first part's product was released: O_t is at rest again when that
         // product has completed (the issuer waits for the rest of P before it touches O_t).
@@ -406,13 +405,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         float mx = -INFINITY;
 #pragma unroll
         for (int c = kFirstChunks; c < 4; ++c) mx = fmaxf(mx, chunk_max(c));
+        if (over) l += part_sum;  // a row within its limit keeps its sum: it does not depend on its neighbours
         move_reference(over ? fmaxf(m_used, mx * g.scale_log2) : m_used, true);
         sum2 = pack2(0.0f, 0.0f);
 #pragma unroll
         for (int c = kFirstChunks; c < 4; ++c) sum2 = emit_chunk(c, m_used, sum2);
-        part_sum = total(sum2);
+        if (over) tile_sum = total(sum2);
       }
-      l += part_sum;
+      l += tile_sum;
       publish(&sh->p_full[t]);
     }
     if (ok && my_tiles > 0 && (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_done[t]), 0, sh, g.status, 20)))) {

@@ -1,6 +1,7 @@
 """Full self-attention (head_dim 128) against the dense fp64 softmax of the reference's test fixture, on the
 reference's own shapes, seeds and bound (tests/test_nn_kernels_attention_synthetic.cu:4-160)."""
 import ctypes as C
+import zlib
 
 import numpy as np
 import pytest
@@ -129,6 +130,15 @@ def test_last_wave_as_single_query_tiles(seq, heads):
         one = attention(*(t[:, h * D:(h + 1) * D].contiguous() for t in (q, k, v)), 1, 1)
         assert torch.equal(out[:, h * D:(h + 1) * D], one)
     assert sfq.device_status() == 0
+
+
+@pytest.mark.parametrize("seq,heads,scale,crc", [(1500, 2, 1.0, 0xBF518A00), (2051, 4, 0.3, 0x633D8771), (513, 40, 1.0, 0x323EB421)])
+def test_bits_of_seeded_calls(seq, heads, scale, crc):
+    """How a key tile's probabilities are handed to the second product is a matter of speed alone: their sum is one chain over the
+    tile's keys, and a call's bits are those of the kernel that handed them over in one part (its checksums). A sum per part
+    shows in a few of a million elements."""
+    q, k, v = (bf16_tensor(oracle.to_bf16(data(seq, heads, 300 + i + seq, scale))) for i in range(3))
+    assert zlib.crc32(bits(attention(q, k, v, heads, heads)).tobytes()) == crc
 
 
 def test_against_torch_on_a_longer_sequence():
