@@ -1,5 +1,5 @@
-// LoRA side branch of a Linear on B200: y += (x A^T) B^T with bf16 factors, both products on the tcgen05 bf16 GEMM,
-// the addition fused into the second product's epilogue.
+// LoRA side branch of a Linear on B200: y += (x A^T) B^T with bf16 factors, in one launch for ranks up to 128 and widths that
+// are multiples of 8, as two tcgen05 bf16 GEMMs otherwise and where input and output overlap (an update in place).
 //
 // Mirrors slopfab::cuda::LoraRunner (include/slopfab/cuda/lora.cuh:14-37, src/cuda/lora.cu:16-93): same names,
 // argument meaning and errors. Differences, all of them stated here:
@@ -9,8 +9,8 @@
 //     order of a scalar loop; a tensor-core product cannot reproduce that order, so `exact` is accepted and the
 //     result is within the tolerance the reference's own test allows its tensor arm (2^-8 absolute on O(1) data,
 //     tests/test_lora_backends.cu:120), not bit-identical to the scalar arm.
-//   * Scratch holds the hidden activations of 2048 rows (the reference: hidden + delta of 256 rows); longer inputs
-//     are processed in slices of that many rows. There is no delta buffer: the second GEMM adds into y.
+//   * Scratch holds the hidden activations of 2048 rows (the reference: hidden + delta of 256 rows); as two GEMMs longer
+//     inputs are processed in slices of that many rows. There is no delta buffer: the second GEMM adds into y.
 //   * Ranks that are not a multiple of 8 are zero-padded on upload (a 16-byte row pitch is what the TMA needs);
 //     `in` must be a multiple of 8.
 #pragma once

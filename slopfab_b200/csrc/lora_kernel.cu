@@ -200,6 +200,10 @@ bool lora_fused(const __nv_bfloat16* x, const __nv_bfloat16* a, const __nv_bfloa
                 cudaStream_t stream) {
   auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   if (rank <= 0 || rank > 128 || rank % 8 != 0 || in % 8 != 0 || out % 8 != 0 || !aligned(x) || !aligned(a) || !aligned(b) || !aligned(y)) return false;
+  // A CTA fetches y ahead of its stores, and the CTAs that share a row tile each read all of its x rows while the others store: x and
+  // y have to be apart. An update in place goes through the two GEMMs, where a slice's hidden rows are complete before its y is touched.
+  const __nv_bfloat16 *x_end = x + size_t(rows) * in, *y_end = y + size_t(rows) * out;
+  if (x < y_end && y < x_end) return false;
   if (rank <= 32)
     launch<4, 16>(x, a, b, y, rows, in, out, rank, stream);
   else if (rank <= 64)

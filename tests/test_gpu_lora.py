@@ -78,6 +78,35 @@ def test_lora_in_one_launch(rows, k, rank, out):
     assert sfq.device_status() == 0
 
 
+@pytest.mark.parametrize("rows,width,rank,lead", [(300, 512, 32, 0), (2368, 1024, 128, 0), (2500, 512, 16, 0), (700, 512, 8, 48)])
+def test_update_in_place(rows, width, rank, lead):
+    """y is x, or starts `lead` rows in front of it: every row of x counts as it was before the call (one slice of 2048 rows, or
+    slices that do not meet), on fewer row tiles than SMs, where the one-launch kernel would read x while it is being updated."""
+    g = torch.Generator("cuda").manual_seed(rows)
+    buf = torch.randn((rows + lead, width), device="cuda", generator=g).to(torch.bfloat16)
+    a = (torch.randn((rank, width), generator=torch.Generator().manual_seed(1)) / width ** 0.5).float().numpy()
+    b = (0.1 * torch.randn((width, rank), generator=torch.Generator().manual_seed(2))).float().numpy()
+    before = buf.double()
+    x0, y0 = before[lead:], before[:rows]
+    da, db = (torch.from_numpy(t).cuda().to(torch.bfloat16).double() for t in (a, b))
+    hidden = x0 @ da.T
+    want = y0 + hidden @ db.T
+    slack = 1.01 * 2.0 ** -8 * (2 * hidden.abs() @ db.abs().T + want.abs()) + 1e-5  # the three roundings, as above
+    runner = LoraRunner()
+    runner.attach(1, a, b)
+    start = buf.clone()
+    first = None
+    for _ in range(5):
+        buf.copy_(start)
+        runner.apply(1, buf[lead:], buf[:rows])
+        got = buf.clone()
+        assert bool(((got[:rows].double() - want).abs() <= slack).all())
+        assert torch.equal(got[rows:], start[rows:])
+        assert first is None or torch.equal(got, first)
+        first = got
+    assert sfq.device_status() == 0
+
+
 def test_two_factor_pairs_and_staged_upload():
     rows, k, out = 200, 256, 256
     x, a1, b1 = case(rows, k, 16, out, 1)
