@@ -98,3 +98,22 @@ def test_head_groups_and_table_alignment(rows, heads, aligned):
     sfq.check(sfq.lib.sfq_head_norm_rope(sfq.ptr(t), heads * 128, sfq.ptr(dw), dc.data_ptr() + 4 * off, ds.data_ptr() + 4 * off, rows, heads,
                                          128, 1e-6, sfq.stream_ptr()))
     assert np.array_equal(bits(t), want)
+
+
+def test_subnormal_table_entries_count_as_zero():
+    # products that are normal numbers although the table entry is not, in the low and in the high half, beside a partner's product
+    # that is small enough for the difference to show; eight channels apart, i.e. in lanes with nothing else to canonicalise
+    rows, heads = 3, 9
+    x = np.zeros((rows, heads * 128), np.float32)
+    x += oracle.make_data(rows * heads * 128, 77, 1.0).reshape(rows, heads * 128)
+    cos, sin = np.ones((rows, 96), np.float32), np.ones((rows, 96), np.float32)
+    for i, (a, b, c, s) in enumerate([(4.0, 1e-37, 1.0, 1e-38), (4.0, 1e-37, 1.0, -1e-38), (-1e3, 1e-37, 1e-38, 1.0),
+                                      (1e-37, 4.0, -1.1e-38, 1.0), (1e-37, -4.0, 1.0, 1.17e-38), (3e-38, 1e4, 1.0, 1e-40)]):
+        j = 8 * i
+        x[:, j::128], x[:, j + 48::128] = a, b
+        cos[:, j], sin[:, j] = c, s
+    bits_in = oracle.to_bf16(x).reshape(rows, heads * 128)
+    want = oracle.head_norm_rope(bits_in, heads, None, cos, sin, 1e-6)
+    flushed = [np.where(np.abs(t) < np.float32(1.17549435e-38), np.copysign(np.float32(0), t), t).astype(np.float32) for t in (cos, sin)]
+    assert np.array_equal(want, oracle.head_norm_rope(bits_in, heads, None, *flushed, 1e-6))
+    assert np.array_equal(run(bits_in, heads * 128, heads, None, cos, sin), want)
