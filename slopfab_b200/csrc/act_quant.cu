@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
         // per-16 fp4 (src/cuda/nvfp4_gemm.cu:107-158): this thread's eight elements and its neighbour's share a scale
         uint32_t m = hmax2(hmax2(habs2(n[0]), habs2(n[1])), hmax2(habs2(n[2]), habs2(n[3])));
         m = hmax2(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
-        m = hmax2(m, m >> 16);
+        m = hmax2(hmax2(m, m >> 16), 0u);  // the reference's maximum starts at 0, which a block of NaNs alone leaves: scale 0
         uint32_t s8 = row < a.rows ? uint32_t(__nv_cvt_float_to_fp8(__uint_as_float(m << 16) * (1.0f / 6.0f), __NV_SATFINITE, __NV_E4M3)) : 0u;
         const float rcp = __ldg(kE4m3Reciprocal.v + s8);
         const ptx::f32x2 rcp2 = ptx::pack2(rcp, rcp);

@@ -347,3 +347,43 @@ def test_norm_in_front_of_the_fp4_quantizer(rows, dim, modulate):
         got = _u8(fs)
         assert np.array_equal(got[shift_bytes:shift_bytes + nb], tiled)
         assert (got[:shift_bytes] == 0x55).all() and (got[shift_bytes + nb:] == 0x55).all()
+
+
+@pytest.mark.parametrize("dim", [256, 1024, 5120, 6144, 7168])
+@pytest.mark.parametrize("modulate", [False, True])
+def test_norm_and_fp4_of_rows_with_infinities_and_nans(dim, modulate):
+    """A NaN or an infinity makes the row's reciprocal NaN or zero: the normed row is NaN throughout, or zeros with NaNs. The block
+    maximum is the reference's, which starts at 0 and ignores NaN: scale bytes equal the CPU statement's, rows beside them are
+    untouched, in both layouts."""
+    rows = 9
+    x = gaussian_bf16((rows, dim), seed=dim)
+    x[1, 5] = 0x7FC0                       # a NaN
+    x[3, dim - 1] = 0x7F80                 # an infinity
+    x[4, 17], x[4, 18] = 0xFF80, 0x7F80    # infinities of both signs
+    x[6, :] = 0xFFC1                       # NaNs alone
+    x[7, :] = 0x7F7F                       # the largest values: the sum of squares overflows
+    rng = np.random.default_rng(dim)
+    w = oracle.to_bf16((1.0 + 0.1 * rng.standard_normal(dim)).astype(np.float32))
+    scale, shift = ((0.1 * rng.standard_normal((3, dim))).astype(np.float32) for _ in range(2))
+    idx = (np.arange(rows) % 3).astype(np.int32)
+    dx, dw, dsc, dsh, di = bf16_tensor(x), bf16_tensor(w), dev(scale), dev(shift), dev(idx)
+    norm = sfq.Norm(sfq.ptr(dw), sfq.ptr(dsc) if modulate else None, sfq.ptr(dsh) if modulate else None, sfq.ptr(di) if modulate else None, 1e-5)
+    normed = oracle.rmsnorm_bf16(x, w, 1e-5, *((scale, shift, idx) if modulate else ()))
+    packed, scales, _ = oracle.nvfp4_quantize_act(normed)
+    assert not scales[1].any() and not scales[6].any()
+    finite = ((normed & 0x7F80) != 0x7F80).reshape(rows, dim // 2, 2).all(axis=2)  # code bytes without a NaN, whose code is the hardware's
+    q = torch.full((rows, dim // 2), 0xA5, dtype=torch.uint8, device="cuda")
+    s = torch.full((128 * dim // 16,), 0xA5, dtype=torch.uint8, device="cuda")
+    out = torch.empty((rows, dim), dtype=torch.bfloat16, device="cuda")
+    for layout in (sfq.NVFP4_ACT_REFERENCE, sfq.NVFP4_ACT_GEMM_FEED):
+        sfq.check(sfq.lib.sfq_quantize_nvfp4_block(sfq.ptr(dx), C.byref(norm), sfq.ptr(q), sfq.ptr(s), sfq.ptr(out), rows, dim, layout, S))
+        got_s, got_q = _u8(s), _u8(q)
+        if layout == sfq.NVFP4_ACT_GEMM_FEED:
+            slots = np.array([[oracle.lib.orc_nvfp4_scale_slot(r, b, dim // 16) for b in range(dim // 16)] for r in range(rows)])
+            got_s, got_q = got_s[slots], ((got_q << 4) | (got_q >> 4)).astype(np.uint8)
+        else:
+            got_s = got_s[:rows * dim // 16].reshape(rows, dim // 16)
+        assert np.array_equal(got_s, scales), layout
+        assert np.array_equal(got_q[finite], packed[finite]), layout
+        nan = (normed & 0x7FFF) > 0x7F80
+        assert np.array_equal(bits(out)[~nan], normed[~nan]) and bool(((bits(out)[nan] & 0x7FFF) > 0x7F80).all())
