@@ -900,7 +900,7 @@ __global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __re
         }
         r[k] = bf16_pair(out[0], out[1]);
       }
-      if (rotates) {
+      if (rotates && head0 + 2 * i < heads) {  // a head that does not exist is zeros: not a reason for the step-by-step path
         if (least < kMinNormal) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
