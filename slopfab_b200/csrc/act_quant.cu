@@ -770,9 +770,8 @@ void quantize_nvfp4_block(const __nv_bfloat16* x, const NormArgs& norm, uint8_t*
 // What bounds it: HBM (read and write 256 bytes per head) once the instruction count is down, so a warp takes EIGHT heads of
 // one row, four per half warp: four 16-byte loads per lane in flight, the row's cos / sin read once for all of them, and the
 // serial part of the norm - the integer Newton reciprocal - run once for the eight heads side by side in different lanes.
-// The canonicalisation costs one running minimum beside the tables' own, done as they are loaded: a lane whose channels, products
-// and results are all normal numbers has nothing to canonicalise; one that saw a smaller magnitude (a zero counts) recomputes its
-// eight channels step by step.
+// The canonicalisation costs one running minimum: a lane whose channels, table entries, products and results are all normal numbers
+// has nothing to canonicalise; one that saw a smaller magnitude (a zero counts) recomputes its eight channels step by step.
 // Measured, q and k of 4747 rows x 40 heads: 61 us (3.2 TB/s); one warp per head with the reciprocal in one lane and the
 // canonicalisation in every channel: 436 us.
 namespace {
@@ -844,8 +843,6 @@ __global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __re
 #pragma unroll
       for (int i = 0; i < 8; ++i) c[i] = __ldg(cos_tab + at + i), s[i] = __ldg(sin_tab + at + i);
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) c[i] = rope_float_value(c[i]), s[i] = rope_float_value(s[i]);  // once for all of the row's heads
   }
   if constexpr (NORM) {
     float sum[kPer];
@@ -881,12 +878,15 @@ __global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __re
   if constexpr (ROPE) {
     const int partner = low ? lane + 6 : (rotates ? lane - 6 : lane);
     constexpr float kMinNormal = 1.17549435e-38f;
+    float least_entry = kMinNormal;  // a subnormal table entry can give normal products
+#pragma unroll
+    for (int i = 0; i < 8; ++i) least_entry = fminf(least_entry, fminf(fabsf(c[i]), fabsf(s[i])));
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
       uint32_t o[4], r[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) o[k] = __shfl_sync(0xFFFFFFFFu, h[i][k], partner);
-      float least = kMinNormal;  // of every magnitude that the reference would canonicalise
+      float least = least_entry;  // of every magnitude that the reference would canonicalise
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         float out[2];
