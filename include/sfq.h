@@ -458,9 +458,9 @@ SFQ_API int sfq_attention_forward(const void* d_q_bf16, int ld_q, const void* d_
  * adapter's scale already folded into b) and are rounded to bf16 on upload. `row_offset`/`out` select the rows
  * of b that belong to one view of a fused projection (q, k or v). Several attach calls under one key add
  * several factor pairs; apply runs all of them; an unknown key is a no-op. Both products accumulate
- * in fp32, hidden and product are rounded to bf16 like the reference's; one launch does all of it for ranks up to 128 and
- * widths that are multiples of 8, two tcgen05 bf16 GEMMs with the addition in the second one's epilogue otherwise and where x and
- * y overlap (y may be x itself; each factor pair then reads x as the one before left it). */
+ * in fp32, hidden and product are rounded to bf16 like the reference's. One launch does all of it for widths that are multiples
+ * of 8 and ranks up to 64 (up to 128 where that is faster); two tcgen05 bf16 GEMMs, with the addition in the second one's
+ * epilogue, otherwise and where x and y overlap (y may be x itself; each factor pair then reads x as the one before left it). */
 typedef struct sfq_lora sfq_lora;
 SFQ_API int sfq_lora_create(sfq_lora** out);
 SFQ_API void sfq_lora_destroy(sfq_lora* l);

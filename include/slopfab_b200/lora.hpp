@@ -1,5 +1,6 @@
-// LoRA side branch of a Linear on B200: y += (x A^T) B^T with bf16 factors, in one launch for ranks up to 128 and widths that
-// are multiples of 8, as two tcgen05 bf16 GEMMs otherwise and where input and output overlap (an update in place).
+// LoRA side branch of a Linear on B200: y += (x A^T) B^T with bf16 factors, in one launch for ranks up to 64 (up to 128 where
+// that is faster) and widths that are multiples of 8, as two tcgen05 bf16 GEMMs otherwise and where input and output overlap (an update
+// in place).
 //
 // Mirrors slopfab::cuda::LoraRunner (include/slopfab/cuda/lora.cuh:14-37, src/cuda/lora.cu:16-93): same names,
 // argument meaning and errors. Differences, all of them stated here:

@@ -93,7 +93,8 @@ void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k,
                        cudaStream_t stream);
 
 // LoRA side branch in one launch (lora_kernel.cu): y[rows,out] += bf16(bf16(x a^T) b^T), a [rank,in], b [out,rank]; false,
-// with nothing launched, when rank > 128, a width is no multiple of 8, an operand is not 16-byte aligned or x and y overlap.
+// with nothing launched, when rank > 128, a width is no multiple of 8, an operand is not 16-byte aligned, x and y overlap, or two
+// GEMMs are the faster way.
 bool lora_fused(const __nv_bfloat16* x, const __nv_bfloat16* a, const __nv_bfloat16* b, __nv_bfloat16* y, int rows, int in, int out, int rank,
                 cudaStream_t stream);
 

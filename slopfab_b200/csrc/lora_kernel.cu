@@ -204,6 +204,15 @@ bool lora_fused(const __nv_bfloat16* x, const __nv_bfloat16* a, const __nv_bfloa
   // y have to be apart. An update in place goes through the two GEMMs, where a slice's hidden rows are complete before its y is touched.
   const __nv_bfloat16 *x_end = x + size_t(rows) * in, *y_end = y + size_t(rows) * out;
   if (x < y_end && y < x_end) return false;
+  // Above rank 64 every CTA reads all of A (in x rank) from L2 for its 32 rows, with registers for no more than two slices in flight,
+  // so what decides is in x rank, and whether the two GEMMs need more than one slice. This kernel against two GEMMs, inputs from HBM:
+  // one slice (2048 rows) 2560 -> 5120 rank 72 48.1 / 58.2 us, rank 128 60.4 / 56.3; 5120 -> 5120 rank 72 70.7 / 66.6; 512 rows 13824 -> 5120
+  // rank 128 199 / 79. More (4096 rows) 13824 -> 5120 rank 72 169 / 190; rank 128 5120 -> 5120 113 / 126, 7680 -> 5120 146 / 139, and with few
+  // outputs 5120 -> 1024 85 / 75 (20000 rows 286 / 337). Ranks up to 64: never slower (closest: rank 64, 2048 rows 13824 -> 512, 75.8 / 74.8).
+  const size_t factor = size_t(in) * rank;
+  const bool one_launch = rank <= 64 || (rows <= 2048 ? factor <= 200000
+                                                      : rank <= 80 || (factor <= 660000 && (in <= out || in <= 2560 || rows > 8192)));
+  if (!one_launch) return false;
   if (rank <= 32)
     launch<4, 16>(x, a, b, y, rows, in, out, rank, stream);
   else if (rank <= 64)

@@ -1,8 +1,8 @@
 // LoraRunner: the low-rank side branch of a Linear (src/cuda/lora.cu:16-93).
 //   hidden = bf16(x A^T)
 //   y      = bf16(y + bf16(hidden B^T))
-// One launch (lora_kernel.cu) wherever that kernel takes the operands; otherwise -- ranks above 128, an output width that is no
-// multiple of 8, x and y that overlap -- two tcgen05 bf16 GEMMs per slice of kRows rows, N = rank and K = rank, the addition in
+// One launch (lora_kernel.cu) wherever that kernel takes the call; otherwise -- ranks above 64 of wide inputs, an output width that is
+// no multiple of 8, x and y that overlap -- two tcgen05 bf16 GEMMs per slice of kRows rows, N = rank and K = rank, the addition in
 // the second one's epilogue. Which calls overlap is known only at apply(), which must not allocate, so attach() reserves the two
 // GEMMs' scratch for every factor pair. The epilogue used is the gated residual y = bf16(fma(gate, branch, y)) with a gate of ones: fma(1, b, y) is y + b
 // rounded once, i.e. launch_add_bf16 (src/cuda/nn_pointwise.cu:241) applied to the rounded product.

@@ -55,6 +55,9 @@ def test_lora_apply_matches_the_reference_statement(rows, k, rank, out_total, of
 @pytest.mark.parametrize("rows,k,rank,out", [
     (1, 512, 4, 512), (31, 520, 32, 40), (33, 1032, 33, 1000), (64, 4104, 64, 520), (95, 2048, 65, 2056), (300, 512, 128, 13824),
     (4737, 520, 16, 264),   # more row tiles than SMs: no split of the features
+    (64, 1560, 128, 520), (64, 1568, 128, 520),       # ranks above 64, one slice of rows: the widest input of the one launch, two GEMMs beyond
+    (2048, 2776, 72, 264), (2049, 2784, 72, 264),     # ... more than one slice
+    (2049, 5152, 128, 5152), (2049, 5160, 128, 5160), (2049, 2568, 128, 264), (8200, 2568, 128, 264),
     (200, 512, 136, 512),   # past the one-launch kernel: two GEMMs
     (200, 512, 8, 500),     # an output width that is no multiple of 8: two GEMMs
 ])
