@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(256) linear_f32_kernel(const float* __restrict
     }
 }
 
-// The same product with the rows in tiles of at most 16, for the few rows the DiT calls it with: bound by reading the weight once. A CTA of four warps
+// The same product with the rows in tiles of at most 16, for few rows (the DiT's timesteps) and long sums: bound by reading the weight once. A CTA of four warps
 // takes F output features and R rows and splits K between its 128 threads, 16 bytes of fp32 weight (8 of bf16) per thread,
 // feature and step, so a warp reads 512 contiguous bytes of each weight row and 2 F such loads are in flight per thread;
 // the products run as packed pairs (even and odd k in the two halves of an f32x2 accumulator). x is small and shared by
@@ -499,12 +499,20 @@ void launch_linear_f32(const float* x, const WT* w, const void* bias, bool bias_
                        cudaStream_t stream) {
   const dim3 grid((out_features + 63) / 64, (rows + 63) / 64);
   if (grid.y > 65535) throw std::invalid_argument("linear_f32: too many rows for one launch");
-  // The row kernel wherever its loads are aligned and its flat grid fits: 5120 -> 15360 in fp32, it against the tiled kernel, 1 row
-  // 48 / 1052 us, 64 rows 580 / 1323, 512 rows 4243 / 4383; 200 rows of 1024 -> 512 29 / 147.
+  // The row kernel where its loads are aligned, its flat grid fits and it is the faster one. Its time is its CTAs' (row tiles of up to
+  // 16 x features / F, each a fixed part worth 800 steps of K -- set-up, the butterfly -- and K); the tiled kernel's is one tile's
+  // chain over K plus its tiles'. The constants, in the row kernel's steps of 6 ps, are fitted to 900 shapes of 64 <= K <= 5120, 128 to
+  // 30720 features and 1 to 4096 rows (F = 4 and 16 rows; one feature per CTA costs 0.55 of that, one row 0.3, four 0.6). Row kernel against tiled in fp32: 5120 -> 15360,
+  // 1 row 48 / 1052 us, 64 rows 580 / 1323; 5120 -> 5120, 512 rows 1460 / 1566, 4096 rows 12489 / 9958; 256 -> 30720, 16 rows 59 / 74, 17
+  // rows 107 / 74, 64 rows 204 / 82; 64 -> 5120, 16 rows 16 / 16, 64 rows 39 / 21; 1024 -> 512, 1024 rows 145 / 223, 4096 rows 522 / 307.
   const bool wide = in_features % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(w) % (4 * sizeof(WT)) == 0;
-  if (wide && size_t(out_features) * ((rows + 15) / 16) <= size_t(0x7FFFFFFF)) {
-    // four features per CTA while that leaves every SM its four CTAs, one otherwise
-    if (out_features >= 4 * 4 * device_sm_count())
+  // four features per CTA while that leaves every SM its four CTAs, one otherwise
+  const int features = out_features >= 4 * 4 * device_sm_count() ? 4 : 1;
+  const double k = in_features, row_ctas = double((rows + 15) / 16) * ((out_features + features - 1) / features);
+  const double row_cost = row_ctas * (800 + k) * (features == 4 ? 1.0 : 0.55) * (rows <= 1 ? 0.3 : rows <= 4 ? 0.6 : 1.0);
+  const double tiled_cost = k * ((sizeof(WT) == 4 ? 26700 : 21000) + 60.0 * grid.x * grid.y);
+  if (wide && row_cost <= tiled_cost && size_t(out_features) * ((rows + 15) / 16) <= size_t(0x7FFFFFFF)) {
+    if (features == 4)
       launch_rows_for<WT, 4>(x, w, bias, bias_is_bf16, y, rows, out_features, in_features, stream);
     else
       launch_rows_for<WT, 1>(x, w, bias, bias_is_bf16, y, rows, out_features, in_features, stream);

@@ -109,6 +109,25 @@ def test_forward_f32_row_tiles(fmt, rows, n, k):
     assert bool(((got.double() - want).abs() <= steps * 2.0 ** -24 * terms).all())
 
 
+@pytest.mark.parametrize("fmt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,n,k", [(64, 30720, 256), (33, 5120, 64), (513, 2560, 512), (3000, 512, 512), (600, 9000, 1024)])
+def test_forward_f32_of_many_rows_or_short_sums(fmt, rows, n, k):
+    """Where the tiled kernel is the faster one it runs whatever the alignment allows: the bits of a call are those of the same call
+    with an x that only the tiled kernel can read. Bound: one fp32 rounding per term, by 2^-24 of the terms' magnitudes at most."""
+    g = torch.Generator("cuda").manual_seed(rows + n)
+    x = torch.randn((rows, k), device="cuda", generator=g)
+    w = torch.randn((n, k), device="cuda", generator=g).mul_(0.05).to(fmt)
+    weight = sfq.new_weight(format=sfq.F32 if fmt == torch.float32 else sfq.BF16, data=sfq.ptr(w), out_features=n, in_features=k)
+    runner = sfq.LinearRunner()
+    got = runner.forward_f32(weight, x)
+    shifted = torch.empty(rows * k + 1, device="cuda")[1:].view(rows, k)
+    shifted.copy_(x)
+    assert torch.equal(got, runner.forward_f32(weight, shifted))
+    want = x.double() @ w.double().T
+    terms = x.double().abs() @ w.double().abs().T
+    assert bool(((got.double() - want).abs() <= (k + 1) * 2.0 ** -24 * terms).all())
+
+
 def test_forward_f32_refuses_what_it_does_not_build():
     t = torch.zeros(256 * 256, dtype=torch.float32, device="cuda")
     runner = sfq.LinearRunner()
