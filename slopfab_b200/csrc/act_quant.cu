@@ -360,9 +360,14 @@ __global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
 // (2.64 TB/s), 4747 rows 30 us; the one-row kernel with the row in shared memory took 1018 and 58 us. Not faster: 256 threads
 // (555 us), CTAs that stay with the next rows prefetched and the tables in shared memory (469 us, fewer warps per SM), the
 // reciprocal in warp 0 alone behind a second barrier (407 us).
-constexpr int kNormThreads = 128;
+// FEW rows leave nothing else on the SM to hide a CTA's latencies, and 128 threads meet the weight and the tables of a wide row in up
+// to 16 dependent steps. There a CTA has 256 threads and one row, and everything the row needs is on its way before the tree. As
+// long as all CTAs are resident at once: two per SM up to 8192 wide (four packs per thread), one beyond. Modulated, fp4 out, inputs
+// from HBM, FEW against 128 threads: 64 rows of 3072 8.2 / 12.3 us, 5120 10.2 / 14.3, 16384 14.3 / 22.5; 296 rows of 5120 10.2 / 14.3, of
+// 13824 22.5 / 20.5; 444 of 5120 14.3 / 14.3; 888 of 5120 18.4 / 14.3.
+template <bool FEW> constexpr int kNormThreads = FEW ? 256 : 128;
 // Rows a CTA takes at a time: two while a thread's share of a row is at most six packs (dim <= 6144), one beyond that.
-template <int MAXP> constexpr int kNormRows = MAXP <= 6 ? 2 : 1;
+template <int MAXP, bool FEW> constexpr int kNormRows = MAXP <= 6 && !FEW ? 2 : 1;
 
 // 1 / decode(s8) correctly rounded for the positive e4m3 scales, 0 for scale 0 (and for the NaN code, which is never produced).
 struct E4m3Reciprocals {
@@ -392,9 +397,10 @@ template <bool HIGH_EVEN> __device__ __forceinline__ uint32_t e2m1_word(const fl
   return w;
 }
 
-template <int MODE, int MAXP>
-__global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_kernel(const FusedArgs args, int total_rows) {
-  constexpr int R = kNormRows<MAXP>;
+template <int MODE, int MAXP, bool FEW>
+__global__ void __launch_bounds__(kNormThreads<FEW>, FEW ? (MAXP <= 4 ? 2 : 1) : (MAXP <= 2 ? 8 : 4)) norm_rows_kernel(const FusedArgs args, int total_rows) {
+  constexpr int T = kNormThreads<FEW>, R = kNormRows<MAXP, FEW>;
+  constexpr int V = 256 / T;  // virtual threads per thread
   FusedArgs a = args;
   ptx::grid_dependency_release();
   a.x = ptx::grid_dependency_wait(a.x);
@@ -404,7 +410,7 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
   const int row0 = blockIdx.x * R;
   if (MODE == kNormFp4Feed && row0 >= a.rows) {  // padding rows of the last 128-row scale tile: zero scales
     for (int r = 0; r < R && row0 + r < total_rows; ++r)
-      for (int c = tid; c < chunks; c += kNormThreads) a.scales[nvfp4_scale_offset(row0 + r, c, chunks)] = 0;
+      for (int c = tid; c < chunks; c += T) a.scales[nvfp4_scale_offset(row0 + r, c, chunks)] = 0;
     return;
   }
   uint4 raw[R][MAXP];
@@ -412,7 +418,7 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
   for (int j = 0; j < MAXP; ++j)
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int p = tid + j * kNormThreads;
+      const int p = tid + j * T;
       raw[r][j] = make_uint4(0, 0, 0, 0);
       if (p < packs && row0 + r < a.rows) raw[r][j] = reinterpret_cast<const uint4*>(a.x + size_t(row0 + r) * a.dim)[p];
     }
@@ -421,20 +427,44 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
 #pragma unroll
     for (int r = 0; r < R; ++r) index[r] = __ldg(a.mod_index + min(row0 + r, a.rows - 1));
   }
-  // sum of squares: the chains of virtual threads t (even packs) and t + 128 (odd ones), the shfl_down tree of their virtual
+  // the weight and the tables of pack j; FEW fetches all of them here, ahead of the row's tree
+  constexpr int A = FEW ? MAXP : 1;
+  uint4 wr[A];
+  ptx::f32x2 sc[A][4], sh[A][4];
+  auto load_weight = [&](int j) { return tid + j * T < packs ? __ldg(reinterpret_cast<const uint4*>(a.norm_w) + tid + j * T) : make_uint4(0, 0, 0, 0); };
+  auto load_tables = [&](int j, int row_index, ptx::f32x2 (&s)[4], ptx::f32x2 (&h)[4]) {
+    const size_t at = size_t(row_index) * a.dim + size_t(tid + j * T < packs ? tid + j * T : 0) * 8;
+    const float4* sp = reinterpret_cast<const float4*>(a.mod_scale + at);
+    const float4* hp = reinterpret_cast<const float4*>(a.mod_shift + at);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float4 s4 = __ldg(sp + i), h4v = __ldg(hp + i);
+      s[2 * i] = ptx::pack2(s4.x, s4.y), s[2 * i + 1] = ptx::pack2(s4.z, s4.w);
+      h[2 * i] = ptx::pack2(h4v.x, h4v.y), h[2 * i + 1] = ptx::pack2(h4v.z, h4v.w);
+    }
+  };
+  if constexpr (FEW) {
+#pragma unroll
+    for (int j = 0; j < MAXP; ++j) {
+      wr[j] = load_weight(j);
+      if (a.mod_scale != nullptr) load_tables(j, index[0], sc[j], sh[j]);
+    }
+  }
+  // sum of squares: the chains of virtual threads t and, of 128, t + 128 (odd packs), the shfl_down tree of their virtual
   // warps, then the tree over the eight warps' totals
-  float sum[R][2];
+  float sum[R][V];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    sum[r][0] = sum[r][1] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < V; ++k) sum[r][k] = 0.0f;
 #pragma unroll
     for (int j = 0; j < MAXP; ++j) {  // absent packs are zeros: fma(0, 0, s) = s
       const uint32_t u[4] = {raw[r][j].x, raw[r][j].y, raw[r][j].z, raw[r][j].w};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float lo = __uint_as_float(u[i] << 16), hi = __uint_as_float(u[i] & 0xFFFF0000u);
-        sum[r][j & 1] = __fmaf_rn(lo, lo, sum[r][j & 1]);
-        sum[r][j & 1] = __fmaf_rn(hi, hi, sum[r][j & 1]);
+        sum[r][j % V] = __fmaf_rn(lo, lo, sum[r][j % V]);
+        sum[r][j % V] = __fmaf_rn(hi, hi, sum[r][j % V]);
       }
     }
   }
@@ -443,10 +473,12 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int k = 0; k < 2; ++k) sum[r][k] = __fadd_rn(sum[r][k], __shfl_down_sync(0xFFFFFFFFu, sum[r][k], off));
+      for (int k = 0; k < V; ++k) sum[r][k] = __fadd_rn(sum[r][k], __shfl_down_sync(0xFFFFFFFFu, sum[r][k], off));
   if (lane == 0) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) warp_tot[r][warp] = sum[r][0], warp_tot[r][warp + 4] = sum[r][1];
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int k = 0; k < V; ++k) warp_tot[r][warp + k * (T / 32)] = sum[r][k];
   }
   __syncthreads();
   // Every warp folds the totals itself: lanes 8 r .. 8 r + 7 hold row r (the reference's steps 16 and 8 add zeros).
@@ -460,27 +492,21 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
 
 #pragma unroll
   for (int j = 0; j < MAXP; ++j) {
-    const int p = tid + j * kNormThreads;
+    const int p = tid + j * T;
     const bool active = p < packs;
     if (!__any_sync(0xFFFFFFFFu, active)) break;
-    uint4 wr = make_uint4(0, 0, 0, 0);
-    if (active) wr = __ldg(reinterpret_cast<const uint4*>(a.norm_w) + p);
-    const uint32_t wu[4] = {wr.x, wr.y, wr.z, wr.w};
-    ptx::f32x2 sc[4], sh[4];
+    constexpr bool kFetched = FEW;
+    const int at = kFetched ? j : 0;
+    if constexpr (!kFetched) wr[0] = load_weight(j);
+    const uint32_t wu[4] = {wr[at].x, wr[at].y, wr[at].z, wr[at].w};
+    const ptx::f32x2 one = ptx::pack2(1.0f, 1.0f);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int row = row0 + r;
       if (a.mod_scale != nullptr && (r == 0 || index[r] != index[r - 1])) {
-        const size_t at = size_t(index[r]) * a.dim + size_t(active ? p : 0) * 8;
-        const float4* sp = reinterpret_cast<const float4*>(a.mod_scale + at);
-        const float4* hp = reinterpret_cast<const float4*>(a.mod_shift + at);
-        const ptx::f32x2 one = ptx::pack2(1.0f, 1.0f);
+        if constexpr (!kFetched) load_tables(j, index[r], sc[0], sh[0]);
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const float4 s4 = __ldg(sp + i), h4v = __ldg(hp + i);
-          sc[2 * i] = ptx::add2(one, ptx::pack2(s4.x, s4.y)), sc[2 * i + 1] = ptx::add2(one, ptx::pack2(s4.z, s4.w));
-          sh[2 * i] = ptx::pack2(h4v.x, h4v.y), sh[2 * i + 1] = ptx::pack2(h4v.z, h4v.w);
-        }
+        for (int i = 0; i < 4; ++i) sc[at][i] = ptx::add2(one, sc[at][i]);
       }
       const uint32_t u[4] = {raw[r][j].x, raw[r][j].y, raw[r][j].z, raw[r][j].w};
       const ptx::f32x2 inv2 = ptx::pack2(inv[r], inv[r]);
@@ -489,7 +515,7 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
       for (int i = 0; i < 4; ++i) {
         const ptx::f32x2 x2 = ptx::pack2(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xFFFF0000u));
         ptx::f32x2 v = ptx::mul2(ptx::mul2(x2, inv2), ptx::pack2(__uint_as_float(wu[i] << 16), __uint_as_float(wu[i] & 0xFFFF0000u)));
-        if (a.mod_scale != nullptr) v = ptx::fma2(v, sc[i], sh[i]);
+        if (a.mod_scale != nullptr) v = ptx::fma2(v, sc[at][i], sh[at][i]);
         float lo, hi;
         ptx::unpack2(v, lo, hi);
         const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
@@ -519,8 +545,8 @@ __global__ void __launch_bounds__(kNormThreads, MAXP <= 2 ? 8 : 4) norm_rows_ker
           s8 |= __shfl_xor_sync(0xFFFFFFFFu, s8, 2);
           s8 |= __shfl_xor_sync(0xFFFFFFFFu, s8, 4);
           if (active && (lane & 7) == 0 && row < total_rows) {
-            // 64 blocks further on are 16 tiles of 512 bytes
-            uint8_t* dst = a.scales + nvfp4_scale_offset(row, tid >> 1, chunks) + size_t(j) * (16 * 512);
+            // T / 2 blocks further on are T / 8 tiles of 512 bytes
+            uint8_t* dst = a.scales + nvfp4_scale_offset(row, tid >> 1, chunks) + size_t(j) * (T / 8 * 512);
             if ((reinterpret_cast<uintptr_t>(dst) & 3) == 0)
               *reinterpret_cast<uint32_t*>(dst) = s8;
             else  // an array that starts off a word boundary
@@ -587,21 +613,29 @@ template <int MODE> void launch_fused(const FusedArgs& a, cudaStream_t stream, c
   check_launch(launch_overlapped(size_t(a.rows) * a.dim * 4, fused_act_kernel<MODE>, dim3(grid), dim3(threads), smem, stream, a), what);
 }
 
+template <int MODE, int MAXP, bool FEW> cudaError_t launch_norm_as(const FusedArgs& a, int total_rows, cudaStream_t stream) {
+  constexpr int R = kNormRows<MAXP, FEW>;
+  return launch_overlapped(size_t(a.rows) * a.dim * 3, norm_rows_kernel<MODE, MAXP, FEW>, dim3((total_rows + R - 1) / R), dim3(kNormThreads<FEW>), 0,
+                           stream, a, total_rows);
+}
+
 // A thread's packs per row decide the registers of the kernel.
 template <int MODE> void launch_norm(const FusedArgs& a, int total_rows, cudaStream_t stream, const char* what) {
   check_row_args(a, what);
-  const int per_thread = (a.dim / 8 + kNormThreads - 1) / kNormThreads;
-  const auto grid = [&](int r) { return (total_rows + r - 1) / r; };
-  const size_t bytes = size_t(a.rows) * a.dim * 3;
+  const auto packs = [&](int threads) { return (a.dim / 8 + threads - 1) / threads; };
+  const bool few = a.rows <= device_sm_count() * (packs(kNormThreads<true>) <= 4 ? 2 : 1);
+  const int per_thread = packs(few ? kNormThreads<true> : kNormThreads<false>);
   cudaError_t e = cudaSuccess;
-  if (per_thread <= 2)
-    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 2>, dim3(grid(kNormRows<2>)), dim3(kNormThreads), 0, stream, a, total_rows);
-  else if (per_thread <= 5)
-    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 5>, dim3(grid(kNormRows<5>)), dim3(kNormThreads), 0, stream, a, total_rows);
-  else if (per_thread <= 6)
-    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 6>, dim3(grid(kNormRows<6>)), dim3(kNormThreads), 0, stream, a, total_rows);
+  if (few)
+    e = per_thread <= 1   ? launch_norm_as<MODE, 1, true>(a, total_rows, stream)
+        : per_thread <= 3 ? launch_norm_as<MODE, 3, true>(a, total_rows, stream)
+        : per_thread <= 4 ? launch_norm_as<MODE, 4, true>(a, total_rows, stream)
+                          : launch_norm_as<MODE, 8, true>(a, total_rows, stream);
   else
-    e = launch_overlapped(bytes, norm_rows_kernel<MODE, 16>, dim3(grid(kNormRows<16>)), dim3(kNormThreads), 0, stream, a, total_rows);
+    e = per_thread <= 2   ? launch_norm_as<MODE, 2, false>(a, total_rows, stream)
+        : per_thread <= 5 ? launch_norm_as<MODE, 5, false>(a, total_rows, stream)
+        : per_thread <= 6 ? launch_norm_as<MODE, 6, false>(a, total_rows, stream)
+                          : launch_norm_as<MODE, 16, false>(a, total_rows, stream);
   check_launch(e, what);
 }
 

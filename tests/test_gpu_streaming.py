@@ -314,7 +314,9 @@ def test_pointwise_kernels_match_reference():
     assert np.array_equal(bits(dx), want)
 
 
-@pytest.mark.parametrize("rows,dim", [(1, 64), (3, 192), (2, 2048), (131, 2112), (5, 5120), (4, 6144), (3, 6208), (1, 16384)])
+@pytest.mark.parametrize("rows,dim", [(1, 64), (3, 192), (2, 2048), (131, 2112), (5, 5120), (4, 6144), (3, 6208), (1, 16384),
+                                      (7, 8192), (9, 8256), (296, 5120), (148, 8256),  # a CTA of 256 threads per row, on 148 SMs
+                                      (297, 64), (301, 2048), (299, 2112), (297, 5120), (384, 6144), (298, 6208), (149, 8256), (151, 16384)])
 @pytest.mark.parametrize("modulate", [False, True])
 def test_norm_in_front_of_the_fp4_quantizer(rows, dim, modulate):
     # rows per CTA and packs per thread of the norm kernel at their edges: one, three and more packs, odd row counts, padding rows
@@ -349,13 +351,12 @@ def test_norm_in_front_of_the_fp4_quantizer(rows, dim, modulate):
         assert (got[:shift_bytes] == 0x55).all() and (got[shift_bytes + nb:] == 0x55).all()
 
 
-@pytest.mark.parametrize("dim", [256, 1024, 5120, 6144, 7168])
+@pytest.mark.parametrize("rows,dim", [(9, 256), (9, 1024), (9, 5120), (9, 6144), (9, 7168), (300, 256), (301, 5120), (303, 6144), (160, 8256)])
 @pytest.mark.parametrize("modulate", [False, True])
-def test_norm_and_fp4_of_rows_with_infinities_and_nans(dim, modulate):
+def test_norm_and_fp4_of_rows_with_infinities_and_nans(rows, dim, modulate):
     """A NaN or an infinity makes the row's reciprocal NaN or zero: the normed row is NaN throughout, or zeros with NaNs. The block
     maximum is the reference's, which starts at 0 and ignores NaN: scale bytes equal the CPU statement's, rows beside them are
     untouched, in both layouts."""
-    rows = 9
     x = gaussian_bf16((rows, dim), seed=dim)
     x[1, 5] = 0x7FC0                       # a NaN
     x[3, dim - 1] = 0x7F80                 # an infinity
@@ -373,7 +374,7 @@ def test_norm_and_fp4_of_rows_with_infinities_and_nans(dim, modulate):
     assert not scales[1].any() and not scales[6].any()
     finite = ((normed & 0x7F80) != 0x7F80).reshape(rows, dim // 2, 2).all(axis=2)  # code bytes without a NaN, whose code is the hardware's
     q = torch.full((rows, dim // 2), 0xA5, dtype=torch.uint8, device="cuda")
-    s = torch.full((128 * dim // 16,), 0xA5, dtype=torch.uint8, device="cuda")
+    s = torch.full((sfq.lib.sfq_nvfp4_act_scale_bytes(rows, dim),), 0xA5, dtype=torch.uint8, device="cuda")
     out = torch.empty((rows, dim), dtype=torch.bfloat16, device="cuda")
     for layout in (sfq.NVFP4_ACT_REFERENCE, sfq.NVFP4_ACT_GEMM_FEED):
         sfq.check(sfq.lib.sfq_quantize_nvfp4_block(sfq.ptr(dx), C.byref(norm), sfq.ptr(q), sfq.ptr(s), sfq.ptr(out), rows, dim, layout, S))
