@@ -52,7 +52,6 @@ struct FusedArgs {
   uint8_t* packed;
   uint8_t* scales;
   __nv_bfloat16* bf16_out;  // normed activation (optional) or the rotated one (rot-only mode)
-  int beside;  // rotation only: wait for the kernel in front at the end instead of at the start (see kernels.cuh)
 };
 
 // ---- integer-exact norm reciprocal (include/slopfab/cuda/deterministic_math.cuh:26-197) ----
@@ -194,7 +193,7 @@ __device__ __forceinline__ void process_row(const FusedArgs& a, const int row, u
     const float inv = bcast[0];
     if (active) {
       const uint4* wp = reinterpret_cast<const uint4*>(a.norm_w) + tid * 2;
-      const uint4 w0 = __ldg(wp), w1 = __ldg(wp + 1);
+      const uint4 w0 = wp[0], w1 = wp[1];
       const __nv_bfloat162* wh0 = reinterpret_cast<const __nv_bfloat162*>(&w0);
       const __nv_bfloat162* wh1 = reinterpret_cast<const __nv_bfloat162*>(&w1);
       float w[16];
@@ -209,7 +208,7 @@ __device__ __forceinline__ void process_row(const FusedArgs& a, const int row, u
         const float4* sh = reinterpret_cast<const float4*>(a.mod_shift + mod);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float4 s4 = __ldg(sc + j), h4v = __ldg(sh + j);
+          const float4 s4 = sc[j], h4v = sh[j];
           const float ss[4] = {s4.x, s4.y, s4.z, s4.w}, hh[4] = {h4v.x, h4v.y, h4v.z, h4v.w};
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -318,11 +317,12 @@ __device__ __forceinline__ void process_row(const FusedArgs& a, const int row, u
 // The kernel: a CTA walks rows blockIdx.x, blockIdx.x + gridDim.x, ... and loads the NEXT row's 32 bytes per
 // thread before working on the current one, so every resident warp always has a load in flight (one row per
 // CTA without prefetch keeps too few bytes in flight to cover HBM latency).
-template <int MODE>
-__global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
+// BESIDE: the kernel in front neither writes x nor reads the output: wait for it at the end instead of at the start (see kernels.cuh).
+template <int MODE, bool BESIDE>
+__global__ void __launch_bounds__(1024, 1) fused_act_kernel(const FusedArgs a) {
   extern __shared__ __align__(16) uint8_t smem[];
   ptx::grid_dependency_release();
-  if (MODE != kModeRotOnly || !a.beside) a.x = ptx::grid_dependency_wait(a.x);
+  if constexpr (!BESIDE) ptx::grid_dependency_wait();
   const int chunks = a.dim >> 4;
   const bool active = int(threadIdx.x) < chunks;
   auto load = [&](int row, uint4& r0, uint4& r1) {
@@ -330,8 +330,8 @@ __global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
     r1 = r0;
     if (active && row < a.rows) {
       const uint4* src = reinterpret_cast<const uint4*>(a.x + size_t(row) * a.dim) + threadIdx.x * 2;
-      r0 = __ldg(src);
-      r1 = __ldg(src + 1);
+      r0 = src[0];
+      r1 = src[1];
     }
   };
   uint4 r0, r1, n0, n1;
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(1024, 1) fused_act_kernel(FusedArgs a) {
     r0 = n0;
     r1 = n1;
   }
-  if (MODE == kModeRotOnly && a.beside) ptx::grid_dependency_wait();
+  if constexpr (BESIDE) ptx::grid_dependency_wait();
 }
 
 // ---- RMSNorm [+ modulate], alone or in front of the per-16-block fp4 quantizer ---------------------------------------
@@ -398,12 +398,11 @@ template <bool HIGH_EVEN> __device__ __forceinline__ uint32_t e2m1_word(const fl
 }
 
 template <int MODE, int MAXP, bool FEW>
-__global__ void __launch_bounds__(kNormThreads<FEW>, FEW ? (MAXP <= 4 ? 2 : 1) : (MAXP <= 2 ? 8 : 4)) norm_rows_kernel(const FusedArgs args, int total_rows) {
+__global__ void __launch_bounds__(kNormThreads<FEW>, FEW ? (MAXP <= 4 ? 2 : 1) : (MAXP <= 2 ? 8 : 4)) norm_rows_kernel(const FusedArgs a, int total_rows) {
   constexpr int T = kNormThreads<FEW>, R = kNormRows<MAXP, FEW>;
   constexpr int V = 256 / T;  // virtual threads per thread
-  FusedArgs a = args;
   ptx::grid_dependency_release();
-  a.x = ptx::grid_dependency_wait(a.x);
+  ptx::grid_dependency_wait();
   __shared__ float warp_tot[R][8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int packs = a.dim >> 3, chunks = a.dim >> 4;
@@ -425,20 +424,20 @@ __global__ void __launch_bounds__(kNormThreads<FEW>, FEW ? (MAXP <= 4 ? 2 : 1) :
   int index[R] = {};
   if (a.mod_scale != nullptr) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) index[r] = __ldg(a.mod_index + min(row0 + r, a.rows - 1));
+    for (int r = 0; r < R; ++r) index[r] = a.mod_index[min(row0 + r, a.rows - 1)];
   }
   // the weight and the tables of pack j; FEW fetches all of them here, ahead of the row's tree
   constexpr int A = FEW ? MAXP : 1;
   uint4 wr[A];
   ptx::f32x2 sc[A][4], sh[A][4];
-  auto load_weight = [&](int j) { return tid + j * T < packs ? __ldg(reinterpret_cast<const uint4*>(a.norm_w) + tid + j * T) : make_uint4(0, 0, 0, 0); };
+  auto load_weight = [&](int j) { return tid + j * T < packs ? reinterpret_cast<const uint4*>(a.norm_w)[tid + j * T] : make_uint4(0, 0, 0, 0); };
   auto load_tables = [&](int j, int row_index, ptx::f32x2 (&s)[4], ptx::f32x2 (&h)[4]) {
     const size_t at = size_t(row_index) * a.dim + size_t(tid + j * T < packs ? tid + j * T : 0) * 8;
     const float4* sp = reinterpret_cast<const float4*>(a.mod_scale + at);
     const float4* hp = reinterpret_cast<const float4*>(a.mod_shift + at);
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const float4 s4 = __ldg(sp + i), h4v = __ldg(hp + i);
+      const float4 s4 = sp[i], h4v = hp[i];
       s[2 * i] = ptx::pack2(s4.x, s4.y), s[2 * i + 1] = ptx::pack2(s4.z, s4.w);
       h[2 * i] = ptx::pack2(h4v.x, h4v.y), h[2 * i + 1] = ptx::pack2(h4v.z, h4v.w);
     }
@@ -600,17 +599,17 @@ void check_row_args(const FusedArgs& a, const char* what) {
     throw std::invalid_argument(std::string(what) + ": modulation needs scale, shift and the row index");
 }
 
-template <int MODE> void launch_fused(const FusedArgs& a, cudaStream_t stream, const char* what) {
+template <int MODE, bool BESIDE = false> void launch_fused(const FusedArgs& a, cudaStream_t stream, const char* what) {
   check_row_args(a, what);
   const int threads = ((a.dim / 16 + 31) / 32) * 32;
   const size_t smem = size_t(threads) * 17 * 4 + (256 + 16) * 4 + (a.norm_w ? size_t(a.dim) * 2 : 0);
-  reserve_dynamic_smem(reinterpret_cast<const void*>(&fused_act_kernel<MODE>), smem, what);
+  reserve_dynamic_smem(reinterpret_cast<const void*>(&fused_act_kernel<MODE, BESIDE>), smem, what);
   // As many CTAs as stay resident at once; each walks rows with a stride of the grid size.
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_act_kernel<MODE>, threads, smem) != cudaSuccess || per_sm < 1)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fused_act_kernel<MODE, BESIDE>, threads, smem) != cudaSuccess || per_sm < 1)
     per_sm = 1;
   const int grid = std::min(a.rows, per_sm * device_sm_count());
-  check_launch(launch_overlapped(size_t(a.rows) * a.dim * 4, fused_act_kernel<MODE>, dim3(grid), dim3(threads), smem, stream, a), what);
+  check_launch(launch_overlapped(size_t(a.rows) * a.dim * 4, fused_act_kernel<MODE, BESIDE>, dim3(grid), dim3(threads), smem, stream, a), what);
 }
 
 template <int MODE, int MAXP, bool FEW> cudaError_t launch_norm_as(const FusedArgs& a, int total_rows, cudaStream_t stream) {
@@ -672,9 +671,11 @@ void convrot(const __nv_bfloat16* x, __nv_bfloat16* out, int rows, int dim, int 
   if (group == 256 && dim <= 16384) {
     FusedArgs a = base_args(x, NormArgs{}, rows, dim);
     a.apply_convrot = 1;
-    a.beside = beside ? 1 : 0;
     a.bf16_out = out;
-    launch_fused<kModeRotOnly>(a, stream, "convrot");
+    if (beside)
+      launch_fused<kModeRotOnly, true>(a, stream, "convrot");
+    else
+      launch_fused<kModeRotOnly>(a, stream, "convrot");
     return;
   }
   if (group > 256) throw std::runtime_error("convrot: groups above 256 are not supported");
@@ -712,10 +713,10 @@ size_t nvfp4_act_scale_bytes(int rows, int dim) {
 // with the rows padded to a multiple of 128 (the pad rows' scales are written as zero).
 namespace {
 template <bool FEED>
-__global__ void __launch_bounds__(256) quantize_nvfp4_flat_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ packed,
+__global__ void __launch_bounds__(256) quantize_nvfp4_flat_kernel(const __nv_bfloat16* x, uint8_t* __restrict__ packed,
                                                                   uint8_t* __restrict__ scales, int rows, int padded_rows, int chunks) {
   ptx::grid_dependency_release();
-  x = ptx::grid_dependency_wait(x);
+  ptx::grid_dependency_wait();
   // item g = (row, chunk): advance by the grid's stride without a division per item
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x;
@@ -726,8 +727,8 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_flat_kernel(const __nv_bfl
     b = a;
     if (r < rows) {
       const uint4* src = reinterpret_cast<const uint4*>(x) + (size_t(r) * chunks + cc) * 2;
-      a = __ldg(src);
-      b = __ldg(src + 1);
+      a = src[0];
+      b = src[1];
     }
   };
   auto emit = [&](int r, int cc, const uint4& a, const uint4& b) {
@@ -842,8 +843,8 @@ __device__ __forceinline__ uint32_t bf16_pair(float lo, float hi) {
 }
 
 template <bool NORM, bool ROPE>
-__global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __restrict__ x, int ld, const __nv_bfloat16* __restrict__ w,
-                                                             const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
+__global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __restrict__ x, int ld, const __nv_bfloat16* w,
+                                                             const float* cos_tab, const float* sin_tab,
                                                              int tables_vec, int rows, int heads, float eps) {
   constexpr int kPer = kHeadsPerWarp / 2;  // heads per half warp
   ptx::grid_dependency_release();
@@ -869,13 +870,13 @@ __global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __re
     if (tables_vec) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const float4 c4 = __ldg(reinterpret_cast<const float4*>(cos_tab + at) + i), s4 = __ldg(reinterpret_cast<const float4*>(sin_tab + at) + i);
+        const float4 c4 = reinterpret_cast<const float4*>(cos_tab + at)[i], s4 = reinterpret_cast<const float4*>(sin_tab + at)[i];
         c[4 * i] = c4.x, c[4 * i + 1] = c4.y, c[4 * i + 2] = c4.z, c[4 * i + 3] = c4.w;
         s[4 * i] = s4.x, s[4 * i + 1] = s4.y, s[4 * i + 2] = s4.z, s[4 * i + 3] = s4.w;
       }
     } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) c[i] = __ldg(cos_tab + at + i), s[i] = __ldg(sin_tab + at + i);
+      for (int i = 0; i < 8; ++i) c[i] = cos_tab[at + i], s[i] = sin_tab[at + i];
     }
   }
   if constexpr (NORM) {
@@ -899,7 +900,7 @@ __global__ void __launch_bounds__(256) head_norm_rope_kernel(__nv_bfloat16* __re
     const float mine = (l & 1) ? odd : even;
     // mean = RNE(sum / 128), the same as the product with the power of two
     const float inv_mine = rsqrt_q30(__fadd_rn(__fmul_rn(mine, 1.0f / 128.0f), eps));
-    const uint4 wr = __ldg(reinterpret_cast<const uint4*>(w + l * 8));
+    const uint4 wr = *reinterpret_cast<const uint4*>(w + l * 8);
     const uint32_t wu[4] = {wr.x, wr.y, wr.z, wr.w};
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {

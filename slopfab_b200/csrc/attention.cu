@@ -457,11 +457,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
 }
 
 // V [seq, width] (row pitch ld_v) -> V^T [width, ld_t] with the columns [seq, ld_t) zeroed.
-__global__ void __launch_bounds__(256) transpose_v_kernel(const __nv_bfloat16* __restrict__ v, int ld_v, __nv_bfloat16* __restrict__ vt, int ld_t,
+__global__ void __launch_bounds__(256) transpose_v_kernel(const __nv_bfloat16* v, int ld_v, __nv_bfloat16* __restrict__ vt, int ld_t,
                                                           int seq, int width) {
   __shared__ __nv_bfloat16 tile[64][66];
   grid_dependency_release();
-  v = grid_dependency_wait(v);
+  grid_dependency_wait();
   const int s0 = blockIdx.x * 64, w0 = blockIdx.y * 64;
   for (int i = threadIdx.x; i < 64 * 64; i += 256) {
     const int rs = i >> 6, cw = i & 63;

@@ -155,7 +155,7 @@ __device__ __forceinline__ void flush_chunk(const uint4 (&packed)[4], uint4* sta
         // add_gated_kernel (src/cuda/nn_pointwise.cu:16-37) on the value this GEMM would have stored
         const uint4 cur = *out;
         const float4* gp = reinterpret_cast<const float4*>(gate + size_t(gate_idx[i]) * gate_ld + unit * 8);
-        const float4 g0 = __ldg(gp), g1 = __ldg(gp + 1);
+        const float4 g0 = gp[0], g1 = gp[1];
         const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
         const __nv_bfloat162* bp = reinterpret_cast<const __nv_bfloat162*>(&val);
         const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&cur);
@@ -184,7 +184,7 @@ __device__ __forceinline__ void gate_rows_for(const GemmArgs& g, int warp_row0, 
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int r = warp_row0 + 8 * i + (lane >> 2);
-    idx[i] = (g.gate != nullptr && r < g.M) ? __ldg(g.gate_index + r) : 0;
+    idx[i] = (g.gate != nullptr && r < g.M) ? g.gate_index[r] : 0;
   }
 }
 

@@ -431,10 +431,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int col = swiglu ? (et < BN / 2 ? tn * (BN / 2) + et : inner + tn * (BN / 2) + et - BN / 2) : col_base + et;
         float cs = g.global_scale, bs = 0.0f;
         if (col < g.N) {
-          if constexpr (KIND == kI8) cs = __ldg(g.col_scale + col);
+          if constexpr (KIND == kI8) cs = g.col_scale[col];
           if (has_bias)
             bs = g.bias_is_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(g.bias)[col])
-                                : __ldg(static_cast<const float*>(g.bias) + col);
+                                : static_cast<const float*>(g.bias)[col];
         }
         cs_s[et] = cs;
         bs_s[et] = bs;
@@ -454,7 +454,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const int tile_row0 = tm * kPairBM + int(rank) * kBM;
       const int row = tile_row0 + quad * 32 + lane;
       const bool row_ok = row < g.M;
-      const float rs = (KIND == kI8 && row_ok) ? __ldg(g.row_scale + row) : 1.0f;
+      const float rs = (KIND == kI8 && row_ok) ? g.row_scale[row] : 1.0f;
       __nv_bfloat16* yrow = g.y + size_t(row_ok ? row : 0) * g.ldy;
       const int warp_row0 = tile_row0 + quad * 32;
       const int rows_ok = max(0, min(32, g.M - warp_row0));
@@ -467,7 +467,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const float* gate_row = nullptr;
       if constexpr (EPI == kEpiGated) {
         gate_rows_for(g, warp_row0, lane, gate_idx);
-        if (row_ok) gate_row = g.gate + size_t(__ldg(g.gate_index + row)) * g.N;
+        if (row_ok) gate_row = g.gate + size_t(g.gate_index[row]) * g.N;
       }
       uint32_t r[kMaxJ][32];
 #pragma unroll
@@ -563,7 +563,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               if (col < g.N) {
                 __nv_bfloat16 o = __ushort_as_bfloat16((unsigned short)((w4[q >> 1] >> (16 * (q & 1))) & 0xFFFFu));
                 if (gate_row != nullptr)
-                  o = __float2bfloat16(__fmaf_rn(__ldg(gate_row + col), __bfloat162float(o), __bfloat162float(yrow[col])));
+                  o = __float2bfloat16(__fmaf_rn(gate_row[col], __bfloat162float(o), __bfloat162float(yrow[col])));
                 yrow[col] = o;
               }
             }

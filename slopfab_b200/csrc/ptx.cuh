@@ -36,22 +36,13 @@ template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setma
 // first of these returns when everything in front has completed and its writes are visible: it stands before the kernel's
 // first access to memory that an earlier kernel may write or still read. The second lets the next kernel's blocks start
 // once every block of this one has executed it (or left).
+//
+// Global memory is written while such a kernel is resident, so none of it is read-only data: its loads are ordinary ones, with no
+// __ldg and no `const ... __restrict__` parameter, from which the compiler would make read-only loads by itself. Those are not
+// ordered behind the wait, whatever the compiler is told about their addresses: with one in a branch beside the wait, a rotation
+// read the rows that the kernel in front was about to write.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// The same with a pointer that the loads behind it use: read-only (non-coherent) loads are not ordered by a memory clobber,
-// an address that comes out of the wait is.
-template <class T> __device__ __forceinline__ const T* grid_dependency_wait(const T* p) {
-  grid_dependency_wait();
-  asm volatile("" : "+l"(p)::"memory");
-  return p;
-}
-// ... or with an index, for a kernel that has no two registers to spare for a pointer it otherwise reads from the parameters.
-__device__ __forceinline__ int grid_dependency_wait(int i) {
-  grid_dependency_wait();
-  asm volatile("" : "+r"(i)::"memory");
-  return i;
-}
-
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));

@@ -98,11 +98,12 @@ __device__ __forceinline__ float div127(float m) {
 // threads (K <= 16384, whole warps) one.
 template <int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB)
-quantize_int8_pairs_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ row_scale,
+quantize_int8_pairs_kernel(const __nv_bfloat16* x, int8_t* __restrict__ q, float* __restrict__ row_scale,
                            int rows, int dim) {
   extern __shared__ __align__(16) uint8_t smem[];
   ptx::grid_dependency_release();
-  const int tid = ptx::grid_dependency_wait(int(threadIdx.x)), lane = tid & 31, warp = tid >> 5;
+  ptx::grid_dependency_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
   const int chunks = dim >> 4;
   const bool active = tid < chunks;
@@ -118,12 +119,12 @@ quantize_int8_pairs_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restri
     if (active && pair < pairs) {
       const int r0 = 2 * pair;
       const uint4* s0 = reinterpret_cast<const uint4*>(x + size_t(r0) * dim) + tid * 2;
-      r[0] = __ldg(s0);
-      r[1] = __ldg(s0 + 1);
+      r[0] = s0[0];
+      r[1] = s0[1];
       if (r0 + 1 < rows) {
         const uint4* s1 = reinterpret_cast<const uint4*>(x + size_t(r0 + 1) * dim) + tid * 2;
-        r[2] = __ldg(s1);
-        r[3] = __ldg(s1 + 1);
+        r[2] = s1[0];
+        r[3] = s1[1];
       }
     }
   };
@@ -224,11 +225,12 @@ constexpr int wide_max_threads(int nc) { return nc == 2 ? 384 : (nc == 3 ? 320 :
 
 template <int NC>
 __global__ void __launch_bounds__(wide_max_threads(NC), 2)
-quantize_int8_pairs_wide_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ row_scale,
+quantize_int8_pairs_wide_kernel(const __nv_bfloat16* x, int8_t* __restrict__ q, float* __restrict__ row_scale,
                                 int rows, int dim) {
   extern __shared__ __align__(16) uint8_t smem[];
   ptx::grid_dependency_release();
-  const int tid = ptx::grid_dependency_wait(int(threadIdx.x)), lane = tid & 31, warp = tid >> 5;
+  ptx::grid_dependency_wait();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nwarps = blockDim.x >> 5;
   f2* tile = reinterpret_cast<f2*>(smem) + (tid >> 4) * kGroupTile;
   uint8_t* bytes = smem + size_t(blockDim.x >> 4) * kGroupTile * 8 + (tid >> 4) * kGroupBytesOut;
@@ -244,10 +246,10 @@ quantize_int8_pairs_wide_kernel(const __nv_bfloat16* __restrict__ x, int8_t* __r
     const uint4* s1 = reinterpret_cast<const uint4*>(x + size_t(two ? r0 + 1 : r0) * dim);
     auto load = [&](int k, uint4 (&r)[4]) {
       const int c = k * blockDim.x + tid;
-      r[0] = __ldg(s0 + 2 * c);
-      r[1] = __ldg(s0 + 2 * c + 1);
-      r[2] = two ? __ldg(s1 + 2 * c) : make_uint4(0, 0, 0, 0);
-      r[3] = two ? __ldg(s1 + 2 * c + 1) : make_uint4(0, 0, 0, 0);
+      r[0] = s0[2 * c];
+      r[1] = s0[2 * c + 1];
+      r[2] = two ? s1[2 * c] : make_uint4(0, 0, 0, 0);
+      r[3] = two ? s1[2 * c + 1] : make_uint4(0, 0, 0, 0);
     };
     uint4 raw[2][4];  // this chunk's 64 bytes and the next chunk's, already in flight
     load(0, raw[0]);

@@ -30,7 +30,7 @@ void reserve_dynamic_smem(const void* kernel, size_t bytes, const char* what);
 
 // Launches `kernel` so that its blocks may start before the previous kernel of the stream has finished (programmatic
 // stream serialization). The kernel must execute grid_dependency_wait() (ptx.cuh) before it touches memory that an earlier
-// kernel writes or reads. What it saves is the drain of one kernel, the launch latency and the fill of the next: about 2 us
+// kernel writes or reads, unconditionally, and read none of it through the read-only path (see there). What it saves is the drain of one kernel, the launch latency and the fill of the next: about 2 us
 // per launch, which is most of a small Linear. `bytes` is what the kernel moves: a launch above kOverlapBytes is made the plain
 // way (the kernel's wait then returns at once), because there the early blocks cost more than the gap they hide -- they take
 // the SMs in the order the previous kernel leaves them, and a NVFP4 Linear of 13950 x 5120 -> 13824 measured 420.5 us overlapped
