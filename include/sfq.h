@@ -294,9 +294,11 @@ SFQ_API int sfq_gemm_bf16(const void* d_x_bf16, const void* d_w_bf16, const sfq_
  *   lost load: the producer warp leaves out the loads of pipeline iteration `iteration` (>= 0) while still announcing
  *     their bytes, and every bounded wait gives up after `wait_cycles` clocks instead of about a second. The launch then
  *     ends by the kernels' own abort path -- status code in sfq_device_status, loads drained, TMEM freed -- which is
- *     what the test of that path checks; the output of such a launch is unspecified. */
+ *     what the test of that path checks; the output of such a launch is unspecified.
+ *   no clusters: kernels are chosen as on a device that cannot schedule clusters of CTAs (0 switches it off). */
 SFQ_API void sfq_test_gemm_variant(int tile_n, int band_m, int max_ctas);
 SFQ_API void sfq_test_gemm_lost_load(int iteration, long long wait_cycles);
+SFQ_API void sfq_test_gemm_no_clusters(int on);
 
 /* ---- LinearRunner (include/slopfab/cuda/linear.cuh:182-242) ---------------- */
 

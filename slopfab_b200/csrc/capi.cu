@@ -369,5 +369,6 @@ int sfq_attention_forward(const void* d_q_bf16, int ld_q, const void* d_k_bf16, 
 }
 void sfq_test_gemm_variant(int tile_n, int band_m, int max_ctas) { sfq::set_test_gemm_variant(tile_n, band_m, max_ctas); }
 void sfq_test_gemm_lost_load(int iteration, long long wait_cycles) { sfq::set_test_gemm_lost_load(iteration, wait_cycles); }
+void sfq_test_gemm_no_clusters(int on) { sfq::set_test_gemm_no_clusters(on != 0); }
 
 }  // extern "C"

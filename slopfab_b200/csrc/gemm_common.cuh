@@ -224,5 +224,27 @@ CUtensorMap make_map(const void* base, size_t rows, size_t row_bytes, int box_ro
 
 int sm_count() { return device_sm_count(); }
 
+// How many clusters of `size` CTAs the current device can run at once (their CTAs have to fit one GPC); 0 when none can. The
+// kernel's shared memory has to be reserved already.
+template <class K> int max_clusters(K kernel, int size, size_t smem) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sm_count() / size * size);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = size;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters <= 0) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters;
+}
+
 }  // namespace
 }  // namespace sfq

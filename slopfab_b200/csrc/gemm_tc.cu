@@ -476,15 +476,24 @@ void launch(const void* a, const void* w, size_t row_bytes, const GemmArgs& g, c
 // those do, as long as each CTA keeps kMinSplitStages slabs (below that the exchange of the partial sums costs more than the
 // shorter loop saves). 77 x 5120 -> 13824 nvfp4, quantizer and launch gaps included: 20.5 us, 29.0 with 256-wide tiles.
 constexpr int kMinSplitStages = 8;
+template <int KIND, int SPLIT> bool split_fits(const GemmArgs& g) {  // this device can schedule the clusters
+  static PerDevice<int> cache;
+  return !g.test_no_clusters && cache.get([] {
+    auto kernel = gemm_kernel<KIND, 128, 2, false, SPLIT>;
+    constexpr size_t smem = Cfg<KIND, 128, 2, SPLIT>::kSmemBytes;
+    reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, "sfq gemm");
+    return max_clusters(kernel, SPLIT, smem);
+  }) > 0;
+}
 template <int KIND, int ACC256>
 void launch_few_rows(const void* a, const void* w, size_t row_bytes, const GemmArgs& g, cudaStream_t stream) {
   const int tiles = (g.N + 127) / 128, sms = sm_count();
   const int stages = int((row_bytes + kSlabBytes - 1) / kSlabBytes);
   if (tiles > sms || g.gate != nullptr)
     launch<KIND, 256, ACC256>(a, w, row_bytes, g, stream);
-  else if (4 * tiles <= sms && stages >= 4 * kMinSplitStages)
+  else if (4 * tiles <= sms && stages >= 4 * kMinSplitStages && split_fits<KIND, 4>(g))
     launch_epi<KIND, 128, 2, false, 4>(a, w, row_bytes, g, stream);
-  else if (2 * tiles <= sms && stages >= 2 * kMinSplitStages)
+  else if (2 * tiles <= sms && stages >= 2 * kMinSplitStages && split_fits<KIND, 2>(g))
     launch_epi<KIND, 128, 2, false, 2>(a, w, row_bytes, g, stream);
   else
     launch<KIND, 128, 2>(a, w, row_bytes, g, stream);

@@ -41,6 +41,7 @@ struct GemmArgs {
   int band_m = 0;         // row tiles per raster band (0 = default)
   bool serial_launch = false;  // no overlap with the previous kernel of the stream: the launch also follows another stream's work
   int max_ctas = 0;       // 0 = one CTA per SM
+  bool test_no_clusters = false;  // as on a device that cannot schedule clusters
   int tile_n = 0;         // 128 or 256 select the one-CTA kernel with that tile width; 0 = default (CTA pairs, 256 x 256)
   int tail_split = -1;    // CTA-pair kernel: trailing tiles cut into two 128-column halves (-1 = let the launcher choose)
   // test hooks (see runtime.h); never set on a runner's path

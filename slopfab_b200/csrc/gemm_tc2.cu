@@ -598,29 +598,8 @@ CUtensorMap make_scale_map(const void* base, size_t row_tiles, size_t k_atoms, i
 }
 
 template <int KIND, int ACC, int EPI> int max_pairs() {  // the same for both TAIL variants
-  // Clusters of two need both CTAs in one GPC; ask the runtime how many pairs fit at once.
   static PerDevice<int> cache;
-  return cache.get([] {
-    using C = PairCfg<KIND, ACC>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * sm_count());
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = C::kSmemBytes;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2;
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveClusters(&clusters, gemm_pair_kernel<KIND, ACC, EPI, false>, &cfg);
-    if (e != cudaSuccess || clusters <= 0) {
-      cudaGetLastError();
-      return 0;
-    }
-    return clusters;
-  });
+  return cache.get([] { return max_clusters(gemm_pair_kernel<KIND, ACC, EPI, false>, 2, PairCfg<KIND, ACC>::kSmemBytes); });
 }
 
 template <int KIND, int ACC, int EPI>
@@ -629,7 +608,7 @@ bool launch_pair_epi(const void* a, const void* w, size_t row_bytes, const GemmA
   reserve_dynamic_smem(reinterpret_cast<const void*>(&gemm_pair_kernel<KIND, ACC, EPI, false>), C::kSmemBytes, "sfq gemm");
   reserve_dynamic_smem(reinterpret_cast<const void*>(&gemm_pair_kernel<KIND, ACC, EPI, true>), C::kSmemBytes, "sfq gemm");
   const int pairs_fit = max_pairs<KIND, ACC, EPI>();
-  if (pairs_fit <= 0) return false;  // no room for clusters of two: the caller uses the one-CTA kernel
+  if (pairs_fit <= 0 || g.test_no_clusters) return false;  // no room for clusters of two: the caller uses the one-CTA kernel
   const CUtensorMap ma = make_map(a, size_t(g.M), row_bytes, kBM);
   const CUtensorMap mb = make_map(w, size_t(g.N), row_bytes, kPairBN / 2);
   const CUtensorMap mbn = make_map(w, size_t(g.N), row_bytes, kPairBN / 4);
@@ -713,24 +692,8 @@ bool gemm_pair_w4a8(const int8_t* a, const uint8_t* w_packed, const GemmArgs& g,
   auto kernel = gemm_pair_kernel<kI8, 2, kEpiPlain, false, true>;
   reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), C::kSmemBytes, "sfq gemm");
   static PerDevice<int> cache;
-  const int pairs_fit = cache.get([&] {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * sm_count());
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = C::kSmemBytes;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = 2, attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters <= 0) {
-      cudaGetLastError();
-      return 0;
-    }
-    return clusters;
-  });
-  if (pairs_fit <= 0) return false;
+  const int pairs_fit = cache.get([&] { return max_clusters(kernel, 2, C::kSmemBytes); });
+  if (pairs_fit <= 0 || g.test_no_clusters) return false;
   const CUtensorMap ma = make_map(a, size_t(g.M), size_t(g.K), kBM);
   // nibbles [N, K/2]: boxes of 64 bytes x 128 rows, unswizzled, zero beyond the array
   CUtensorMap mw;

@@ -14,6 +14,7 @@ int* g_status[kMaxDevices] = {};
 // Test hooks of the stand-alone GEMM entry points; each thread has its own, a runner never reads them.
 struct GemmHooks {
   int tile_n = 0, band_m = 0, max_ctas = 0;
+  bool no_clusters = false;
   int drop_iteration = -1;
   long long wait_cycles = 0;
 };
@@ -94,10 +95,13 @@ void set_test_gemm_lost_load(int iteration, long long wait_cycles) {
   t_hooks.wait_cycles = wait_cycles > 0 ? wait_cycles : 0;
 }
 
+void set_test_gemm_no_clusters(bool on) { t_hooks.no_clusters = on; }
+
 void apply_test_hooks(GemmArgs& g) {
   g.tile_n = t_hooks.tile_n;
   g.band_m = t_hooks.band_m;
   g.max_ctas = t_hooks.max_ctas;
+  g.test_no_clusters = t_hooks.no_clusters;
   g.test_drop_iteration = t_hooks.drop_iteration;
   g.wait_cycles = t_hooks.wait_cycles;
 }

@@ -58,6 +58,8 @@ void set_test_gemm_variant(int tile_n, int band_m, int max_ctas);
 // Lost load: the producer skips the loads of pipeline iteration `iteration` (>= 0) while still announcing their bytes, and
 // every bounded wait gives up after `wait_cycles` clocks instead of the default second; -1 / 0 switch both off.
 void set_test_gemm_lost_load(int iteration, long long wait_cycles);
+// No clusters: the launchers choose as on a device that cannot schedule clusters of CTAs.
+void set_test_gemm_no_clusters(bool on);
 void apply_test_hooks(GemmArgs& g);
 
 // A value computed once per device (occupancy answers and the like), keyed by the device that is current at the call.

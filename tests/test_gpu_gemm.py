@@ -192,6 +192,38 @@ def test_gemm_of_few_rows_equals_the_256_wide_kernel(M, N, slabs, kind):
         assert bool(((f - want).abs() <= 2.0 ** -7 * (2 * want.abs() + bias.abs()) + 1e-5 * want.abs().max()).all())
 
 
+@pytest.mark.parametrize("M,N,K", [(77, 512, 8192), (128, 4864, 4096), (300, 512, 1024)])  # four ways, two ways, CTA pairs
+def test_gemm_on_a_device_without_clusters(M, N, K):
+    """Where clusters cannot be scheduled every plain GEMM runs as single CTAs: the bits are those of the one-CTA kernel."""
+    rng = np.random.default_rng(M + N)
+    a, w = dev(rng.integers(-128, 128, size=(M, K), dtype=np.int8)), dev(rng.integers(-127, 128, size=(N, K), dtype=np.int8))
+    rs, cs = dev((rng.random(M) * 0.05 + 1e-3).astype(np.float32)), dev((rng.random(N) * 0.01 + 1e-4).astype(np.float32))
+    x, v = bf16_tensor(gaussian_bf16((M, K), seed=M)), torch.randn((N, K), device="cuda").mul_(0.02).to(torch.bfloat16)
+    ep8, ep16 = sfq.Epilogue(sfq.ptr(rs), sfq.ptr(cs), 1.0, None, sfq.F32, sfq.ACT_NONE), sfq.Epilogue(None, None, 1.0, None, sfq.F32, sfq.ACT_NONE)
+
+    def run():
+        y8, y16 = (torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+        sfq.check(sfq.lib.sfq_gemm_int8(sfq.ptr(a), sfq.ptr(w), C.byref(ep8), sfq.ptr(y8), M, N, K, S))
+        sfq.check(sfq.lib.sfq_gemm_bf16(sfq.ptr(x), sfq.ptr(v), C.byref(ep16), sfq.ptr(y16), M, N, K, S))
+        _status_clean()
+        return y8, y16
+
+    plain = run()
+    sfq.lib.sfq_test_gemm_variant(128 if M <= 128 else 256, 0, 0)
+    single = run()
+    sfq.lib.sfq_test_gemm_variant(0, 0, 0)
+    sfq.lib.sfq_test_gemm_no_clusters(1)
+    try:
+        alone = run()
+        y = torch.empty((M, N // 2), dtype=torch.bfloat16, device="cuda")
+        ep = sfq.Epilogue(sfq.ptr(rs), sfq.ptr(cs), 1.0, None, sfq.F32, sfq.ACT_SWIGLU)
+        assert sfq.lib.sfq_gemm_int8(sfq.ptr(a), sfq.ptr(w), C.byref(ep), sfq.ptr(y), M, N, K, S) == sfq.ERR_RUNTIME  # needs pairs, as ever
+    finally:
+        sfq.lib.sfq_test_gemm_no_clusters(0)
+    assert torch.equal(alone[0], plain[0]) and torch.equal(alone[0], single[0]) and torch.equal(alone[1], single[1])
+    assert M > 128 or not torch.equal(alone[1], plain[1])  # with clusters the sums of few rows are divided: another order
+
+
 def _nvfp4_case(M, N, K, seed):
     rng = np.random.default_rng(seed)
     w = (0.02 * rng.standard_normal((N, K))).astype(np.float32)
