@@ -270,7 +270,8 @@ SFQ_API int sfq_gemm_nvfp4(const uint8_t* d_a_packed, const uint8_t* d_a_scale_t
 /* The same product with its result quantized for the next one: what sfq_quantize_nvfp4_block(GEMM_FEED, no norm) makes of
  * the bf16 y that sfq_gemm_nvfp4 would have stored, byte for byte, without that y. Columns C = N (SFQ_ACT_SWIGLU: N / 2);
  * d_out_packed [M, C / 2] and d_out_scale_tiled (sfq_nvfp4_act_scale_bytes(M, C)), both 16-byte aligned and not the operand's
- * buffers. No gated residual. No counterpart in the reference, which quantizes in a launch of its own. */
+ * buffers. No gated residual. Where CTA pairs cannot be scheduled the bf16 y goes through stream-ordered scratch (SFQ_ACT_SWIGLU
+ * needs pairs, as in sfq_gemm_nvfp4). No counterpart in the reference, which quantizes in a launch of its own. */
 SFQ_API int sfq_gemm_nvfp4_quantized(const uint8_t* d_a_packed, const uint8_t* d_a_scale_tiled, const uint8_t* d_w_packed,
                                      const uint8_t* d_w_scale_tiled, const sfq_epilogue* ep, uint8_t* d_out_packed,
                                      uint8_t* d_out_scale_tiled, int M, int N, int K, void* stream);

@@ -24,6 +24,7 @@
 // abort flag and fall through to the common exit, where the producer waits
 // (bounded) for its own copies in flight and TMEM is released.
 #include "gemm_common.cuh"
+#include "kernels.cuh"
 
 namespace sfq {
 namespace {
@@ -499,6 +500,29 @@ void launch_few_rows(const void* a, const void* w, size_t row_bytes, const GemmA
     launch<KIND, 128, 2>(a, w, row_bytes, g, stream);
 }
 
+// The quantized result where CTA pairs cannot be scheduled: the bf16 result in stream-ordered scratch, then the stand-alone quantizer.
+// Same bytes. (The SwiGLU epilogue exists for pairs alone and is refused in here.)
+void quantize_plain_result(const uint8_t* a, const uint8_t* w, const GemmArgs& g, cudaStream_t stream) {
+  const auto check = [](cudaError_t e) {
+    if (e != cudaSuccess) throw std::runtime_error(std::string("sfq gemm nvfp4: scratch for the quantized result: ") + cudaGetErrorString(e));
+  };
+  const int cols = g.act == SFQ_ACT_SWIGLU ? g.N / 2 : g.N;
+  void* y = nullptr;
+  check(cudaMallocAsync(&y, size_t(g.M) * cols * sizeof(__nv_bfloat16), stream));
+  try {
+    GemmArgs plain = g;
+    plain.q_out = plain.q_scale_tiled = nullptr;
+    plain.y = static_cast<__nv_bfloat16*>(y);
+    plain.ldy = cols;
+    gemm_nvfp4(a, w, plain, stream);
+    quantize_nvfp4_block(plain.y, NormArgs{}, g.q_out, g.q_scale_tiled, nullptr, g.M, cols, SFQ_NVFP4_ACT_GEMM_FEED, stream);
+  } catch (...) {
+    cudaFreeAsync(y, stream);
+    throw;
+  }
+  check(cudaFreeAsync(y, stream));
+}
+
 }  // namespace
 
 void gemm_int8(const int8_t* a, const int8_t* w, const GemmArgs& g, cudaStream_t stream) {
@@ -532,7 +556,7 @@ void gemm_nvfp4(const uint8_t* a, const uint8_t* w, const GemmArgs& g, cudaStrea
     if (!g.q_scale_tiled || reinterpret_cast<uintptr_t>(g.q_out) % 16 != 0 || reinterpret_cast<uintptr_t>(g.q_scale_tiled) % 16 != 0)
       throw std::invalid_argument("sfq gemm nvfp4: the quantized result needs codes and scales, both 16-byte aligned");
     if (g.q_out == a || g.q_scale_tiled == g.a_scale_tiled) throw std::invalid_argument("sfq gemm nvfp4: the quantized result may not overwrite the operand");
-    if (!gemm_pair_nvfp4(a, w, g, stream)) throw std::runtime_error("sfq gemm nvfp4: the quantized result needs the CTA-pair kernel, which this device cannot schedule");
+    if (!gemm_pair_nvfp4(a, w, g, stream)) quantize_plain_result(a, w, g, stream);
     return;
   }
   // One-CTA form: a 256-wide tile has one accumulator (256 columns + the scale slots); 128-wide tiles have two

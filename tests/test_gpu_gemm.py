@@ -13,6 +13,7 @@ import torch
 
 import oracle
 import slopfab_b200 as sfq
+from slopfab_b200.block import BlockWeights, Nvfp4Block, Nvfp4Linear
 from helpers import (P, bf16_tensor, bits, dev, gaussian_bf16, pack_nvfp4, pack_w4a8, pack_w6a8, ref_check, ref_dev,
                      ref_weight_from, synthetic_packed_int8)
 
@@ -296,6 +297,58 @@ def test_gemm_nvfp4_quantized_result_equals_gemm_then_quantizer(M, N, K, act):
         _status_clean()
         assert torch.equal(got_q[:-256].view(M, cols // 2), want_q) and torch.equal(got_s[:-256], want_s)
         assert bool((got_q[-256:] == 0xA5).all()) and bool((got_s[-256:] == 0xA5).all())
+
+
+@pytest.mark.parametrize("M", [77, 300])
+def test_gemm_nvfp4_quantized_result_on_a_device_without_clusters(M):
+    """The result goes through bf16 scratch and the stand-alone quantizer there; eagerly and captured, and in a block, which used to
+    run on such devices in its GELU form. SwiGLU is refused, as in the GEMM itself."""
+    N, K = 512, 1024
+    g = torch.Generator("cuda").manual_seed(M)
+    x = torch.randn((M, K), device="cuda", generator=g).to(torch.bfloat16)
+    data, scale, top = pack_nvfp4((0.02 * np.random.default_rng(1).standard_normal((N, K))).astype(np.float32))
+    w, sw = dev(data), dev(scale)
+    a = torch.empty((M, K // 2), dtype=torch.uint8, device="cuda")
+    sa = torch.empty(sfq.lib.sfq_nvfp4_act_scale_bytes(M, K), dtype=torch.uint8, device="cuda")
+    sfq.check(sfq.lib.sfq_quantize_nvfp4_block(sfq.ptr(x), None, sfq.ptr(a), sfq.ptr(sa), None, M, K, sfq.NVFP4_ACT_GEMM_FEED, S))
+    q = torch.zeros((M, N // 2), dtype=torch.uint8, device="cuda")
+    s = torch.zeros(sfq.lib.sfq_nvfp4_act_scale_bytes(M, N), dtype=torch.uint8, device="cuda")
+    ep = lambda act: sfq.Epilogue(None, None, top, None, sfq.F32, act)  # noqa: E731
+    run = lambda act: sfq.lib.sfq_gemm_nvfp4_quantized(sfq.ptr(a), sfq.ptr(sa), sfq.ptr(w), sfq.ptr(sw), C.byref(ep(act)), sfq.ptr(q), sfq.ptr(s),  # noqa: E731
+                                                       M, N, K, sfq.stream_ptr())
+    hidden, heads, ffn = 1024, 8, 2048
+    lin = lambda n, k: Nvfp4Linear(*(dev(t) for t in pack_nvfp4((0.02 * np.random.default_rng(n).standard_normal((n, k))).astype(np.float32))[:2]), 1e-5, n, k)  # noqa: E731
+    ones = torch.ones(hidden, dtype=torch.bfloat16, device="cuda")
+    weights = BlockWeights(lin(3 * hidden, hidden), lin(hidden, hidden), lin(ffn, hidden), lin(hidden, ffn), ones, ones)
+    mod = {name: 0.1 * torch.randn((3, hidden), device="cuda", generator=g) for name in ("scale_msa", "shift_msa", "gate_msa", "scale_mlp", "shift_mlp", "gate_mlp")}
+    index = torch.zeros(M, dtype=torch.int32, device="cuda")
+    block = Nvfp4Block(M, hidden, heads, ffn)
+    want_x = block.forward(x.clone(), weights, mod, index)
+    sfq.lib.sfq_test_gemm_no_clusters(1)
+    try:
+        for act in (sfq.ACT_NONE, sfq.ACT_GELU_TANH):
+            y = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+            sfq.check(sfq.lib.sfq_gemm_nvfp4(sfq.ptr(a), sfq.ptr(sa), sfq.ptr(w), sfq.ptr(sw), C.byref(ep(act)), sfq.ptr(y), M, N, K, S))
+            want_q, want_s = torch.empty_like(q), torch.empty_like(s)
+            sfq.check(sfq.lib.sfq_quantize_nvfp4_block(sfq.ptr(y), None, sfq.ptr(want_q), sfq.ptr(want_s), None, M, N, sfq.NVFP4_ACT_GEMM_FEED, S))
+            sfq.check(run(act))
+            assert torch.equal(q, want_q) and torch.equal(s, want_s)
+            graph = torch.cuda.CUDAGraph()
+            torch.cuda.synchronize()
+            with torch.cuda.graph(graph):
+                sfq.check(run(act))
+            q.zero_(), s.zero_()
+            for _ in range(2):
+                graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(q, want_q) and torch.equal(s, want_s)
+        assert run(sfq.ACT_SWIGLU) == sfq.ERR_RUNTIME
+        got_x = block.forward(x.clone(), weights, mod, index)
+    finally:
+        sfq.lib.sfq_test_gemm_no_clusters(0)
+    # another order of fp32 sums at most, i.e. a last bf16 bit here and there that the fp4 codes behind it amplify
+    assert float((got_x.float() - want_x.float()).norm() / want_x.float().norm()) < 2e-2
+    _status_clean()
 
 
 def test_gemm_nvfp4_quantized_refusals():
