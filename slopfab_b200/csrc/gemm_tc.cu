@@ -312,7 +312,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
         }
       }
       asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (!(ok = wait_barrier(smem_u32(&sh->acc_full[a]), aph, sh, g.status, 4))) {
+      // One verdict per warp: lanes of a warp that went different ways here would wait for each other, some at a warp-wide
+      // instruction, some at the cluster barrier.
+      if (!(ok = wait_barrier_warp(smem_u32(&sh->acc_full[a]), aph, sh, g.status, 4))) {
         if constexpr (SPLIT > 1) cluster_wait(), cluster_sync_all();  // the other CTAs are not left waiting
         break;
       }

@@ -1,4 +1,4 @@
-"""The abort path of the CTA-pair GEMMs: a bounded wait that runs out must end the launch by itself.
+"""The abort path of the GEMMs, on CTA pairs and on clusters that divide K: a bounded wait that runs out must end the launch by itself.
 
 Every barrier wait in the GEMM kernels has a limit; past it a thread records a status code, raises its CTA's abort
 flag, the producer lets the copies in flight land, the accumulator memory (TMEM) is handed back and the kernel
@@ -65,12 +65,15 @@ def _nvfp4_launch(M, N, K, seed):
     return launch, want, keep
 
 
-@pytest.mark.parametrize("kind", ["int8", "nvfp4"])
-def test_a_lost_load_ends_through_the_abort_path(kind):
-    M, N, K = 512, 512, 2048  # CTA-pair kernel, four tiles, 16 (int8) or 8 (fp4) pipeline stages per tile
+@pytest.mark.parametrize("kind,M,N,K", [
+    ("int8", 512, 512, 2048), ("nvfp4", 512, 512, 2048),  # CTA-pair kernel, four tiles, 16 (int8) or 8 (fp4) pipeline stages per tile
+    ("int8", 77, 512, 4096), ("nvfp4", 77, 512, 8192),    # few rows, K divided over clusters of four CTAs, eight stages each
+    ("int8", 128, 4864, 2304), ("nvfp4", 33, 4864, 4608),  # ... of two (on 148 SMs), nine stages each
+])
+def test_a_lost_load_ends_through_the_abort_path(kind, M, N, K):
     launch, want, keep = (_int8_launch if kind == "int8" else _nvfp4_launch)(M, N, K, seed=11)
     assert sfq.device_status() == 0
-    sfq.lib.sfq_test_gemm_lost_load(5, WAIT_CYCLES)  # every pair's sixth stage never arrives
+    sfq.lib.sfq_test_gemm_lost_load(5, WAIT_CYCLES)  # every pair's or CTA's sixth stage never arrives
     try:
         launch()
         torch.cuda.synchronize()  # returns: the kernel ended by itself
