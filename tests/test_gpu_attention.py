@@ -132,6 +132,59 @@ def test_last_wave_as_single_query_tiles(seq, heads):
     assert sfq.device_status() == 0
 
 
+def heads_of_whole_blocks(seq):
+    """A head count whose launch keeps every block of 256 queries in one CTA of two query tiles: the last wave is more than half full."""
+    sms, blocks = torch.cuda.get_device_properties(0).multi_processor_count, -(-seq // 256)
+    heads = next(h for h in range(1, 4 * sms) if 2 * (blocks * h % sms) > sms)
+    assert blocks * heads < 16 * sms
+    return heads
+
+
+@pytest.mark.parametrize("seq", [257, 385, 513, 1000])
+@pytest.mark.parametrize("aligned_v", [True, False])
+def test_whole_blocks_of_two_query_tiles(seq, aligned_v):
+    """Two query tiles per CTA throughout, V as it lies and transposed: against torch, and each head bit for bit the same head alone
+    (which runs as single query tiles)."""
+    heads = heads_of_whole_blocks(seq)
+    g = torch.Generator("cuda").manual_seed(seq)
+    q, k, v = (torch.randn((seq, heads * D), device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    if not aligned_v:
+        shifted = torch.empty(seq * heads * D + 8, dtype=torch.bfloat16, device="cuda")[3:3 + seq * heads * D].view(seq, heads * D)
+        shifted.copy_(v)
+        v = shifted
+    out = attention(q, k, v, heads, heads)
+    sh = lambda t: t.view(seq, heads, D).transpose(0, 1).float()  # noqa: E731
+    want = torch.nn.functional.scaled_dot_product_attention(sh(q), sh(k), sh(v)).transpose(0, 1).reshape(seq, heads * D)
+    assert bool(((out.float() - want).abs() <= 1e-3 + 1e-2 * want.abs()).all())
+    for h in (0, heads // 2, heads - 1):
+        one = attention(*(t[:, h * D:(h + 1) * D].contiguous() for t in (q, k, v)), 1, 1)
+        assert torch.equal(out[:, h * D:(h + 1) * D], one)
+    assert sfq.device_status() == 0
+
+
+@pytest.mark.parametrize("aligned_v", [True, False])
+@pytest.mark.parametrize("spike", [0, 95, 96, 128 + 95, 128 + 127, 256 + 110, 399, "ramp"])
+def test_reference_that_moves_in_whole_blocks(spike, aligned_v):
+    """The maxima of the tests above through CTAs of two query tiles: every query head is the same one, over one key / value head."""
+    seq = 400
+    heads = heads_of_whole_blocks(seq)
+    q, k, v = data(seq, 1, 81, 1.0), data(seq, 1, 82, 0.3), data(seq, 1, 83, 1.0)
+    if spike == "ramp":
+        k = oracle.from_bf16(oracle.to_bf16(np.where(q[0:1] < 0, -1.0, 1.0) * (0.2 + 3.0 * np.arange(seq) / seq).astype(np.float32)[:, None]))
+    else:
+        k[spike] = oracle.from_bf16(oracle.to_bf16((4.0 * np.where(q[spike // 2] < 0, -1.0, 1.0)).astype(np.float32)))
+    want = oracle.attention(q, k, v, 1, 1, D, 1.0 / np.sqrt(D))
+    dq, dk, dv = (bf16_tensor(oracle.to_bf16(t)) for t in (q, k, v))
+    if not aligned_v:
+        shifted = torch.empty(seq * D + 8, dtype=torch.bfloat16, device="cuda")[5:5 + seq * D].view(seq, D)
+        shifted.copy_(dv)
+        dv = shifted
+    out = attention(dq.repeat(1, heads), dk, dv, heads, 1)
+    close(want, oracle.from_bf16(bits(out[:, :D].contiguous())))
+    assert torch.equal(out, out[:, :D].repeat(1, heads))
+    assert sfq.device_status() == 0
+
+
 @pytest.mark.parametrize("seq,heads,scale,crc", [(1500, 2, 1.0, 0xBF518A00), (2051, 4, 0.3, 0x633D8771), (513, 40, 1.0, 0x323EB421)])
 def test_bits_of_seeded_calls(seq, heads, scale, crc):
     """How a key tile's probabilities are handed to the second product is a matter of speed alone: their sum is one chain over the
