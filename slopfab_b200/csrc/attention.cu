@@ -122,7 +122,7 @@ __device__ __forceinline__ f32x2 exp2_pair_fma(f32x2 x) {
 // the rest, so that most of O += P V runs under the last chunk's exponentials instead of behind them. A query tile's own chain
 // (scores -> softmax -> product -> next scores) is what bounds the kernel, not the tensor pipe. 40 heads, 18900 / 4747 tokens:
 // one part 6.00 / 0.534 ms, three chunks first 5.83 / 0.505 ms, two chunks first 5.93 / 0.517 ms.
-constexpr int kFirstChunks = 3;
+constexpr int kFirstChunks = 3;  // the issuer's products below are cut for this value
 constexpr int kFmaPairsOfFour = 1;  // of every four pairs of probabilities, how many take the FMA-pipe exponential
 
 // TAIL: the units of the last wave run as CTAs of one query tile each (see attention_forward). Without it every CTA has two
@@ -247,17 +247,14 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       tc_fence_after_sync();
       if (elect_one()) {
         mma_f16_ts_x4<kStep>(d, a, b, idesc_pv, j ? 1u : 0u);
-        if (kFirstChunks == 3) mma_f16_ts_x2<kStep>(d, a + 32, b + kKeys64, idesc_pv, 1u);
+        mma_f16_ts_x2<kStep>(d, a + 32, b + kKeys64, idesc_pv, 1u);
         tc_commit(smem_u32(&sh->pv_part[t]));
       }
       __syncwarp();
       if (!wait(&sh->p_full[t], j & 1, 19)) return false;
       tc_fence_after_sync();
       if (elect_one()) {
-        if (kFirstChunks == 3)
-          mma_f16_ts_x2<kStep>(d, a + 48, b + kKeys64 + 2 * kStep, idesc_pv, 1u);
-        else
-          mma_f16_ts_x4<kStep>(d, a + 32, b + kKeys64, idesc_pv, 1u);
+        mma_f16_ts_x2<kStep>(d, a + 48, b + kKeys64 + 2 * kStep, idesc_pv, 1u);
         if (t == int(two)) tc_commit(smem_u32(&sh->v_empty[st]));
         if (!more) tc_commit(smem_u32(&sh->pv_done[t]));
       }
