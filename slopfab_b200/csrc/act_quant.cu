@@ -384,19 +384,6 @@ struct E4m3Reciprocals {
 };
 __device__ const E4m3Reciprocals kE4m3Reciprocal;
 
-// Eight values -> four bytes of e2m1 pairs. HIGH_EVEN: the even element in the high nibble (GEMM feed), else in the low one.
-template <bool HIGH_EVEN> __device__ __forceinline__ uint32_t e2m1_word(const float (&v)[8]) {
-  uint32_t w;
-  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b0, %1, %2;\n\tcvt.rn.satfinite.e2m1x2.f32 b1, %3, %4;\n\t"
-      "cvt.rn.satfinite.e2m1x2.f32 b2, %5, %6;\n\tcvt.rn.satfinite.e2m1x2.f32 b3, %7, %8;\n\t"
-      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
-      : "=r"(w)
-      : "f"(v[HIGH_EVEN ? 0 : 1]), "f"(v[HIGH_EVEN ? 1 : 0]), "f"(v[HIGH_EVEN ? 2 : 3]), "f"(v[HIGH_EVEN ? 3 : 2]),
-        "f"(v[HIGH_EVEN ? 4 : 5]), "f"(v[HIGH_EVEN ? 5 : 4]), "f"(v[HIGH_EVEN ? 6 : 7]), "f"(v[HIGH_EVEN ? 7 : 6]));
-  return w;
-}
-
 template <int MODE, int MAXP, bool FEW>
 __global__ void __launch_bounds__(kNormThreads<FEW>, FEW ? (MAXP <= 4 ? 2 : 1) : (MAXP <= 2 ? 8 : 4)) norm_rows_kernel(const FusedArgs a, int total_rows) {
   constexpr int T = kNormThreads<FEW>, R = kNormRows<MAXP, FEW>;
@@ -527,7 +514,7 @@ __global__ void __launch_bounds__(kNormThreads<FEW>, FEW ? (MAXP <= 4 ? 2 : 1) :
         uint32_t m = hmax2(hmax2(habs2(n[0]), habs2(n[1])), hmax2(habs2(n[2]), habs2(n[3])));
         m = hmax2(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
         m = hmax2(hmax2(m, m >> 16), 0u);  // the reference's maximum starts at 0, which a block of NaNs alone leaves: scale 0
-        uint32_t s8 = row < a.rows ? uint32_t(__nv_cvt_float_to_fp8(__uint_as_float(m << 16) * (1.0f / 6.0f), __NV_SATFINITE, __NV_E4M3)) : 0u;
+        uint32_t s8 = row < a.rows ? uint32_t(fp4_scale_byte(m)) : 0u;
         const float rcp = __ldg(kE4m3Reciprocal.v + s8);
         const ptx::f32x2 rcp2 = ptx::pack2(rcp, rcp);
         float q[8];
@@ -705,7 +692,7 @@ size_t nvfp4_act_scale_bytes(int rows, int dim) {
 }
 
 // ---- per-16-block fp4 quantizer without a norm in front (the Linear's own case) --------------------------------------
-// The same arithmetic as the fp4 branch of process_row (quantize_act_kernel, src/cuda/nvfp4_gemm.cu:107-158): per 16
+// The arithmetic of fp4_block.cuh (quantize_act_kernel, src/cuda/nvfp4_gemm.cu:107-158): per 16
 // elements s8 = e4m3_rn_sat(amax / 6), inv = 1 / decode(s8) (0 for an all-zero block), code = e2m1_rn_sat(x * inv). A
 // block's scale depends on that block alone, so there is nothing to exchange between threads: the activation is walked as
 // a flat array of 16-element blocks, two per thread in flight, with no barrier and no shared memory, the maximum on
