@@ -474,10 +474,12 @@ void launch(const void* a, const void* w, size_t row_bytes, const GemmArgs& g, c
     launch_epi<KIND, BN, ACC, false>(a, w, row_bytes, g, stream);
 }
 
-// At most 128 rows: the launch is bound by reading the weight, and an SM takes in no more than about 100 GB/s, so what counts
-// is how many SMs read. 128-wide tiles where 256-wide ones would leave SMs idle; and K split two or four ways where even
-// those do, as long as each CTA keeps kMinSplitStages slabs (below that the exchange of the partial sums costs more than the
-// shorter loop saves). 77 x 5120 -> 13824 nvfp4, quantizer and launch gaps included: 20.5 us, 29.0 with 256-wide tiles.
+// At most 128 rows: a launch is its start-up and first loads (4 us), the weight at a rate that grows with the number of SMs that
+// read it, and the epilogue of one tile (1 us, 4 with GELU). nvfp4, 77 rows, from times at different K: 54 SMs read 3.2 TB/s, 108
+// SMs 5.5 (4.8 as 54 pairs that share K), all 148 6.3. So the tiles are 128 wide where 256-wide ones would leave SMs idle, and K is split two or four ways
+// where even those do, as long as each CTA keeps kMinSplitStages slabs (below that the exchange of the partial sums costs more than
+// the shorter loop saves). 77 x 5120 -> 13824 nvfp4 with GELU: 14.3 us (11.5 without), 17.2 with the quantizer in front of it; 29.0
+// with 256-wide tiles and launches that do not overlap.
 constexpr int kMinSplitStages = 8;
 template <int KIND, int SPLIT> bool split_fits(const GemmArgs& g) {  // this device can schedule the clusters
   static PerDevice<int> cache;
