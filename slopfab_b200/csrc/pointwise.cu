@@ -51,19 +51,27 @@ __global__ void add_gated_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloa
   x[at] = __float2bfloat16(fmaf(g, __bfloat162float(branch[at]), __bfloat162float(x[at])));
 }
 
-// Eight elements per thread, 128-bit accesses; same arithmetic as add_gated_kernel. Launched plainly: its blocks live for one memory
-// round trip, and the two instructions of an overlapped launch at the head of each cost more than the gap they hide (30000 x 256
-// 18.5 us, 32.0 with them; 5000 x 5120 22.5 / 28.8 back to back; 75600 x 5120 360 / 396).
-__global__ void add_gated_vec_kernel(__nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ branch,
-                                     const float* __restrict__ gate, const int32_t* __restrict__ a, int packs) {
+constexpr int kGatedThreads = 128;
+
+// Eight elements per thread, 128-bit accesses; same arithmetic as add_gated_kernel. A block lives for one memory round trip, so the
+// two instructions of an overlapped launch at its head cost a launch of many waves more than the gap they hide (75600 x 5120 360 us, 396
+// with them; 30000 x 256 18.5 / 32.0; 2000 rows 8.4 / 11.6), and save it in a launch of two waves or less: a block of the DiT of 310 rows
+// takes 157 us with them, 163 without, of 460 rows 162 / 170, of 2000 rows 441 / 433.
+template <bool OVERLAP>
+__global__ void __launch_bounds__(kGatedThreads) add_gated_vec_kernel(__nv_bfloat16* x, const __nv_bfloat16* branch, const float* gate, const int32_t* a,
+                                                                      int packs) {
+  if constexpr (OVERLAP) {
+    grid_dependency_release();
+    grid_dependency_wait();
+  }
   const size_t row = blockIdx.x;
   const int p = blockIdx.y * blockDim.x + threadIdx.x;
   if (p >= packs) return;
   const size_t dim = size_t(packs) * 8;
   const float4* g = reinterpret_cast<const float4*>(gate + size_t(a[row]) * dim) + p * 2;
   uint4* xp = reinterpret_cast<uint4*>(x + row * dim) + p;
-  const uint4 xv = *xp, bv = __ldg(reinterpret_cast<const uint4*>(branch + row * dim) + p);
-  const float4 g0 = __ldg(g), g1 = __ldg(g + 1);
+  const uint4 xv = *xp, bv = reinterpret_cast<const uint4*>(branch + row * dim)[p];
+  const float4 g0 = g[0], g1 = g[1];
   const float gg[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
   const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
   const __nv_bfloat162* bh = reinterpret_cast<const __nv_bfloat162*>(&bv);
@@ -142,10 +150,15 @@ void add_gated(__nv_bfloat16* x, const __nv_bfloat16* branch, const float* gate,
   if (!x || !branch || !gate || !index) throw std::invalid_argument("add_gated: null buffer");
   const bool vec = dim % 8 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(branch) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(gate) % 16 == 0;
-  if (vec)
-    add_gated_vec_kernel<<<dim3(rows, (dim / 8 + 127) / 128), 128, 0, stream>>>(x, branch, gate, index, dim / 8);
-  else
+  if (vec) {
+    const dim3 grid(rows, (dim / 8 + kGatedThreads - 1) / kGatedThreads);
+    const bool two_waves = size_t(rows) * grid.y <= size_t(2) * (2048 / kGatedThreads) * device_sm_count();
+    const cudaError_t e = two_waves ? launch_overlapped(0, add_gated_vec_kernel<true>, grid, dim3(kGatedThreads), 0, stream, x, branch, gate, index, dim / 8)
+                                    : launch_overlapped(kNoOverlap, add_gated_vec_kernel<false>, grid, dim3(kGatedThreads), 0, stream, x, branch, gate, index, dim / 8);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("add_gated: ") + cudaGetErrorString(e));
+  } else {
     add_gated_kernel<<<dim3(rows, (dim + 255) / 256), 256, 0, stream>>>(x, branch, gate, index, dim);
+  }
   check_launch("add_gated");
 }
 

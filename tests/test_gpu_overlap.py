@@ -159,6 +159,28 @@ def test_head_norm_and_rope(operand):
     assert not torch.equal(old, t["x"]) and all(torch.equal(g, t["x"]) for g in got)
 
 
+@pytest.mark.parametrize("rows", [300, 1500])  # launched overlapped and plainly
+@pytest.mark.parametrize("operand", ["x", "branch", "gate", "index"])
+def test_gated_residual(operand, rows):
+    dim = 5120
+    sizes = {"x": 2 * rows * dim, "branch": 2 * rows * dim, "gate": 12 * dim, "index": 4 * rows}
+    front = Front(sizes[operand], zeros=operand in ("gate", "index"))
+    t = {"x": bf16((rows, dim), 1), "branch": bf16((rows, dim), 2), "gate": bf16((3, dim), 3).float(),
+         "index": torch.arange(rows, device="cuda", dtype=torch.int32) % 3}
+    dtype = {"x": "bf16", "branch": "bf16", "gate": torch.float32, "index": torch.int32}[operand]
+    t[operand] = front.view(torch.bfloat16 if dtype == "bf16" else dtype, *t[operand].shape)
+    source = t["x"].clone()
+
+    def call():
+        sfq.check(lib.sfq_add_gated(ptr(t["x"]), ptr(t["branch"]), ptr(t["gate"]), ptr(t["index"]), rows, dim, sfq.stream_ptr()))
+        out = t["x"].clone()
+        if operand != "x":
+            t["x"].copy_(source)  # the kernel works in place
+        return [out]
+
+    agrees(front, random_bytes(front, dtype), call)
+
+
 @pytest.mark.parametrize("operand,offset", [("q", 0), ("k", 0), ("v", 0), ("v", 6)])
 @pytest.mark.parametrize("seq,heads", [(300, 4), (513, 40)])
 def test_attention(operand, offset, seq, heads):
