@@ -16,7 +16,7 @@
 //               softmax warpgroups run with 232 registers, the first warpgroup with 40), one query row per thread with all 128 keys of the
 //               tile: S from TMEM, P = exp2(s - m) as bf16 pairs back into TMEM, the running sum, and - only when the
 //               part's probabilities sum to more than 2^15, i.e. the row has outgrown the reference maximum m the
-//               accumulator was last scaled to - the true running maximum, a rescale of O in TMEM and the tile's
+//               accumulator was last scaled to - the true running maximum, a rescale of O in TMEM and the part's
 //               probabilities again. A stale reference changes nothing in exact arithmetic (numerator and denominator
 //               carry the same factor); the limit keeps every p far inside the range of bf16 and fp32, and no maximum over
 //               the scores is computed on the common path.
@@ -53,7 +53,7 @@ struct AttnShared {
   uint32_t tmem_base;
   volatile int abort;
 };
-constexpr int kAttnSmem = 1024 /* alignment slack */ + 6 * kTileBytes /* Q x2, K x2, V^T x2 */ + 1024;
+constexpr int kAttnSmem = 1024 /* alignment slack */ + 6 * kTileBytes /* Q x2, K x2, V x2 */ + 1024;
 
 struct AttnArgs {
   __nv_bfloat16* out;
