@@ -4,22 +4,27 @@
 // (include/slopfab/cuda/attention.cuh:176-196): q, k, v are [seq, heads * 128] row-major bf16, exactly the thirds of the
 // fused QKV projection; queries may be a compact chunk of the sequence; no mask exists anywhere in the model.
 //
-// One CTA owns TWO tiles of 128 queries of one head and walks the keys in tiles of 128 with an online softmax, so that the
-// softmax of one query tile runs while the tensor pipe works on the other tile's products:
+// One CTA owns TWO tiles of 128 queries of one head and walks the keys in steps of 64 with an online softmax. The scores of a
+// query tile lie in two halves of 64 columns that take turns, so a step's scores are computed while the softmax warps work on the
+// step before: a query tile's chain (scores -> softmax -> product -> next scores) never stands still at either end.
 //   warp 0      TMA producer: both Q tiles once, then a two-stage ring of K and V tiles [128 keys x 128 d]. The second product
 //               reads V as it lies, as an N-major operand (its N is d, its K the keys), or - VT, where its rows are not aligned -
 //               V transposed once per call by transpose_v_kernel, [128 d x 128 keys], K-major like the other operands
-//   warp 1      issues, per key tile j: O0 += P0(j) V(j), S0 = Q0 K(j+1)^T, O1 += P1(j) V(j), S1 = Q1 K(j+1)^T (8 MMAs
-//               128x128x16 each; the product with V in two parts, as its probabilities arrive). S and O of both query tiles live in TMEM (4 x 128 columns); P is read by the second
-//               product straight from TMEM, where it overwrites the first 64 columns of the scores it was computed from
-//   warps 4-7   softmax of query tile 0, warps 8-11 of query tile 1 (warps 2-3 only hand their registers over: the
-//               softmax warpgroups run with 232 registers, the first warpgroup with 40), one query row per thread with all 128 keys of the
-//               tile: S from TMEM, P = exp2(s - m) as bf16 pairs back into TMEM, the running sum, and - only when the
-//               part's probabilities sum to more than 2^15, i.e. the row has outgrown the reference maximum m the
-//               accumulator was last scaled to - the true running maximum, a rescale of O in TMEM and the part's
+//   warp 1      one lane issues, per step h and query tile t: O_t += P_t(h) V(h) (four MMAs 128x128x16), S_t(h + 2) = Q_t K(h + 2)^T
+//               (eight MMAs 128x64x16) over the columns P_t(h) was read from, and a commit. S and O of both query tiles live in
+//               TMEM (4 x 128 columns); P is read by the second product straight from TMEM, where it overwrites the first
+//               32 columns of the 64 scores it was computed from
+//   warps 4-7   softmax of query tile 0, warps 8-11 of query tile 1 (warps 2-3 only hand their registers over), one query row per
+//               thread with all 64 keys of the step: S from TMEM, P = exp2(s - m) as bf16 pairs back into TMEM, the running sum,
+//               and - only when the step's probabilities sum to more than 2^15, i.e. the row has outgrown the reference maximum m the
+//               accumulator was last scaled to - the true running maximum, a rescale of O in TMEM and the step's
 //               probabilities again. A stale reference changes nothing in exact arithmetic (numerator and denominator
 //               carry the same factor); the limit keeps every p far inside the range of bf16 and fp32, and no maximum over
 //               the scores is computed on the common path.
+// 40 heads, 2048 / 4747 / 18900 tokens in bursts: 0.096 / 0.403 / 5.47 ms; steps of 128 keys, whose next scores wait for the product that
+// still reads P from their columns, 0.107 / 0.448 / 5.72 ms. What bounds it now (timing-only ablations at 18900 tokens): the
+// tensor side alone takes 4.6 ms, most of it shared memory (a 128x64x16 MMA reads 6 KB in the 32 cycles its arithmetic takes and runs
+// in 48), the softmax side alone 4.2.
 // Every wait is bounded; a wait that runs out stores a code in the status word and the CTA leaves.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -43,13 +48,14 @@ using namespace ptx;
 constexpr int kTile = 128;             // queries per query tile (two per CTA), keys per step, head_dim
 constexpr int kSlab = kTile * 128;     // 128 rows x 128 bytes: 64 bf16 columns of a tile
 constexpr int kTileBytes = 2 * kSlab;  // [128 x 128] bf16
+constexpr int kStep = 64;              // keys per softmax step: half a key tile, half of a query tile's score columns
 constexpr int kAttnThreads = 384;  // warpgroup 0: producer, MMA issuer, two idle warps; warpgroups 1 and 2: the softmax of query tiles 0 and 1
-constexpr int kAttnRegsLean = 40, kAttnRegsSoftmax = 232;  // after setmaxnreg: 128 x 40 + 256 x 232 = 384 x 168, what the launch allocates (56 / 216: 1.3 % slower)
+constexpr int kAttnRegsLean = 64, kAttnRegsSoftmax = 216;  // after setmaxnreg: 128 x 64 + 256 x 216 < 384 x 168, what the launch allocates
 constexpr int kTailWaves = 16;
-constexpr float kTileSumLimit = 32768.0f;  // either part of a key tile's probabilities (96 and 32 keys) may sum to this before the reference maximum moves, so a tile to twice that
+constexpr float kTileSumLimit = 32768.0f;  // a row's probabilities of a key tile may sum to this before its reference maximum moves
 
 struct AttnShared {
-  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_part[2], p_full[2], pv_part[2], pv_done[2];
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2][2], p_full[2][2];
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -118,11 +124,6 @@ __device__ __forceinline__ f32x2 exp2_pair_fma(f32x2 x) {
   unpack2(t, t0, t1);
   return pack2(__int_as_float(__float_as_int(p0) + (__float_as_int(t0) << 23)), __int_as_float(__float_as_int(p1) + (__float_as_int(t1) << 23)));
 }
-// A query tile's probabilities are handed to the second product in two parts: the first kFirstChunks chunks of 32 keys, then
-// the rest, so that most of O += P V runs under the last chunk's exponentials instead of behind them. A query tile's own chain
-// (scores -> softmax -> product -> next scores) is what bounds the kernel, not the tensor pipe. 40 heads, 18900 / 4747 tokens:
-// one part 6.00 / 0.534 ms, three chunks first 5.83 / 0.505 ms, two chunks first 5.93 / 0.517 ms.
-constexpr int kFirstChunks = 3;  // the issuer's products below are cut for this value
 constexpr int kFmaPairsOfFour = 1;  // of every four pairs of probabilities, how many take the FMA-pipe exponential
 
 // TAIL: the units of the last wave run as CTAs of one query tile each (see attention_forward). Without it every CTA has two
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   uint8_t* v_s = smem + 4 * kTileBytes;   // two stages
   AttnShared* sh = reinterpret_cast<AttnShared*>(smem + 6 * kTileBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = int(warp_uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   const int tail_cta = TAIL ? int(blockIdx.x) - g.whole : -1;
   const int unit = tail_cta < 0 ? int(blockIdx.x) : g.whole + (tail_cta >> 1);
   const int q0 = (TAIL ? unit % g.q_blocks : unit) * (2 * kTile) + (tail_cta < 0 ? 0 : (tail_cta & 1) * kTile);
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   if (TAIL && q0 >= g.seq_q) return;  // the second half of a split block may have no queries
   const bool two = !TAIL || (tail_cta < 0 && q0 + kTile < g.seq_q);  // otherwise query tile 0 alone
   const int kv_head = head / g.group;
-  const int tiles = (g.seq_kv + kTile - 1) / kTile;
+  const int tiles = (g.seq_kv + kTile - 1) / kTile, steps = (g.seq_kv + kStep - 1) / kStep;
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&sh->q_full), 1);
@@ -155,11 +156,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       mbar_init(smem_u32(&sh->k_empty[i]), 1);
       mbar_init(smem_u32(&sh->v_full[i]), 1);
       mbar_init(smem_u32(&sh->v_empty[i]), 1);
-      mbar_init(smem_u32(&sh->s_full[i]), 1);   // per query tile: the scores of the current key tile are in TMEM
-      mbar_init(smem_u32(&sh->p_part[i]), 4);   // per query tile: its four softmax warps have written P of the first chunks (and rescaled O)
-      mbar_init(smem_u32(&sh->p_full[i]), 4);   // per query tile: ... of the remaining chunks
-      mbar_init(smem_u32(&sh->pv_part[i]), 1);  // per query tile: O += P V over the first chunks' keys has completed
-      mbar_init(smem_u32(&sh->pv_done[i]), 1);  // per query tile: O += P V of the last key tile has completed
+      for (int half = 0; half < 2; ++half) {  // per query tile i and half of its score columns
+        mbar_init(smem_u32(&sh->s_full[i][half]), 1);  // the product that read the half has completed, and the next scores are in it
+        mbar_init(smem_u32(&sh->p_full[i][half]), 4);  // the four softmax warps have written P over it (and rescaled O)
+      }
     }
     sh->abort = 0;
     fence_barrier_init();
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   tc_fence_after_sync();
   grid_dependency_release();
   grid_dependency_wait();  // q, k and the transposed v
-  const uint32_t tmem = sh->tmem_base;  // columns: S/P of tile 0 [0,128), of tile 1 [128,256), O of tile 0 [256,384), of tile 1 [384,512)
+  const uint32_t tmem = warp_uniform(sh->tmem_base);  // columns: S/P of tile 0 [0,128), of tile 1 [128,256), O of tile 0 [256,384), of tile 1 [384,512)
 
   // Each role's code sits directly under its warpgroup's setmaxnreg, so the compiler budgets it accordingly.
   if (warp < 4) {
@@ -208,71 +208,79 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (converged warp, one elected lane issues)
-    // Issue order per key tile j: O0 += P0(j) V(j); S0 = Q0 K(j+1)^T; O1 += P1(j) V(j); S1 = Q1 K(j+1)^T. The tensor pipe
-    // executes what one thread issues in order, so S_t(j+1) overwrites the columns P_t(j) lived in only after the
-    // product that read them, and a completed S_t(j+1) also says that O_t holds the sum up to tile j.
-    constexpr uint32_t idesc = idesc_bf16(kTile, kTile);
-    const uint32_t full_mask = 0xffffffffu;
-    // A barrier that has already completed costs one non-suspending probe and a vote; only a real wait takes the polling loop.
-    auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
-      if (__all_sync(full_mask, mbar_test_wait(smem_u32(bar), parity))) return true;
-      return bool(__all_sync(full_mask, attn_wait(smem_u32(bar), parity, sh, g.status, code)));
-    };
-    bool ok = wait(&sh->q_full, 0, 13);
-    auto issue_s = [&](int t, int j) {  // S_t = Q_t K_j^T
-      const int st = j & 1;
-      // the second query tile reads the K tile the first one has just waited for
-      if (t == 0 && !wait(&sh->k_full[st], (j >> 1) & 1, 14)) return false;
-      tc_fence_after_sync();
-      if (elect_one())  // eight MMAs, the commit for the softmax warps and, behind the second query tile, the one that frees K
-        mma_f16_x8_commit(tmem + t * kTile, smem_desc_sw128(smem_u32(q_s + t * kTileBytes)), smem_desc_sw128(smem_u32(k_s + st * kTileBytes)),
-                          idesc, 0u, kSlab >> 4, smem_u32(&sh->s_full[t]), smem_u32(&sh->k_empty[st]), t == int(two) ? 1u : 0u);
-      __syncwarp();
-      return true;
-    };
-    // O_t += P_t V_j in two parts: the keys of the first chunks of probabilities as soon as those are written, the rest
-    // when the last chunk is. A = P_t in tensor memory [queries x keys], 16 keys (eight 32-bit columns of bf16 pairs) per
-    // MMA; B = V [keys x d], N-major (16 keys are two groups of eight 128-byte rows), or V^T [d x keys] (four MMAs per slab of
-    // 64 keys, 32 bytes of each row apiece).
-    constexpr uint32_t idesc_pv = VT ? idesc : idesc | kIdescBMajorN;
-    constexpr uint64_t kStep = VT ? 2 : 16 * 128 >> 4;                    // 16 keys on
-    constexpr uint64_t kKeys64 = VT ? uint64_t(kSlab >> 4) : 4 * kStep;   // 64 keys on
-    auto issue_pv = [&](int t, int j, bool more) {
-      const int st = j & 1;
-      const uint32_t d = tmem + 2 * kTile + t * kTile, a = tmem + t * kTile;
-      const uint64_t b = VT ? smem_desc_sw128(smem_u32(v_s + st * kTileBytes)) : smem_desc_sw128_mn(smem_u32(v_s + st * kTileBytes), kSlab);
-      if (t == 0 && !wait(&sh->v_full[st], (j >> 1) & 1, 16)) return false;
-      if (!wait(&sh->p_part[t], j & 1, 17)) return false;
-      tc_fence_after_sync();
-      if (elect_one()) {
-        mma_f16_ts_x4<kStep>(d, a, b, idesc_pv, j ? 1u : 0u);
-        mma_f16_ts_x2<kStep>(d, a + 32, b + kKeys64, idesc_pv, 1u);
-        tc_commit(smem_u32(&sh->pv_part[t]));
+    // ------------------------------------------------------------ MMA issuer (one lane)
+    // The tensor pipe executes what one thread issues in order, so S_t(h + 2) overwrites the columns P_t(h) lived in only after
+    // the product that read them, and the commit behind both, on the half's s_full, also says that O_t holds the sum up to
+    // step h. It is sent without scores, too, at the end of the keys.
+    constexpr uint32_t idesc_s = idesc_bf16(kTile, kStep);
+    constexpr uint32_t idesc_pv = VT ? idesc_bf16(kTile, kTile) : idesc_bf16(kTile, kTile) | kIdescBMajorN;
+    // B of the second product = V [keys x d], N-major (16 keys are two groups of eight 128-byte rows), or V^T [d x keys] (four
+    // MMAs per slab of 64 keys, 32 bytes of each row apiece)
+    constexpr uint64_t kKeys16 = VT ? 2 : 16 * 128 >> 4;                   // 16 keys on
+    constexpr uint64_t kKeys64 = VT ? uint64_t(kSlab >> 4) : 4 * kKeys16;  // 64 keys on
+    if (elect_one()) {
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code) {  // one non-suspending probe; only a real wait takes the polling loop
+        return mbar_test_wait(smem_u32(bar), parity) || attn_wait(smem_u32(bar), parity, sh, g.status, code);
+      };
+      auto issue_s = [&](int t, int half, uint64_t k_desc) {  // scores of query tile t and 64 keys into that half of its columns
+        const uint64_t a = smem_desc_sw128(smem_u32(q_s + t * kTileBytes)), b = k_desc + half * (kStep * 128 >> 4);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint64_t adv = uint64_t((i >> 2) * (kSlab >> 4) + (i & 3) * 2);
+          mma_f16(tmem + t * kTile + half * kStep, a + adv, b + adv, idesc_s, i ? 1u : 0u);
+        }
+      };
+      bool ok = wait(&sh->q_full, 0, 13) && wait(&sh->k_full[0], 0, 14);
+      if (ok) {
+        tc_fence_after_sync();
+        for (int half = 0; half < (steps > 1 ? 2 : 1); ++half)
+          for (int t = 0; t < (two ? 2 : 1); ++t) {
+            issue_s(t, half, smem_desc_sw128(smem_u32(k_s)));
+            tc_commit(smem_u32(&sh->s_full[t][half]));
+          }
+        tc_commit(smem_u32(&sh->k_empty[0]));
       }
-      __syncwarp();
-      if (!wait(&sh->p_full[t], j & 1, 19)) return false;
-      tc_fence_after_sync();
-      if (elect_one()) {
-        mma_f16_ts_x2<kStep>(d, a + 48, b + kKeys64 + 2 * kStep, idesc_pv, 1u);
-        if (t == int(two)) tc_commit(smem_u32(&sh->v_empty[st]));
-        if (!more) tc_commit(smem_u32(&sh->pv_done[t]));
+      for (int j = 0; j < tiles && ok; ++j) {
+        const int st = j & 1;
+        const uint64_t k_desc = smem_desc_sw128(smem_u32(k_s + (st ^ 1) * kTileBytes));
+        const uint64_t v_desc = VT ? smem_desc_sw128(smem_u32(v_s + st * kTileBytes)) : smem_desc_sw128_mn(smem_u32(v_s + st * kTileBytes), kSlab);
+        if (!(ok = wait(&sh->v_full[st], (j >> 1) & 1, 16))) break;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int h = 2 * j + half;
+          if (h >= steps || !ok) break;
+          const bool more = h + 2 < steps;
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (t == 1 && !two) break;
+            if (!(ok = wait(&sh->p_full[t][half], j & 1, 17))) break;
+            tc_fence_after_sync();
+            // A = P_t in tensor memory [queries x keys], 16 keys (eight 32-bit columns of bf16 pairs) per MMA
+            const uint32_t d = tmem + 2 * kTile + t * kTile, a = tmem + t * kTile + half * kStep;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mma_f16_ts(d, a + 8 * i, v_desc + half * kKeys64 + i * kKeys16, idesc_pv, (i || h) ? 1u : 0u);
+            if (more) {
+              if (half == 0 && t == 0) {  // the first reader of the next K tile waits for it
+                if (!(ok = wait(&sh->k_full[st ^ 1], ((j + 1) >> 1) & 1, 14))) break;
+                tc_fence_after_sync();
+              }
+              issue_s(t, half, k_desc);
+            }
+            tc_commit(smem_u32(&sh->s_full[t][half]));
+          }
+          if (half == 1 || h + 1 == steps) tc_commit(smem_u32(&sh->v_empty[st]));
+          if (more && (half == 1 || h + 3 == steps)) tc_commit(smem_u32(&sh->k_empty[st ^ 1]));
+        }
       }
-      __syncwarp();
-      return true;
-    };
-    if (ok) ok = issue_s(0, 0) && (!two || issue_s(1, 0));
-    for (int j = 0; j < tiles && ok; ++j) {
-      const bool more = j + 1 < tiles;
-      ok = issue_pv(0, j, more) && (!more || issue_s(0, j + 1)) && (!two || (issue_pv(1, j, more) && (!more || issue_s(1, j + 1))));
     }
+    __syncwarp();
   }
   } else {
     reg_inc<kAttnRegsSoftmax>();
     // ------------------------------------------------------------ softmax, rescale, output
     // Warps 4-7 serve query tile 0, warps 8-11 query tile 1; within a tile a warp owns the 32 rows of the TMEM quadrant
-    // it may access (warp index % 4) and a thread one query row with all 128 keys of the tile, so nothing is exchanged
-    // between threads. While the softmax of one query tile runs, the tensor pipe works on the other tile's products.
+    // it may access (warp index % 4) and a thread one query row with all 64 keys of the step, so nothing is exchanged
+    // between threads.
     const int t = (warp - 4) >> 2;
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
@@ -282,11 +290,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     float m_used = -INFINITY;  // the maximum the accumulator and the running sum are expressed against (log2 units)
     float l = 0.0f;
     bool ok = true;
-    uint32_t r[4][32];
+    uint32_t r[2][32];  // the step's scores
     const f32x2 scale2 = pack2(g.scale_log2, g.scale_log2);
-    // p = 2^(s * scale - m) for the 32 keys of chunk c as bf16 pairs, written over columns [16 c, 16 c + 16) of the
-    // scores they came from (chunk 0's columns or, later, ones that are in registers by then); returns their sum.
-    auto emit_chunk = [&](int c, float m, f32x2 sum2) {
+    // p = 2^(s * scale - m) for the 32 keys of chunk c as bf16 pairs, written over columns [16 c, 16 c + 16) of the step's
+    // scores (chunk 0's, which are in registers by then); returns their sum.
+    auto emit_chunk = [&](uint32_t cols, int c, float m, f32x2 sum2) {
       const f32x2 negm2 = pack2(-m, -m);
       uint32_t pk[16];
 #pragma unroll
@@ -306,13 +314,19 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         const __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);  // key 2i in the low half: the lower K index
         pk[i >> 1] = *reinterpret_cast<const uint32_t*>(&pb);
       }
-      tmem_st_32x16(tmem_s + c * 16, pk);
+      tmem_st_32x16(cols + c * 16, pk);
       return sum2;
     };
-    auto mask_chunk = [&](int c, int valid) {  // the keys past the end of the sequence (last tile only)
+    auto load_step = [&](int h) {
+      const uint32_t cols = tmem_s + (h & 1) * kStep;
+      tmem_ld_32x32(cols, r[0]);
+      tmem_ld_32x32(cols + 32, r[1]);
+      tmem_ld_wait();
+      const int valid = g.seq_kv - h * kStep;  // keys of this step that exist; the last step may have fewer than 64
+      if (valid < kStep)
 #pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (c * 32 + i >= valid) r[c][i] = __float_as_uint(-INFINITY);
+        for (int i = 0; i < kStep; ++i)
+          if (i >= valid) r[i >> 5][i & 31] = __float_as_uint(-INFINITY);
     };
     auto chunk_max = [&](int c) {
       float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};  // four short chains instead of one of 32 steps
@@ -340,79 +354,61 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       }
       m_used = m_new;
     };
-    auto publish = [&](uint64_t* bar) {
-      tmem_st_wait();
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(bar));
-    };
     auto total = [&](f32x2 sum2) {
       float a, b;
       unpack2(sum2, a, b);
       return a + b;
     };
-    const int my_tiles = t == 0 || two ? tiles : 0;
-    for (int j = 0; j < my_tiles; ++j) {
-      if (!(ok = __all_sync(0xffffffffu, attn_wait<40>(smem_u32(&sh->s_full[t]), j & 1, sh, g.status, 18)))) break;
+    auto wait_half = [&](int h, int code) {  // the scores of step h are in its half; the product of step h - 2 has completed
+      ok = __all_sync(0xffffffffu, attn_wait<40>(smem_u32(&sh->s_full[t][h & 1]), (h >> 1) & 1, sh, g.status, code));
       tc_fence_after_sync();
-      const int valid = g.seq_kv - j * kTile;  // keys of this tile that exist
-      // The probabilities are computed against the reference maximum the accumulator was last scaled to, which is known
-      // before the tile arrives: chunk 0 is exponentiated while the others are still on their way out of tensor memory. No
-      // maximum is taken on this path: that the reference is still good enough is read off the tile's sum of probabilities.
-      f32x2 sum2 = pack2(0.0f, 0.0f);
-      tmem_ld_32x32(tmem_s, r[0]);
-      tmem_ld_wait();
-#pragma unroll
-      for (int c = 1; c < 4; ++c) tmem_ld_32x32(tmem_s + c * 32, r[c]);
-      if (valid < kTile) mask_chunk(0, valid);
-      if (j > 0) sum2 = emit_chunk(0, m_used, sum2);
-      tmem_ld_wait();  // every score is in registers, so P may overwrite any of the columns they came from
-#pragma unroll
-      for (int c = 1; c < 4; ++c)
-        if (valid < kTile) mask_chunk(c, valid);
-      if (j > 0)
-#pragma unroll
-        for (int c = 1; c < kFirstChunks; ++c) sum2 = emit_chunk(c, m_used, sum2);
-      float part_sum = total(sum2);
-      bool over = j == 0 || !(part_sum <= kTileSumLimit);  // the first tile; a row that outgrew its reference; inf or NaN
-      if (__any_sync(0xffffffffu, over)) {
-        // Rare after the first tiles. The reference becomes the running maximum. S_t(j) was issued behind O_t += P_t V(j-1),
-        // so its completion says that O_t is at rest. The probabilities are computed again against the new reference --
-        // every score is still in registers -- over the ones just written.
-        float mx = -INFINITY;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) mx = fmaxf(mx, chunk_max(c));
-        move_reference(over ? fmaxf(m_used, mx * g.scale_log2) : m_used, j > 0);  // scale > 0: the maximum commutes with it
-        sum2 = pack2(0.0f, 0.0f);
-#pragma unroll
-        for (int c = 0; c < kFirstChunks; ++c) sum2 = emit_chunk(c, m_used, sum2);
-        part_sum = total(sum2);
-      }
-      publish(&sh->p_part[t]);
-      // The tile's probabilities are summed in one chain over all of its keys, as if they were handed over together.
-#pragma unroll
-      for (int c = kFirstChunks; c < 4; ++c) sum2 = emit_chunk(c, m_used, sum2);
-      float tile_sum = total(sum2);
-      over = !(tile_sum - part_sum <= kTileSumLimit);
-      if (__any_sync(0xffffffffu, over)) {
-        // The last keys outgrew the reference after the first part's product was released: O_t is at rest again when that
-        // product has completed (the issuer waits for the rest of P before it touches O_t).
-        if (!(ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_part[t]), j & 1, sh, g.status, 21)))) break;
-        tc_fence_after_sync();
-        float mx = -INFINITY;
-#pragma unroll
-        for (int c = kFirstChunks; c < 4; ++c) mx = fmaxf(mx, chunk_max(c));
-        if (over) l += part_sum;  // a row within its limit keeps its sum: it does not depend on its neighbours
-        move_reference(over ? fmaxf(m_used, mx * g.scale_log2) : m_used, true);
-        sum2 = pack2(0.0f, 0.0f);
-#pragma unroll
-        for (int c = kFirstChunks; c < 4; ++c) sum2 = emit_chunk(c, m_used, sum2);
-        if (over) tile_sum = total(sum2);
-      }
-      l += tile_sum;
-      publish(&sh->p_full[t]);
+      return ok;
+    };
+    const int my_steps = t == 0 || two ? steps : 0;
+    // The first reference is the maximum over the first 128 keys.
+    for (int h = 0; h < min(my_steps, 2); ++h) {
+      if (!wait_half(h, 18)) break;
+      load_step(h);
+      m_used = fmaxf(m_used, fmaxf(chunk_max(0), chunk_max(1)) * g.scale_log2);  // scale > 0: the maximum commutes with it
     }
-    if (ok && my_tiles > 0 && (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->pv_done[t]), 0, sh, g.status, 20)))) {
+    f32x2 sum2 = pack2(0.0f, 0.0f);  // of the 128-key tile so far: one chain over its keys, so that a call's bits do not depend on the steps
+    // One body for both halves: unrolled over them it no longer fits the instruction cache (18900 tokens 5.65 ms, 5.23 as it is).
+#pragma unroll 1
+    for (int h = 0; h < my_steps && ok; ++h) {
+      const int half = h & 1;
+      const uint32_t cols = tmem_s + half * kStep;
+      if (!wait_half(h, 18)) break;
+      load_step(h);
+      // The probabilities are computed against the reference maximum the accumulator was last scaled to. No maximum is taken on
+      // this path: that the reference is still good enough is read off the sum of the probabilities.
+      f32x2 start = half ? sum2 : pack2(0.0f, 0.0f);
+      sum2 = emit_chunk(cols, 0, m_used, start);
+      sum2 = emit_chunk(cols, 1, m_used, sum2);
+      const bool over = !(total(sum2) <= kTileSumLimit);  // a row that outgrew its reference; inf or NaN
+      if (__any_sync(0xffffffffu, over)) {
+        // Rare. The reference becomes the running maximum. O_t is at rest once the product of the step before has completed, which that
+        // step's half says the next time it is handed over. The probabilities are computed again -- every score is still in
+        // registers -- over the ones just written; rows within their limit keep reference and sum, so that they do not
+        // depend on their neighbours.
+        if (h > 0 && !wait_half(h + 1, 21)) break;
+        float m_new = m_used;
+        if (over) {
+          m_new = fmaxf(m_used, fmaxf(chunk_max(0), chunk_max(1)) * g.scale_log2);
+          l += total(start);
+          start = pack2(0.0f, 0.0f);
+        }
+        move_reference(m_new, h > 0);
+        sum2 = emit_chunk(cols, 0, m_used, start);
+        sum2 = emit_chunk(cols, 1, m_used, sum2);
+      }
+      if (half == 1 || h + 1 == my_steps) l += total(sum2);
+      tmem_st_wait();
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh->p_full[t][half]));
+    }
+    if (ok && my_steps > 0 &&  // the last step's product has completed
+        (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->s_full[t][(my_steps - 1) & 1]), ((my_steps + 1) >> 1) & 1, sh, g.status, 20)))) {
       tc_fence_after_sync();
       const float inv = 1.0f / l;
       const int qrow = q0 + t * kTile + row;

@@ -27,6 +27,10 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// The same value in every lane of a converged warp, and known to be: the compiler then keeps what depends on it in uniform
+// registers, which is where the operands of a tcgen05 or TMA instruction have to be.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // Register rebalancing between warpgroups (every thread of a warpgroup executes the same one).
 template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -152,57 +156,6 @@ __device__ __forceinline__ void mma_f16_ts(uint32_t d, uint32_t a_tmem, uint64_t
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
       "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Eight kind::f16 MMAs over one 128-byte-swizzled [rows x 128 columns of 16-bit] operand pair -- two 64-column slabs of
-// `slab16` 16-byte units each, four K = 16 steps of 32 bytes per slab -- and the commits that follow them, as ONE
-// instruction sequence from one thread: the descriptors advance by immediate adds inside the sequence, so the issuing
-// thread spends tens of cycles per MMA instead of rebuilding two 64-bit descriptors for each. `accumulate_first` == 0
-// makes the first MMA overwrite D. `bar2` gets a second commit when `commit2` != 0.
-__device__ __forceinline__ void mma_f16_x8_commit(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate_first,
-                                                  uint32_t slab16, uint32_t bar1, uint32_t bar2, uint32_t commit2) {
-  asm volatile(
-      "{\n\t.reg .pred p, pt, pc;\n\t.reg .b64 s, a1, a2, a3, a4, a5, a6, a7, b1, b2, b3, b4, b5, b6, b7;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\tsetp.ne.b32 pc, %8, 0;\n\tcvt.u64.u32 s, %5;\n\t"
-      "add.s64 a1, %1, 2;\n\tadd.s64 a2, %1, 4;\n\tadd.s64 a3, %1, 6;\n\tadd.s64 a4, %1, s;\n\t"
-      "add.s64 a5, a4, 2;\n\tadd.s64 a6, a4, 4;\n\tadd.s64 a7, a4, 6;\n\t"
-      "add.s64 b1, %2, 2;\n\tadd.s64 b2, %2, 4;\n\tadd.s64 b3, %2, 6;\n\tadd.s64 b4, %2, s;\n\t"
-      "add.s64 b5, b4, 2;\n\tadd.s64 b6, b4, 4;\n\tadd.s64 b7, b4, 6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a1, b1, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a3, b3, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a4, b4, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a5, b5, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a6, b6, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], a7, b7, %3, pt;\n\t"
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
-      "@pc tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t}" ::"r"(d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate_first), "r"(slab16), "r"(bar1), "r"(bar2), "r"(commit2)
-      : "memory");
-}
-// The `_ts` forms: A in tensor memory, two or four K = 16 steps, B advancing by STEP 16-byte units, no commit.
-template <uint64_t STEP> __device__ __forceinline__ void mma_f16_ts_x4(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, pt;\n\t.reg .b64 b1, b2, b3;\n\t.reg .b32 a1, a2, a3;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
-      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
-      "add.s64 b1, %2, %5;\n\tadd.s64 b2, b1, %5;\n\tadd.s64 b3, b2, %5;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, pt;\n\t}" ::"r"(d),
-      "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate_first), "n"(STEP)
-      : "memory");
-}
-template <uint64_t STEP> __device__ __forceinline__ void mma_f16_ts_x2(uint32_t d, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate_first) {
-  asm volatile(
-      "{\n\t.reg .pred p, pt;\n\t.reg .b64 b1;\n\t.reg .b32 a1;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 pt, 0, 0;\n\t"
-      "add.u32 a1, %1, 8;\n\tadd.s64 b1, %2, %5;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, pt;\n\t}" ::"r"(d),
-      "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate_first), "n"(STEP)
       : "memory");
 }
 // Block-scaled e2m1 x e2m1, one ue4m3 scale per 16 elements (four per K=64 instruction).

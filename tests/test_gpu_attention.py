@@ -108,6 +108,31 @@ def test_one_key_that_outgrows_the_reference(spike):
     run_case(q, k, v, heads, heads)
 
 
+@pytest.mark.parametrize("aligned_v", [True, False])
+@pytest.mark.parametrize("seq_q,seq_kv", [(1, 1), (130, 63), (300, 64), (256, 65), (129, 127), (300, 128), (130, 129), (40, 191), (300, 192), (257, 193)])
+def test_edges_of_the_steps_of_64_keys(seq_q, seq_kv, aligned_v):
+    """One step, a full or ragged first or second half of a key tile at the end, one and two query tiles."""
+    heads = 3
+    q, k, v = data(seq_q, heads, 31, 0.3), data(seq_kv, heads, 32, 0.3), data(seq_kv, heads, 33, 1.0)
+    dq, dk, dv = (bf16_tensor(oracle.to_bf16(t)) for t in (q, k, v))
+    if not aligned_v:
+        shifted = torch.empty(seq_kv * heads * D + 8, dtype=torch.bfloat16, device="cuda")[1:1 + seq_kv * heads * D].view(seq_kv, heads * D)
+        shifted.copy_(dv)
+        dv = shifted
+    close(oracle.attention(q, k, v, heads, heads, D, 1.0 / np.sqrt(D)), oracle.from_bf16(bits(attention(dq, dk, dv, heads, heads))))
+    assert sfq.device_status() == 0
+
+
+@pytest.mark.parametrize("spikes", [(63,), (64,), (128 + 63, 128 + 64), (128 + 64, 256), (129, 200, 384)])
+def test_reference_that_moves_at_the_edge_of_a_step(spikes):
+    """Rows outgrow their reference in the first or second half of a key tile, in neighbouring steps, and in the last step."""
+    seq, heads = 385, 2
+    q, k, v = data(seq, heads, 81, 1.0), data(seq, heads, 82, 0.3), data(seq, heads, 83, 1.0)
+    for i, s in enumerate(spikes):
+        k[s] = oracle.from_bf16(oracle.to_bf16(((4.0 + 2 * i) * np.where(q[s // 2] < 0, -1.0, 1.0)).astype(np.float32)))
+    run_case(q, k, v, heads, heads)
+
+
 def test_values_that_do_not_start_on_sixteen_bytes():
     """q, k and out need 16-byte rows, v never did: such a v is copied to the workspace first."""
     seq, heads = 259, 2
