@@ -99,7 +99,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Shared* sh = reinterpret_cast<Shared*>(smem + C::kStages * C::kStageBytes);
 
-  const int warp = threadIdx.x >> 5;
+  // Known to be the same in the whole warp, so that the roles' descriptors, coordinates and barrier addresses are computed in uniform
+  // registers, where tcgen05 and TMA take them from: 13950 x 5120 -> 13824 nvfp4 480 -> 466 us, W4A8 4096 x 5120 -> 5120 113.5 -> 110.7.
+  const int warp = int(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
   const int pair = blockIdx.x >> 1;
@@ -169,7 +171,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   tc_fence_before_sync();
   cluster_sync_all();  // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after_sync();
-  const uint32_t tmem = sh->tmem_base;
+  const uint32_t tmem = warp_uniform(sh->tmem_base);
   // The set-up above ran beside the end of the kernel that writes the activation; the next kernel's may run beside this one's end.
   grid_dependency_release();
   grid_dependency_wait();
