@@ -92,9 +92,20 @@ __device__ __forceinline__ bool attn_wait(uint32_t bar, uint32_t parity, AttnSha
   }
 }
 
-__device__ __forceinline__ float max3(float a, float b, float c) {  // one instruction on sm_100
+// Minima and maxima that a NaN goes through (fminf and fmaxf drop it), one instruction each.
+__device__ __forceinline__ float max3(float a, float b, float c) {
   float d;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float d;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
   return d;
 }
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -108,11 +119,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // x = n + f with n = round(x), f in [-1/2, 1/2]: a cubic for 2^f (relative error 7.5e-5, a sixtieth of the bf16 rounding
 // the result goes through) and n added into the exponent field. Arguments are clamped at -125 below, where the result
 // (~2e-38) is as good as the zero the hardware instruction returns, and at 126 above: a row that has outgrown its
-// reference by that much must still produce a huge value, which the caller's sum test then catches.
+// reference by that much must still produce a huge value, which the caller's sum test then catches. So does a NaN, whose
+// exponent field the addition leaves at 0x7f7fffff, the largest finite number: the caller looks for NaN where it moves the reference.
 __device__ __forceinline__ f32x2 exp2_pair_fma(f32x2 x) {
   float x0, x1;
   unpack2(x, x0, x1);
-  const f32x2 xc = pack2(fminf(fmaxf(x0, -125.0f), 126.0f), fminf(fmaxf(x1, -125.0f), 126.0f));
+  const f32x2 xc = pack2(min_nan(max_nan(x0, -125.0f), 126.0f), min_nan(max_nan(x1, -125.0f), 126.0f));
   const f32x2 magic = pack2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: the sum's low mantissa bits hold round(x)
   const f32x2 t = add2(xc, magic);
   const f32x2 f = sub2(xc, sub2(t, magic));
@@ -334,7 +346,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       for (int i = 0; i < 32; i += 8)
 #pragma unroll
         for (int k = 0; k < 4; ++k) m4[k] = max3(m4[k], __uint_as_float(r[c][i + 2 * k]), __uint_as_float(r[c][i + 2 * k + 1]));
-      return fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      return max_nan(max_nan(m4[0], m4[1]), max_nan(m4[2], m4[3]));
     };
     // The reference maximum becomes m_new in the rows that outgrew it; O and the running sum follow (the TMEM accesses are
     // warp-wide; rows within their limit use a factor of 1). O_t has to be at rest.
@@ -369,7 +381,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     for (int h = 0; h < min(my_steps, 2); ++h) {
       if (!wait_half(h, 18)) break;
       load_step(h);
-      m_used = fmaxf(m_used, fmaxf(chunk_max(0), chunk_max(1)) * g.scale_log2);  // scale > 0: the maximum commutes with it
+      m_used = max_nan(m_used, max_nan(chunk_max(0), chunk_max(1)) * g.scale_log2);  // scale > 0: the maximum commutes with it
     }
     f32x2 sum2 = pack2(0.0f, 0.0f);  // of the 128-key tile so far: one chain over its keys, so that a call's bits do not depend on the steps
     // One body for both halves: unrolled over them it no longer fits the instruction cache (18900 tokens 5.65 ms, 5.23 as it is).
@@ -393,7 +405,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         if (h > 0 && !wait_half(h + 1, 21)) break;
         float m_new = m_used;
         if (over) {
-          m_new = fmaxf(m_used, fmaxf(chunk_max(0), chunk_max(1)) * g.scale_log2);
+          m_new = max_nan(m_used, max_nan(chunk_max(0), chunk_max(1)) * g.scale_log2);
+          m_new = fmaf(m_new, 0.0f, m_new);  // a score of +inf or NaN makes its row NaN: the reference becomes it, and with it all that follows
           l += total(start);
           start = pack2(0.0f, 0.0f);
         }

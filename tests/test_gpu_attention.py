@@ -108,6 +108,32 @@ def test_one_key_that_outgrows_the_reference(spike):
     run_case(q, k, v, heads, heads)
 
 
+def run_not_finite(q, k, v, heads):
+    """Every query head is the same one, over one key / value head; NaN exactly where the dense softmax has it, close elsewhere."""
+    want = oracle.attention(q, k, v, 1, 1, D, 1.0 / np.sqrt(D))
+    dq, dk, dv = (bf16_tensor(oracle.to_bf16(t)) for t in (q, k, v))
+    got = oracle.from_bf16(bits(attention(dq.repeat(1, heads), dk, dv, heads, 1)))
+    for h in (0, heads - 1):
+        part = got[:, h * D:(h + 1) * D]
+        nan = np.isnan(want)
+        assert np.array_equal(nan, np.isnan(part)), (int(nan.sum()), int(np.isnan(part).sum()))
+        close(want[~nan], part[~nan])
+    assert sfq.device_status() == 0
+    return want
+
+
+@pytest.mark.parametrize("whole_blocks", [False, True])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("key", [0, 1, 2, 3, 4, 5, 6, 7, 64, 66, 129, 130, 192, 299])
+def test_one_key_that_is_not_finite(key, value, whole_blocks):
+    """A score that is NaN or +inf makes its row NaN, wherever in a group of eight keys it stands; one that is -inf has no weight."""
+    seq = 300
+    q, k, v = data(seq, 1, 84, 1.0), data(seq, 1, 85, 0.3), data(seq, 1, 86, 1.0)
+    k[key, 5] = value
+    want = run_not_finite(q, k, v, heads_of_whole_blocks(seq) if whole_blocks else 2)
+    assert np.isnan(want).any() and (np.isnan(value) or not np.isnan(want).all())
+
+
 @pytest.mark.parametrize("aligned_v", [True, False])
 @pytest.mark.parametrize("seq_q,seq_kv", [(1, 1), (130, 63), (300, 64), (256, 65), (129, 127), (300, 128), (130, 129), (40, 191), (300, 192), (257, 193)])
 def test_edges_of_the_steps_of_64_keys(seq_q, seq_kv, aligned_v):
