@@ -29,6 +29,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cfloat>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -299,7 +300,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     const uint32_t lane_base = uint32_t(quad * 32) << 16;
     const uint32_t tmem_s = tmem + lane_base + t * kTile;
     const uint32_t tmem_o = tmem + lane_base + 2 * kTile + t * kTile;
-    float m_used = -INFINITY;  // the maximum the accumulator and the running sum are expressed against (log2 units)
+    // The maximum the accumulator and the running sum are expressed against (log2 units). It stays at the lowest number while all of
+    // a row's scores are -inf: against -inf itself they would be NaN.
+    float m_used = -FLT_MAX;
     float l = 0.0f;
     bool ok = true;
     uint32_t r[2][32];  // the step's scores
@@ -423,7 +426,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     if (ok && my_steps > 0 &&  // the last step's product has completed
         (ok = __all_sync(0xffffffffu, attn_wait(smem_u32(&sh->s_full[t][(my_steps - 1) & 1]), ((my_steps + 1) >> 1) & 1, sh, g.status, 20)))) {
       tc_fence_after_sync();
-      const float inv = 1.0f / l;
+      const float inv = m_used > -FLT_MAX ? 1.0f / l : NAN;  // NaN: no score of the row is finite, or one of them is NaN or +inf
       const int qrow = q0 + t * kTile + row;
       const bool row_ok = qrow < g.seq_q;
       __nv_bfloat16* dst = g.out + size_t(row_ok ? qrow : 0) * g.ld_out + head * kTile;

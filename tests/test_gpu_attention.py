@@ -134,6 +134,18 @@ def test_one_key_that_is_not_finite(key, value, whole_blocks):
     assert np.isnan(want).any() and (np.isnan(value) or not np.isnan(want).all())
 
 
+@pytest.mark.parametrize("whole_blocks", [False, True])
+@pytest.mark.parametrize("first", [1, 64, 127, 128, 129, 130, 192, 257, 299, 300])
+def test_keys_of_no_weight_at_the_start(first, whole_blocks):
+    """Rows whose first scores are all -inf are the average of the other keys; a row without any finite score is NaN."""
+    seq = 300
+    q, k, v = data(seq, 1, 87, 1.0), data(seq, 1, 88, 0.3), data(seq, 1, 89, 1.0)
+    q[:, 5] = np.where(np.arange(seq) % 3 == 0, 0.0, np.abs(q[:, 5]) + 0.25)  # 0 * -inf is NaN: every third row
+    k[:first, 5] = -np.inf
+    want = run_not_finite(q, k, v, heads_of_whole_blocks(seq) if whole_blocks else 2)
+    assert np.isnan(want[0]).all() and np.isnan(want[1]).all() == (first == seq)
+
+
 @pytest.mark.parametrize("aligned_v", [True, False])
 @pytest.mark.parametrize("seq_q,seq_kv", [(1, 1), (130, 63), (300, 64), (256, 65), (129, 127), (300, 128), (130, 129), (40, 191), (300, 192), (257, 193)])
 def test_edges_of_the_steps_of_64_keys(seq_q, seq_kv, aligned_v):
