@@ -96,10 +96,10 @@ def test_running_maximum_that_keeps_growing():
     assert sfq.device_status() == 0
 
 
-@pytest.mark.parametrize("spike", [0, 33, 95, 96, 127, 128 + 31, 128 + 95, 128 + 96, 128 + 127, 256 + 110, 399])
+@pytest.mark.parametrize("spike", [0, 33, 95, 96, 127, 128 + 31, 128 + 63, 128 + 64, 128 + 95, 128 + 96, 128 + 127, 256, 256 + 110, 399])
 def test_one_key_that_outgrows_the_reference(spike):
-    """One key raises some rows' scores by more than 2^15 in base-2 units of probability: the reference maximum moves inside that
-    key tile, before the tile's first part of probabilities is handed over or after it, with the accumulator rescaled either way."""
+    """One key raises some rows' scores by more than 2^15 in base-2 units of probability: past the first 128 keys, over which the first
+    reference is taken, the reference maximum moves in that key's step and the accumulator is rescaled."""
     seq, heads = 400, 2
     q, k, v = data(seq, heads, 81, 1.0), data(seq, heads, 82, 0.3), data(seq, heads, 83, 1.0)
     k[spike] = oracle.from_bf16(oracle.to_bf16((4.0 * np.where(q[spike // 2] < 0, -1.0, 1.0)).astype(np.float32)))
@@ -149,7 +149,7 @@ def test_keys_of_no_weight_at_the_start(first, whole_blocks):
 @pytest.mark.parametrize("aligned_v", [True, False])
 @pytest.mark.parametrize("seq_q,seq_kv", [(1, 1), (130, 63), (300, 64), (256, 65), (129, 127), (300, 128), (130, 129), (40, 191), (300, 192), (257, 193)])
 def test_edges_of_the_steps_of_64_keys(seq_q, seq_kv, aligned_v):
-    """One step, a full or ragged first or second half of a key tile at the end, one and two query tiles."""
+    """One step, a full or ragged first or second half of a key tile at the end, in CTAs of one query tile."""
     heads = 3
     q, k, v = data(seq_q, heads, 31, 0.3), data(seq_kv, heads, 32, 0.3), data(seq_kv, heads, 33, 1.0)
     dq, dk, dv = (bf16_tensor(oracle.to_bf16(t)) for t in (q, k, v))
@@ -161,14 +161,114 @@ def test_edges_of_the_steps_of_64_keys(seq_q, seq_kv, aligned_v):
     assert sfq.device_status() == 0
 
 
+@pytest.mark.parametrize("aligned_v", [True, False])
+@pytest.mark.parametrize("seq_kv", [1, 63, 64, 65, 127, 128, 129, 191, 192, 193, 256])
+@pytest.mark.parametrize("seq_q", [256, 300])
+def test_edges_of_the_steps_with_two_query_tiles(seq_q, seq_kv, aligned_v):
+    """The same ends of the keys in CTAs whose second query tile has rows (the launches above run one query tile per CTA, or one
+    whose second tile is empty): every query head is the same one, over one key / value head."""
+    heads = heads_of_whole_blocks(seq_q)
+    q, k, v = data(seq_q, 1, 34, 0.3), data(seq_kv, 1, 35, 0.3), data(seq_kv, 1, 36, 1.0)
+    dq, dk, dv = (bf16_tensor(oracle.to_bf16(t)) for t in (q, k, v))
+    if not aligned_v:
+        shifted = torch.empty(seq_kv * D + 8, dtype=torch.bfloat16, device="cuda")[1:1 + seq_kv * D].view(seq_kv, D)
+        shifted.copy_(dv)
+        dv = shifted
+    out = attention(dq.repeat(1, heads), dk, dv, heads, 1)
+    close(oracle.attention(q, k, v, 1, 1, D, 1.0 / np.sqrt(D)), oracle.from_bf16(bits(out[:, :D].contiguous())))
+    assert torch.equal(out, out[:, :D].repeat(1, heads))
+    assert sfq.device_status() == 0
+
+
 @pytest.mark.parametrize("spikes", [(63,), (64,), (128 + 63, 128 + 64), (128 + 64, 256), (129, 200, 384)])
 def test_reference_that_moves_at_the_edge_of_a_step(spikes):
-    """Rows outgrow their reference in the first or second half of a key tile, in neighbouring steps, and in the last step."""
+    """Spikes at the edges of steps, inside the first 128 keys (where they raise the first reference) and behind them."""
     seq, heads = 385, 2
     q, k, v = data(seq, heads, 81, 1.0), data(seq, heads, 82, 0.3), data(seq, heads, 83, 1.0)
     for i, s in enumerate(spikes):
         k[s] = oracle.from_bf16(oracle.to_bf16(((4.0 + 2 * i) * np.where(q[s // 2] < 0, -1.0, 1.0)).astype(np.float32)))
     run_case(q, k, v, heads, heads)
+
+
+def moves_of_the_reference(scores):
+    """What the kernel's rule does with a row's scores (log2 units): the steps of 64 keys whose sum exceeds 2^15 against the reference,
+    as (step, what exceeded it: the step itself or only the sum carried over from the tile's first half, whether the reference moved)."""
+    reference, carried, found = scores[:128].max(), 0.0, []
+    for step in range(-(-len(scores) // 64)):
+        part = scores[64 * step:64 * step + 64]
+        carried = carried if step % 2 else 0.0
+        alone = np.exp2(part - reference).sum()
+        total = carried + alone
+        if total > 32768:
+            higher = max(reference, part.max())
+            found.append((step, "step" if alone > 32768 else "carried", bool(higher > reference)))
+            reference = higher
+            total = np.exp2(part - reference).sum()
+        carried = total
+    return found
+
+
+@pytest.mark.parametrize("aligned_v", [True, False])
+@pytest.mark.parametrize("whole_blocks", [False, True])
+def test_each_way_a_reference_can_move(whole_blocks, aligned_v):
+    """Rows that outgrow their reference in successive steps, in the first or second half of a key tile alone, in the last step, through the
+    sum of a tile's halves alone (with a higher maximum and without one), several of them in one warp; rows beside them keep their bits."""
+    seq_q, seq_kv = 300, 449
+    plans = {  # of a row: {key: score in log2 units}, 0 elsewhere, and the moves it is made for
+        "successive": ({128 + 10: 30, 192 + 63: 60, 256: 90, 320 + 5: 120, 448: 150},
+                       [(2, "step", True), (3, "step", True), (4, "step", True), (5, "step", True), (7, "step", True)]),
+        "first half": ({256 + 40: 33}, [(4, "step", True)]),
+        "second half": ({192 + 1: 33}, [(3, "step", True)]),
+        "carried": ({j: np.log2(20000 / 64) for j in range(128, 256)}, [(3, "carried", True)]),
+        "carried, no higher": ({j: np.log2(32736 / 64) for j in range(128, 192)}, [(3, "carried", False)]),
+        "within the limit": ({j: np.log2(20000 / 64) for j in range(256, 320)}, []),
+    }
+    rows = {5: "successive", 6: "carried", 7: "within the limit", 40: "first half", 70: "carried, no higher", 71: "second half",
+            133: "successive", 134: "carried, no higher", 200: "carried", 260: "carried", 261: "first half", 290: "within the limit"}
+    q, k, v = data(seq_q, 1, 91, 1.0), data(seq_kv, 1, 92, 0.3), data(seq_kv, 1, 93, 1.0)
+    q[:, :12], k[:, :12] = 0.0, 0.0  # two channels per plan, in which a row of the plan is (8, 1) and everything else 0
+    for row in rows:
+        q[row] = 0.0
+    for i, (name, (scores, _)) in enumerate(plans.items()):
+        for row in (r for r in rows if rows[r] == name):
+            q[row, 2 * i:2 * i + 2] = 8.0, 1.0
+        for key, score in scores.items():
+            dot = np.float32(score * np.sqrt(D) / np.log2(np.e))
+            k[key, 2 * i] = oracle.from_bf16(oracle.to_bf16(np.array([dot / 8], np.float32)))[0]
+            k[key, 2 * i + 1] = oracle.from_bf16(oracle.to_bf16(np.array([dot - 8 * k[key, 2 * i]], np.float32)))[0]
+    scores = q.astype(np.float64) @ k.T.astype(np.float64) / np.sqrt(D) * np.log2(np.e)
+    for row in range(seq_q):
+        assert moves_of_the_reference(scores[row]) == (plans[rows[row]][1] if row in rows else []), row
+    heads = heads_of_whole_blocks(seq_q) if whole_blocks else 2
+    dk, dv = bf16_tensor(oracle.to_bf16(k)), bf16_tensor(oracle.to_bf16(v))
+    if not aligned_v:
+        shifted = torch.empty(seq_kv * D + 8, dtype=torch.bfloat16, device="cuda")[1:1 + seq_kv * D].view(seq_kv, D)
+        shifted.copy_(dv)
+        dv = shifted
+    out = attention(bf16_tensor(oracle.to_bf16(q)).repeat(1, heads), dk, dv, heads, 1)
+    close(oracle.attention(q, k, v, 1, 1, D, 1.0 / np.sqrt(D)), oracle.from_bf16(bits(out[:, :D].contiguous())))
+    assert torch.equal(out, out[:, :D].repeat(1, heads))
+    still = q.copy()
+    moving = [row for row in rows if plans[rows[row]][1]]
+    still[moving] = 0.0
+    alone = attention(bf16_tensor(oracle.to_bf16(still)).repeat(1, heads), dk, dv, heads, 1)
+    others = [row for row in range(seq_q) if row not in moving]
+    assert torch.equal(out[others], alone[others])  # a row's bits do not depend on its neighbours
+    assert sfq.device_status() == 0
+
+
+def test_launches_repeat_bit_for_bit():
+    """The next scores are written over the columns the product before them reads its probabilities from, with nothing between the two
+    but the order in which they were issued: a product that were overtaken would show in some launch of many."""
+    seq, heads = 2048, 40
+    g = torch.Generator("cuda").manual_seed(17)
+    q, k, v = (torch.randn((seq, heads * D), device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+    first = attention(q, k, v, heads, heads)
+    same = torch.ones((), dtype=torch.bool, device="cuda")
+    for _ in range(300):
+        same &= (attention(q, k, v, heads, heads) == first).all()
+    assert bool(same)
+    assert sfq.device_status() == 0
 
 
 def test_values_that_do_not_start_on_sixteen_bytes():
@@ -252,7 +352,8 @@ def test_reference_that_moves_in_whole_blocks(spike, aligned_v):
 def test_bits_of_seeded_calls(seq, heads, scale, crc):
     """How a key tile's probabilities are handed to the second product is a matter of speed alone: their sum is one chain over the
     tile's keys, and a call's bits are those of the kernel that handed them over in one part (its checksums). A sum per part
-    shows in a few of a million elements."""
+    shows in a few of a million elements. No row of these calls outgrows its first reference; one that does has bits that depend on the
+    keys over which its new reference is taken."""
     q, k, v = (bf16_tensor(oracle.to_bf16(data(seq, heads, 300 + i + seq, scale))) for i in range(3))
     assert zlib.crc32(bits(attention(q, k, v, heads, heads)).tobytes()) == crc
 
