@@ -6,7 +6,7 @@
 //
 // One CTA owns TWO tiles of 128 queries of one head and walks the keys in steps of 64 with an online softmax. The scores of a
 // query tile lie in two halves of 64 columns that take turns, so a step's scores are computed while the softmax warps work on the
-// step before: a query tile's chain (scores -> softmax -> product -> next scores) never stands still at either end.
+// step before and a query tile's chain (scores -> softmax -> product -> next scores) has two steps in it at a time.
 //   warp 0      TMA producer: both Q tiles once, then a two-stage ring of K and V tiles [128 keys x 128 d]. The second product
 //               reads V as it lies, as an N-major operand (its N is d, its K the keys), or - VT, where its rows are not aligned -
 //               V transposed once per call by transpose_v_kernel, [128 d x 128 keys], K-major like the other operands
@@ -16,15 +16,18 @@
 //               32 columns of the 64 scores it was computed from
 //   warps 4-7   softmax of query tile 0, warps 8-11 of query tile 1 (warps 2-3 only hand their registers over), one query row per
 //               thread with all 64 keys of the step: S from TMEM, P = exp2(s - m) as bf16 pairs back into TMEM, the running sum,
-//               and - only when the step's probabilities sum to more than 2^15, i.e. the row has outgrown the reference maximum m the
-//               accumulator was last scaled to - the true running maximum, a rescale of O in TMEM and the step's
-//               probabilities again. A stale reference changes nothing in exact arithmetic (numerator and denominator
+//               and - only when the probabilities of the key tile so far sum to more than 2^15, i.e. the row has outgrown the reference
+//               m the accumulator was last scaled to - the maximum of m and this step's scores as the new reference, a rescale of O
+//               in TMEM and the step's probabilities again, none of them above 1. A stale reference, or one that is not the
+//               maximum of all keys so far, changes nothing in exact arithmetic (numerator and denominator
 //               carry the same factor); the limit keeps every p far inside the range of bf16 and fp32, and no maximum over
 //               the scores is computed on the common path.
-// 40 heads, 2048 / 4747 / 18900 tokens in bursts: 0.096 / 0.403 / 5.47 ms; steps of 128 keys, whose next scores wait for the product that
-// still reads P from their columns, 0.107 / 0.448 / 5.72 ms. What bounds it now (timing-only ablations at 18900 tokens): the
-// tensor side alone takes 4.6 ms, most of it shared memory (a 128x64x16 MMA reads 6 KB in the 32 cycles its arithmetic takes and runs
-// in 48), the softmax side alone 4.2.
+// 40 heads, 2048 / 4747 / 18900 tokens in bursts: 0.096 / 0.406 / 5.48 ms (75600: 96.6 ms); steps of 128 keys, whose next scores wait for the
+// product that still reads P from their columns, 0.107 / 0.448 / 5.72 ms. What bounds it (timing-only ablations at 18900 tokens, of a
+// build that took 5.3 to 5.5 ms whole): the tensor side alone takes 4.6 ms, most of it shared memory (a 128x64x16 MMA reads 6 KB in the
+// 32 cycles its arithmetic takes and runs in 48), the softmax side alone 4.2.
+// A row whose scores keep growing pays for its moves: 4747 tokens whose scores rise by 26 (104) log2 units along the keys, where a warp
+// moves in 16 % (60 %) of its steps, 0.490 (0.671) ms; the steps of 128 keys 0.578 (0.653).
 // Every wait is bounded; a wait that runs out stores a code in the status word and the CTA leaves.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -46,14 +49,14 @@ namespace {
 
 using namespace ptx;
 
-constexpr int kTile = 128;             // queries per query tile (two per CTA), keys per step, head_dim
+constexpr int kTile = 128;             // queries per query tile (two per CTA), keys per stage of K and V, head_dim
 constexpr int kSlab = kTile * 128;     // 128 rows x 128 bytes: 64 bf16 columns of a tile
 constexpr int kTileBytes = 2 * kSlab;  // [128 x 128] bf16
 constexpr int kStep = 64;              // keys per softmax step: half a key tile, half of a query tile's score columns
 constexpr int kAttnThreads = 384;  // warpgroup 0: producer, MMA issuer, two idle warps; warpgroups 1 and 2: the softmax of query tiles 0 and 1
 constexpr int kAttnRegsLean = 64, kAttnRegsSoftmax = 216;  // after setmaxnreg: 128 x 64 + 256 x 216 < 384 x 168, what the launch allocates
 constexpr int kTailWaves = 16;
-constexpr float kTileSumLimit = 32768.0f;  // a row's probabilities of a key tile may sum to this before its reference maximum moves
+constexpr float kTileSumLimit = 32768.0f;  // a row's probabilities of a key tile may sum to this before its reference moves
 
 struct AttnShared {
   uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2][2], p_full[2][2];
@@ -115,8 +118,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// 2^x for a pair of arguments on the FMA pipe instead of the special-function unit, which is what the softmax of two
-// query tiles saturates (32768 exponentials per key tile at 16 per clock = the 2048 cycles the tile's products take).
+// 2^x for a pair of arguments on the FMA pipe instead of the special-function unit, which would need 2048 cycles for the 32768
+// exponentials of two query tiles and a key tile (16 per clock), where their products take about 2500. A quarter of the pairs
+// taken here / none, 40 heads in bursts: 2048 tokens 0.0956 / 0.0975 ms, 4747 0.406 / 0.412, 18900 5.48 / 5.52, 75600 level.
 // x = n + f with n = round(x), f in [-1/2, 1/2]: a cubic for 2^f (relative error 7.5e-5, a sixtieth of the bf16 rounding
 // the result goes through) and n added into the exponent field. Arguments are clamped at -125 below, where the result
 // (~2e-38) is as good as the zero the hardware instruction returns, and at 126 above: a row that has outgrown its
@@ -222,9 +226,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (one lane)
-    // The tensor pipe executes what one thread issues in order, so S_t(h + 2) overwrites the columns P_t(h) lived in only after
-    // the product that read them, and the commit behind both, on the half's s_full, also says that O_t holds the sum up to
-    // step h. It is sent without scores, too, at the end of the keys.
+    // S_t(h + 2) overwrites the columns that P_t(h) V(h) reads its A operand from, with nothing between the two but the order of
+    // issue. That the tensor pipe executes MMAs of one thread in order is documented for MMAs of one accumulator and shape; these two
+    // differ in both, so here it is relied on beyond that, as the form in steps of 128 keys relied on it for the accumulators (a
+    // wait for the product's completion in its place would put the round trip back into the chain). The commit behind both, on
+    // the half's s_full, also says that O_t holds the sum up to step h. It is sent without scores, too, at the end of the keys.
     constexpr uint32_t idesc_s = idesc_bf16(kTile, kStep);
     constexpr uint32_t idesc_pv = VT ? idesc_bf16(kTile, kTile) : idesc_bf16(kTile, kTile) | kIdescBMajorN;
     // B of the second product = V [keys x d], N-major (16 keys are two groups of eight 128-byte rows), or V^T [d x keys] (four
@@ -386,8 +392,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       load_step(h);
       m_used = max_nan(m_used, max_nan(chunk_max(0), chunk_max(1)) * g.scale_log2);  // scale > 0: the maximum commutes with it
     }
-    f32x2 sum2 = pack2(0.0f, 0.0f);  // of the 128-key tile so far: one chain over its keys, so that a call's bits do not depend on the steps
-    // One body for both halves: unrolled over them it no longer fits the instruction cache (18900 tokens 5.65 ms, 5.23 as it is).
+    f32x2 sum2 = pack2(0.0f, 0.0f);  // of the 128-key tile so far: one chain over its keys, so that the bits of rows that keep their first reference do not depend on the steps
+    // One body for both halves: two bodies no longer fit the instruction cache (2048 / 4747 / 18900 tokens 0.0988 / 0.417 / 5.58 ms,
+    // 0.0956 / 0.406 / 5.48 as it is).
 #pragma unroll 1
     for (int h = 0; h < my_steps && ok; ++h) {
       const int half = h & 1;
@@ -401,7 +408,8 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       sum2 = emit_chunk(cols, 1, m_used, sum2);
       const bool over = !(total(sum2) <= kTileSumLimit);  // a row that outgrew its reference; inf or NaN
       if (__any_sync(0xffffffffu, over)) {
-        // Rare. The reference becomes the running maximum. O_t is at rest once the product of the step before has completed, which that
+        // Rare. The reference becomes the maximum of itself and this step's scores (itself, where only the sum carried over from the
+        // tile's first half is above the limit: the sum then starts anew). O_t is at rest once the product of the step before has completed, which that
         // step's half says the next time it is handed over. The probabilities are computed again -- every score is still in
         // registers -- over the ones just written; rows within their limit keep reference and sum, so that they do not
         // depend on their neighbours.
@@ -525,8 +533,8 @@ void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k,
     reserve_dynamic_smem(reinterpret_cast<const void*>(kernel), kAttnSmem, "sfq attention");
 
   // V is read as it lies, except one whose rows do not start on 16 bytes, which TMA cannot read: that one is transposed first.
-  // 40 heads in loops of 0.4 s, as it lies against transposed (pass included): 2048 tokens 0.106 / 0.136 ms, 4747 0.499 / 0.548,
-  // 18900 6.60 / 6.79, 75600 102.0 / 102.4.
+  // 40 heads in loops of 0.25 s, as it lies against transposed (pass included): 2048 tokens 0.099 / 0.124 ms, 4747 0.465 / 0.518,
+  // 18900 6.35 / 6.53.
   const bool transposed = reinterpret_cast<uintptr_t>(v) % 16 != 0;
   cudaError_t e = cudaSuccess;
   const int width = kv_heads * kTile, ld_t = padded_keys(seq_kv);
@@ -546,9 +554,10 @@ void attention_forward(const __nv_bfloat16* q, int ld_q, const __nv_bfloat16* k,
   a.status = device_status_word();
   // Units (256 queries of a head) run one per SM, all equally long, so a last wave that is nearly empty costs as much as a full
   // one: 4747 tokens x 40 heads are 760 units = 5.14 waves of 148. When the last wave's units fit the SMs twice over, they run
-  // as two CTAs of one query tile each, which take about 0.6 of the time (a query tile alone has no other tile to share the
-  // tensor pipe with). A row's arithmetic is the same either way. Past kTailWaves waves there is less to gain than the
-  // bookkeeping costs (1.4 % at 75600 tokens x 40 heads, 80 waves).
+  // as two CTAs of one query tile each, which take 0.75 of the time (74 units against 1000 / 4747 / 18900 keys 0.0161 / 0.0542 / 0.191 ms as
+  // single tiles, 0.0213 / 0.0729 / 0.252 whole). 40 heads with the split / without: 2048 tokens 0.0954 / 0.1043 ms, 4747 0.407 / 0.424, 7500
+  // 0.934 / 0.978. A row's arithmetic is the same either way. Past kTailWaves waves little is left to gain: 16200 tokens
+  // (17.3 waves) 4.08 / 4.13 ms, 19200 (20.3) 5.63 / 5.68, 36000 (38.1) level within the noise of 1 %.
   a.q_blocks = (seq_q + 2 * kTile - 1) / (2 * kTile);
   const int units = a.q_blocks * heads, sms = device_sm_count(), rest = units % sms;
   const int split = 2 * rest <= sms && units < kTailWaves * sms && seq_q > kTile ? rest : 0;

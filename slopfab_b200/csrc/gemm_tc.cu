@@ -120,10 +120,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ C
   // Each role's code sits directly under its warpgroup's setmaxnreg, so the compiler budgets it accordingly.
   //
   // The producer, MMA and scale-copy roles run as CONVERGED warps: all 32 lanes walk the loop and poll the
-  // barriers, and one elected lane issues the asynchronous instructions. A lone lane inside a divergent branch
-  // measured ~80 cycles per tcgen05 instruction (its operands are moved into uniform registers one by one);
-  // from a converged warp the same instruction issues in ~50, which is what lets one warp keep the tensor
-  // pipe fed (4 MMAs + 1 commit + 1 wait per 512-cycle stage).
+  // barriers, and one elected lane issues the asynchronous instructions. While the roles branched on a warp index that the
+  // compiler did not know to be uniform, a lone lane measured ~80 cycles per tcgen05 instruction (its operands were moved into
+  // uniform registers one by one) and a converged warp ~50, which is what let one warp keep the tensor pipe fed (4 MMAs + 1
+  // commit + 1 wait per 512-cycle stage). Behind a uniform branch a lone lane issues one in 6 to 10 cycles where the pipe does
+  // not hold it up (raw stream, A in tensor memory), as attention.cu does; the roles here have stayed as they are.
   if (warp < 4) {
     reg_dec<kRegsLean>();
     if (warp == 0) {

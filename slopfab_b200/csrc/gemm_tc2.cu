@@ -100,7 +100,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   Shared* sh = reinterpret_cast<Shared*>(smem + C::kStages * C::kStageBytes);
 
   // Known to be the same in the whole warp, so that the roles' descriptors, coordinates and barrier addresses are computed in uniform
-  // registers, where tcgen05 and TMA take them from: 13950 x 5120 -> 13824 nvfp4 480 -> 466 us, W4A8 4096 x 5120 -> 5120 113.5 -> 110.7.
+  // registers, where tcgen05 and TMA take them from: W4A8 4096 x 5120 -> 5120 113.5 -> 110.7 us; large launches under the power cap
+  // gain no more than their runs differ (13950 x 5120 -> 13824 nvfp4 477 -> 467 us, spread 2.7 %).
   const int warp = int(warp_uniform(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader
